@@ -5,13 +5,14 @@
 // and outputs with fewer are zero-padded), so one kernel covers every convolution.  A convolution
 // is an implicit GEMM:
 //   out[v][co] = sum over taps t, ci of  W[t][co][ci] * in[v + off_t][ci]
-// with M = 128 voxels along x (one tile), N = 32 output channels and K = 27 taps x 32 channels.
-// The tile of tap t is a TMA box of 128 voxels x 32 channels at the shifted coordinates, so the
-// copy engine does the im2col gather and the zero padding at the mesh edges (out-of-range boxes read
-// zeros).  The boxes land 64B-swizzled, the layout the MMA reads K-major; the 27 weight taps stay in
-// shared memory for the CTA's whole life.  One thread issues tcgen05.mma (M128 N32 K16, bf16 in,
-// f32 accumulate) into tensor memory; four epilogue warps read the accumulator back with
-// tcgen05.ld, add bias, a residual and the ReLU, and store bf16 (or the f32 field prediction).
+// with M = 128 voxels along x (one tile), N = 32 output channels of up to three taps and K = 27 taps
+// x 32 channels.  The rows that a tile's taps read are TMA boxes of 130 voxels x 32 channels at the
+// shifted coordinates, so the copy engine does the im2col gather and the zero padding at the mesh
+// edges (out-of-range boxes read zeros).  The boxes land 64B-swizzled, the layout the MMA reads
+// K-major; the 27 weight taps stay in shared memory for the CTA's whole life.  One thread issues
+// tcgen05.mma (M128 K16, bf16 in, f32 accumulate) into tensor memory; epilogue warps read the
+// accumulators back with tcgen05.ld, add bias, a residual and the ReLU, and store bf16 (or the f32
+// field prediction).
 //
 // The backward pass of the input is the same kernel run on the output gradient with the weights
 // flipped in space and transposed in channels (W'[26-t][ci][co] = W[t][co][ci]), with the ReLU
@@ -20,8 +21,8 @@
 // is a GEMM with M = 4 taps x 32 input channels, N = 32 output channels and K = voxels; both
 // operands are tiles of voxels x channels, read MN-major.
 //
-// Warp roles (192 threads): warp 0 issues the TMA copies, warp 1 owns the tensor memory and one
-// of its threads issues the MMAs, warps 2-5 run the epilogue.  Every wait is bounded: a role that
+// Warp roles: one thread issues the TMA copies, one the MMAs, the other warps run the epilogue (each
+// kernel's own comment has the numbers).  Every wait is bounded: a role that
 // gives up sets DEVERR_TIMEOUT and a shared abort flag, the others leave their loops, the copies
 // and MMAs in flight are waited for (bounded again) and the tensor memory is freed.
 
@@ -138,22 +139,23 @@ __device__ __forceinline__ void give_up(volatile int* flag, int* err)
 static constexpr uint32_t A_TILE_BYTES = SUR_TILE * SUR_C * 2; // 8192: 128 voxels x 32 channels
 static constexpr uint32_t W_TAP_BYTES = SUR_C * SUR_C * 2;	   // 2048
 static constexpr uint32_t W_BYTES = SUR_TAPS * W_TAP_BYTES;	   // 55296 (54 x 1024)
-// A stage holds the 130 voxels x0 - 1 .. x0 + 128 of one (y + dy, z + dz) row, which serve the three
-// taps dx = -1, 0, +1 as 128-row operands starting 0, 1 and 2 rows (64 bytes each) into the box.
+// A stage holds the 130 voxels x0 - 1 .. x0 + 128 of one (y + dy, z) row, which serve the three taps
+// dx = -1, 0, +1 as 128-row operands starting 0, 1 and 2 rows (64 bytes each) into the box.
 static constexpr int CONV_ROWS = SUR_TILE + 2;
 static constexpr uint32_t A_BOX_BYTES = CONV_ROWS * SUR_C * 2; // 8320
 static constexpr uint32_t A_STAGE_BYTES = 9216;					// rounded up to 1024
-static constexpr int CONV_PIPES = 3;  // independent pipelines per CTA, sharing the weights
-static constexpr int CONV_STAGES = 6; // stages per pipeline
+static constexpr int CONV_PIPES = 4;  // independent pipelines per CTA, sharing the weights
+static constexpr int CONV_STAGES = 4; // stages per pipeline
+static constexpr int CONV_PLANES = 4; // most output planes of a block
 static constexpr int CONV_THREADS = 32 * (2 * CONV_PIPES + 4 * CONV_PIPES);
-// barriers per pipeline: full and empty per stage, 2 accumulator full, 2 accumulator empty, drain;
-// then the shared weight barrier, the tensor-memory address and the abort flag
-static constexpr int CONV_PIPE_BARS = 2 * CONV_STAGES + 5;
-static constexpr size_t CONV_BAR_BYTES = (CONV_PIPES * CONV_PIPE_BARS + 1) * sizeof(uint64_t) + 2 * sizeof(uint32_t);
-static constexpr size_t CONV_SMEM =
-	1024 + W_BYTES + (size_t)CONV_PIPES * CONV_STAGES * A_STAGE_BYTES + CONV_BAR_BYTES;
+// barriers per pipeline: full and empty per stage and per output plane, drain; then the shared weight
+// barrier, the tensor-memory address and the abort flag
+static constexpr int CONV_PIPE_BARS = 2 * CONV_STAGES + 2 * CONV_PLANES + 1;
+static constexpr size_t CONV_SMEM = 1024 + W_BYTES + (size_t)CONV_PIPES * CONV_STAGES * A_STAGE_BYTES
+									+ (CONV_PIPES * CONV_PIPE_BARS + 1) * sizeof(uint64_t) + 2 * sizeof(uint32_t);
 static_assert(CONV_SMEM <= 227 * 1024, "convolution stages exceed the shared memory of a CTA");
 static_assert(A_BOX_BYTES <= A_STAGE_BYTES && A_STAGE_BYTES % 1024 == 0, "stage layout");
+static_assert(CONV_PIPES * CONV_PLANES * SUR_C == 512, "the accumulators fill the tensor memory");
 
 __device__ __forceinline__ void decode_tile(long long tile, const conv_params& p, int& b, int& z, int& y, int& x0)
 {
@@ -166,24 +168,37 @@ __device__ __forceinline__ void decode_tile(long long tile, const conv_params& p
 	x0 = xt * SUR_TILE;
 }
 
-__device__ __forceinline__ void load_bf16x32(const __nv_bfloat16* src, float (&v)[32])
+// 32 bf16 values of a voxel, as loaded (the epilogue issues these loads before it waits)
+struct bf16x32
 {
-	const uint4* s = reinterpret_cast<const uint4*>(src);
-#pragma unroll
-	for (int i = 0; i < 4; i++)
+	uint4 u[4];
+
+	__device__ __forceinline__ void load(const __nv_bfloat16* src)
 	{
-		const uint4 u = __ldg(s + i);
-		const uint32_t w[4] = { u.x, u.y, u.z, u.w };
+		const uint4* s = reinterpret_cast<const uint4*>(src);
 #pragma unroll
-		for (int j = 0; j < 4; j++)
+		for (int i = 0; i < 4; i++)
+			u[i] = __ldg(s + i);
+	}
+
+	// f(c, value) for each channel
+	template <typename F>
+	__device__ __forceinline__ void each(F f) const
+	{
+#pragma unroll
+		for (int i = 0; i < 4; i++)
 		{
-			const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-			const float2 f = __bfloat1622float2(h);
-			v[8 * i + 2 * j] = f.x;
-			v[8 * i + 2 * j + 1] = f.y;
+			const uint32_t w[4] = { u[i].x, u[i].y, u[i].z, u[i].w };
+#pragma unroll
+			for (int j = 0; j < 4; j++)
+			{
+				const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+				f(8 * i + 2 * j, t.x);
+				f(8 * i + 2 * j + 1, t.y);
+			}
 		}
 	}
-}
+};
 
 __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&v)[32])
 {
@@ -202,10 +217,47 @@ __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&
 	}
 }
 
-// CTA = CONV_PIPES pipelines, each with its own producer thread (warp p), MMA thread (warp
-// CONV_PIPES + p), four epilogue warps, CONV_STAGES stages and two tensor-memory accumulators of
-// 32 columns; all share the 27 weight taps.  Pipeline p of CTA c takes tiles c * CONV_PIPES + p,
-// then every gridDim.x * CONV_PIPES-th tile.
+// One block of the convolution: up to CONV_PLANES output planes z0 .. z0 + count - 1 of one row y and
+// one x tile.  The blocks of a mesh: x tiles fastest, then rows, so that the pipelines at work at one
+// time share most of their input rows in L2.
+struct conv_block
+{
+	int b, z0, count, y, x0;
+
+	__device__ __forceinline__ conv_block(long long i, const conv_params& p)
+	{
+		x0 = (int)(i % p.x_tiles) * SUR_TILE;
+		i /= p.x_tiles;
+		y = (int)(i % p.Y);
+		i /= p.Y;
+		z0 = (int)(i % p.z_blocks) * p.planes;
+		b = (int)(i / p.z_blocks);
+		count = min(p.planes, p.Z - z0);
+	}
+
+	// the input planes that exist
+	__device__ __forceinline__ int first_plane() const { return max(0, z0 - 1); }
+	__device__ __forceinline__ int last_plane(const conv_params& p) const { return min(p.Z - 1, z0 + count); }
+};
+
+// Two things bound the tensor cores here.  An M128 K16 MMA streams 4 KB of activations from shared
+// memory (32 cycles at 128 bytes a cycle) whatever its N, so with N = 32 (one tap, 16 cycles of math) the
+// pipe is busy at most 40 % of the time.  And an MMA that adds to the accumulator of the one before it
+// follows it by about 177 cycles, whatever N (measured at N = 32 and 96), so several chains must run at
+// once.  Hence:
+//  - an input row serves the three taps dz = -1, 0, +1 in one MMA of N = 96: a block keeps the
+//    accumulators of its output planes side by side in tensor memory (32 columns each), input plane z
+//    adds to the columns of planes z - 1, z and z + 1, and the weights of a (dy, dx) pair lie in shared
+//    memory in the order of those columns (dz = +1, 0, -1).  Per output plane that streams
+//    (count + 2) / count rows of A and three taps of B: 72 cycles at 4 planes against 120 with N = 32,
+//    for 48 of math, and loads 3 (count + 2) rows per block instead of 9 count;
+//  - CONV_PIPES pipelines with a block each share the CTA's weights; their accumulators (4 planes x 32
+//    columns each) fill the tensor memory.  A plane's accumulator is handed to the epilogue and back on
+//    its own barriers, so a pipeline's next block starts while its last planes are stored.
+// At 128^3, batch 1, the ten convolutions of a macro-step went from 1.85 to 1.41 ms (with N = 32, three
+// pipelines); one pipeline of 8-plane blocks took 2.38 ms.
+// Each pipeline has a producer thread (warp p), an MMA thread (warp CONV_PIPES + p) and four epilogue
+// warps, one per quadrant of the tensor memory's lanes.
 __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_constant__ CUtensorMap act,
 																	const __grid_constant__ CUtensorMap wmap,
 																	const __grid_constant__ conv_params p)
@@ -213,7 +265,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 	extern __shared__ __align__(1024) unsigned char conv_smem[];
 	unsigned char* base =
 		reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(conv_smem) + 1023) & ~uintptr_t(1023));
-	unsigned char* wsm = base; // 27 taps x [32 co][64 B]
+	unsigned char* wsm = base; // 9 (dy, dx) pairs x 3 dz (+1, 0, -1) x [32 co][64 B]
 	unsigned char* stages0 = base + W_BYTES;
 	uint64_t* bars0 = reinterpret_cast<uint64_t*>(stages0 + (size_t)CONV_PIPES * CONV_STAGES * A_STAGE_BYTES);
 	uint64_t* wbar = bars0 + CONV_PIPES * CONV_PIPE_BARS;
@@ -226,16 +278,11 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 		for (int q = 0; q < CONV_PIPES; q++)
 		{
 			uint64_t* b = bars0 + q * CONV_PIPE_BARS;
-			for (int s = 0; s < CONV_STAGES; s++)
-			{
-				mbar_init(b + s, 1);				// full
-				mbar_init(b + CONV_STAGES + s, 1);	// empty
-			}
-			mbar_init(b + 2 * CONV_STAGES, 1);		// accumulator 0 full
-			mbar_init(b + 2 * CONV_STAGES + 1, 1);	// accumulator 1 full
-			mbar_init(b + 2 * CONV_STAGES + 2, 128); // accumulator 0 empty
-			mbar_init(b + 2 * CONV_STAGES + 3, 128); // accumulator 1 empty
-			mbar_init(b + 2 * CONV_STAGES + 4, 1);	// drain
+			for (int s = 0; s < 2 * CONV_STAGES + CONV_PLANES; s++)
+				mbar_init(b + s, 1); // full, empty, accumulator full
+			for (int s = 0; s < CONV_PLANES; s++)
+				mbar_init(b + 2 * CONV_STAGES + CONV_PLANES + s, 4); // accumulator empty: its four epilogue warps
+			mbar_init(b + CONV_PIPE_BARS - 1, 1);					 // drain
 		}
 		mbar_init(wbar, 1);
 		*abort_flag = 0;
@@ -243,7 +290,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 	}
 	if (warp == CONV_PIPES)
 	{
-		tmem_alloc(tmem_slot, 256); // 2 accumulators of 32 columns per pipeline (192 used)
+		tmem_alloc(tmem_slot, 512);
 		tmem_relinquish();
 	}
 	tc_fence_before();
@@ -252,59 +299,49 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 	const uint32_t tmem = *tmem_slot;
 
 	// this thread's role and pipeline
-	int role, pipe;
-	if (warp < CONV_PIPES)
-	{
-		role = 0;
-		pipe = warp;
-	}
-	else if (warp < 2 * CONV_PIPES)
-	{
-		role = 1;
-		pipe = warp - CONV_PIPES;
-	}
-	else
-	{
-		role = 2;
-		pipe = (warp - 2 * CONV_PIPES) / 4;
-	}
-	uint64_t* bars = bars0 + pipe * CONV_PIPE_BARS;
-	uint64_t* full = bars;
-	uint64_t* empty = bars + CONV_STAGES;
-	uint64_t* acc_full = bars + 2 * CONV_STAGES;
-	uint64_t* acc_empty = acc_full + 2;
-	uint64_t* drain = acc_empty + 2;
+	const int role = warp < CONV_PIPES ? 0 : warp < 2 * CONV_PIPES ? 1 : 2;
+	const int pipe = role == 2 ? (warp - 2 * CONV_PIPES) / 4 : warp % CONV_PIPES;
+	uint64_t* full = bars0 + pipe * CONV_PIPE_BARS;
+	uint64_t* empty = full + CONV_STAGES;
+	uint64_t* acc_full = empty + CONV_STAGES;
+	uint64_t* acc_empty = acc_full + CONV_PLANES;
+	uint64_t* drain = acc_empty + CONV_PLANES;
 	unsigned char* stages = stages0 + (size_t)pipe * CONV_STAGES * A_STAGE_BYTES;
+	const uint32_t acc = tmem + (uint32_t)(pipe * CONV_PLANES * SUR_C);
 	const long long first = (long long)blockIdx.x * CONV_PIPES + pipe;
 	const long long stride = (long long)gridDim.x * CONV_PIPES;
-	const long long my_tiles = first < p.tiles ? (p.tiles - first + stride - 1) / stride : 0;
-	const uint32_t acc_col = tmem + (uint32_t)(pipe * 2 * SUR_C);
 
 	if (role == 0 && lane == 0)
 	{
-		// producer: the weights once (pipeline 0), then one 130-row box per (dy, dz) of each tile
+		// producer: the weights once (pipeline 0), then one 130-row box per input row of each block
 		if (pipe == 0)
 		{
 			mbar_expect_tx(wbar, W_BYTES);
 			for (int t = 0; t < SUR_TAPS; t++)
-				tma_load_2d(wsm + t * W_TAP_BYTES, &wmap, 0, t * SUR_C, wbar);
+				tma_load_2d(wsm + (t % 9 * 3 + 2 - t / 9) * W_TAP_BYTES, &wmap, 0, t * SUR_C, wbar);
 		}
 		long long n = 0;
-		for (long long i = 0; i < my_tiles && !aborted(abort_flag); i++)
+		bool ok = true;
+		for (long long i = first; ok && i < p.tiles && !aborted(abort_flag); i += stride)
 		{
-			int b, z, y, x0;
-			decode_tile(first + i * stride, p, b, z, y, x0);
-			for (int r = 0; r < 9; r++, n++)
-			{
-				const int s = (int)(n % CONV_STAGES);
-				if (!mbar_wait(empty + s, (uint32_t)(((n / CONV_STAGES) & 1) ^ 1)))
+			const conv_block k(i, p);
+			const int z1 = k.last_plane(p);
+			for (int z = k.first_plane(); ok && z <= z1; z++)
+				for (int dy = -1; dy <= 1; dy++)
 				{
-					give_up(abort_flag, p.err);
-					break;
+					if (k.y + dy < 0 || k.y + dy >= p.Y)
+						continue;
+					const int s = (int)(n % CONV_STAGES);
+					if (!mbar_wait(empty + s, (uint32_t)(((n / CONV_STAGES) & 1) ^ 1)))
+					{
+						give_up(abort_flag, p.err);
+						ok = false;
+						break;
+					}
+					mbar_expect_tx(full + s, A_BOX_BYTES);
+					tma_load_5d(stages + s * A_STAGE_BYTES, &act, 0, k.x0 - 1, k.y + dy, z, k.b, full + s);
+					n++;
 				}
-				mbar_expect_tx(full + s, A_BOX_BYTES);
-				tma_load_5d(stages + s * A_STAGE_BYTES, &act, 0, x0 - 1, y + r % 3 - 1, z + r / 3 - 1, b, full + s);
-			}
 		}
 		// the copies issued last land before the CTA exits
 		for (long long k = (n > CONV_STAGES ? n - CONV_STAGES : 0); k < n; k++)
@@ -314,48 +351,80 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 	}
 	else if (role == 1 && lane == 0)
 	{
-		// MMA issuer: per box, taps dx = -1, 0, +1 from rows 0, 1, 2 of the box; two K steps of 16
-		// channels (32 bytes) each
-		constexpr uint32_t idesc = idesc_bf16(SUR_TILE, SUR_C, false, false);
+		// MMA issuer: per input row, taps dx = -1, 0, +1 from rows 0, 1, 2 of the box, two K steps of 16
+		// channels (32 bytes) each, N = 32 x the output planes that the row's plane reaches
 		bool ok = mbar_wait(wbar, 0);
 		if (!ok)
 			give_up(abort_flag, p.err);
 		tc_fence_after();
 		long long n = 0;
-		for (long long i = 0; ok && i < my_tiles && !aborted(abort_flag); i++)
+		uint32_t phase = (1u << CONV_PLANES) - 1; // of the accumulators' empty barriers: free at first
+		for (long long blk = first; ok && blk < p.tiles && !aborted(abort_flag); blk += stride)
 		{
-			const int a = (int)(i & 1);
-			if (!mbar_wait(acc_empty + a, (uint32_t)(((i >> 1) & 1) ^ 1)))
+			const conv_block k(blk, p);
+			const int z1 = k.last_plane(p);
+			int written = 0; // output planes whose accumulators hold a product
+			for (int z = k.first_plane(); ok && z <= z1; z++)
 			{
-				give_up(abort_flag, p.err);
-				break;
-			}
-			tc_fence_after();
-			const uint32_t d = acc_col + (uint32_t)(a * SUR_C);
-			for (int r = 0; r < 9; r++, n++)
-			{
-				const int s = (int)(n % CONV_STAGES);
-				if (!mbar_wait(full + s, (uint32_t)((n / CONV_STAGES) & 1)))
+				const int lo = max(0, z - 1 - k.z0), hi = min(k.count - 1, z + 1 - k.z0);
+				const uint32_t w0 = smem_addr(wsm) + (uint32_t)(1 - (z - k.z0 - lo)) * W_TAP_BYTES;
+				const uint32_t d = acc + (uint32_t)(lo * SUR_C);
+				// the accumulators that this plane starts have been read
+				for (int o = max(written, lo); ok && o <= hi; o++)
+				{
+					ok = mbar_wait(acc_empty + o, (phase >> o) & 1);
+					phase ^= 1u << o;
+				}
+				if (!ok)
 				{
 					give_up(abort_flag, p.err);
-					ok = false;
 					break;
 				}
-				tc_fence_after();
-				const uint32_t a_addr = smem_addr(stages + s * A_STAGE_BYTES);
-#pragma unroll
-				for (int dx = 0; dx < 3; dx++)
+				for (int dy = -1; dy <= 1; dy++)
 				{
-					const uint32_t b_addr = smem_addr(wsm + (3 * r + dx) * W_TAP_BYTES);
+					if (k.y + dy < 0 || k.y + dy >= p.Y)
+						continue;
+					const int s = (int)(n % CONV_STAGES);
+					if (!mbar_wait(full + s, (uint32_t)((n / CONV_STAGES) & 1)))
+					{
+						give_up(abort_flag, p.err);
+						ok = false;
+						break;
+					}
+					tc_fence_after();
+					const uint32_t a_addr = smem_addr(stages + s * A_STAGE_BYTES);
 #pragma unroll
-					for (int k = 0; k < 2; k++)
-						umma_bf16(d, sw64_desc(a_addr + 64 * dx + 32 * k, 16, 512), sw64_desc(b_addr + 32 * k, 16, 512),
-								  idesc, (r | dx | k) != 0);
+					for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+						for (int h = 0; h < 2; h++)
+						{
+							const uint64_t ad = sw64_desc(a_addr + 64 * dx + 32 * h, 16, 512);
+							const uint32_t b_addr = w0 + (uint32_t)(((dy + 1) * 3 + dx) * 3) * W_TAP_BYTES + 32 * h;
+							if (written > hi)
+							{
+								umma_bf16(d, ad, sw64_desc(b_addr, 16, 512), idesc_bf16(SUR_TILE, SUR_C * (hi - lo + 1), false, false), 1);
+								continue;
+							}
+							// the plane's first products: its new accumulators are overwritten
+							if (written > lo)
+								umma_bf16(d, ad, sw64_desc(b_addr, 16, 512),
+										  idesc_bf16(SUR_TILE, SUR_C * (written - lo), false, false), 1);
+							const int fresh = max(written, lo);
+							umma_bf16(acc + (uint32_t)(fresh * SUR_C), ad, sw64_desc(b_addr + (uint32_t)(fresh - lo) * W_TAP_BYTES, 16, 512),
+									  idesc_bf16(SUR_TILE, SUR_C * (hi - fresh + 1), false, false), 0);
+							written = hi + 1;
+						}
+					umma_commit(empty + s); // the stage is free once these MMAs have read it
+					n++;
 				}
-				umma_commit(empty + s); // the stage is free once these MMAs have read it
+				if (!ok)
+					break;
+				// plane z - 1 is complete, and plane z too at the mesh's last plane
+				if (z > k.z0)
+					umma_commit(acc_full + z - 1 - k.z0);
+				if (z == p.Z - 1 && z < k.z0 + k.count)
+					umma_commit(acc_full + z - k.z0);
 			}
-			if (ok)
-				umma_commit(acc_full + a);
 		}
 		// every MMA has completed before the tensor memory is freed
 		umma_commit(drain);
@@ -363,67 +432,70 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 	}
 	else if (role == 2)
 	{
-		// epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. +31, i.e. voxels x0 + 32 (w % 4) + lane
+		// epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. +31, i.e. voxels x0 + 32 (w % 4) + lane;
+		// the residual (or the mask, where that is alone) is loaded before it waits for the accumulator
 		const int q = warp & 3;
 		const int m = q * 32 + lane;
-		for (long long i = 0; i < my_tiles; i++)
+		uint32_t phase = 0; // of the accumulators' full barriers
+		bool ok = true;
+		for (long long blk = first; ok && blk < p.tiles && !aborted(abort_flag); blk += stride)
 		{
-			if (aborted(abort_flag))
-				break;
-			const int a = (int)(i & 1);
-			if (!mbar_wait(acc_full + a, (uint32_t)((i >> 1) & 1)))
+			const conv_block k(blk, p);
+			const int x = k.x0 + m;
+			for (int o = 0; o < k.count; o++)
 			{
-				give_up(abort_flag, p.err);
-				break;
-			}
-			tc_fence_after();
-			float v[32];
-			tmem_ld32(acc_col + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * SUR_C), v);
-			tc_fence_before();
-			mbar_arrive(acc_empty + a);
-
-			int b, z, y, x0;
-			decode_tile(first + i * stride, p, b, z, y, x0);
-			const int x = x0 + m;
-			if (x >= p.X)
-				continue;
-			const long long vox = (((long long)b * p.Z + z) * p.Y + y) * p.X + x;
-			if (p.bias)
-			{
+				const long long vox = (((long long)k.b * p.Z + k.z0 + o) * p.Y + k.y) * p.X + x;
+				bf16x32 ahead;
+				const __nv_bfloat16* from = p.residual ? p.residual : p.mask;
+				if (from && x < p.X)
+					ahead.load(from + vox * SUR_C);
+				if (!mbar_wait(acc_full + o, (phase >> o) & 1))
+				{
+					give_up(abort_flag, p.err);
+					ok = false;
+					break;
+				}
+				phase ^= 1u << o;
+				tc_fence_after();
+				float v[32];
+				tmem_ld32(acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(o * SUR_C), v);
+				tc_fence_before();
+				__syncwarp();
+				if (lane == 0)
+					mbar_arrive(acc_empty + o);
+				if (x >= p.X)
+					continue;
+				if (p.bias)
+				{
 #pragma unroll
-				for (int c = 0; c < 32; c++)
-					v[c] += __ldg(&p.bias[c]);
-			}
-			if (p.residual)
-			{
-				float r[32];
-				load_bf16x32(p.residual + vox * SUR_C, r);
+					for (int c = 0; c < 32; c++)
+						v[c] += __ldg(&p.bias[c]);
+				}
+				if (p.residual)
+				{
+					ahead.each([&](int c, float r) { v[c] += r; });
+				}
+				if (p.relu)
+				{
 #pragma unroll
-				for (int c = 0; c < 32; c++)
-					v[c] += r[c];
-			}
-			if (p.relu)
-			{
+					for (int c = 0; c < 32; c++)
+						v[c] = fmaxf(v[c], 0.f);
+				}
+				if (p.mask)
+				{
+					if (p.residual)
+						ahead.load(p.mask + vox * SUR_C);
+					ahead.each([&](int c, float r) { v[c] = r > 0.f ? v[c] : 0.f; });
+				}
+				if (p.out)
+					store_bf16x32(p.out + vox * SUR_C, v);
+				if (p.out_f32)
+				{
 #pragma unroll
-				for (int c = 0; c < 32; c++)
-					v[c] = fmaxf(v[c], 0.f);
-			}
-			if (p.mask)
-			{
-				float r[32];
-				load_bf16x32(p.mask + vox * SUR_C, r);
-#pragma unroll
-				for (int c = 0; c < 32; c++)
-					v[c] = r[c] > 0.f ? v[c] : 0.f;
-			}
-			if (p.out)
-				store_bf16x32(p.out + vox * SUR_C, v);
-			if (p.out_f32)
-			{
-#pragma unroll
-				for (int c = 0; c < 32; c++)
-					if (c < p.out_ch)
-						p.out_f32[vox * p.out_ch + c] = v[c] + (p.base_f32 ? p.base_f32[vox * p.out_ch + c] : 0.f);
+					for (int c = 0; c < 32; c++)
+						if (c < p.out_ch)
+							p.out_f32[vox * p.out_ch + c] = v[c] + (p.base_f32 ? p.base_f32[vox * p.out_ch + c] : 0.f);
+				}
 			}
 		}
 	}
@@ -432,7 +504,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) sur_conv_kernel(const __grid_
 	if (warp == CONV_PIPES)
 	{
 		tc_fence_after();
-		tmem_dealloc(tmem, 256);
+		tmem_dealloc(tmem, 512);
 	}
 }
 
@@ -666,11 +738,26 @@ int launch_sur_conv(const __nv_bfloat16* in, const __nv_bfloat16* w, conv_params
 	if (!encode_act_map(&act, in, p.X, p.Y, p.Z, p.B, CONV_ROWS) || !encode_weight_map(&wmap, w))
 		return fail(BFVM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a surrogate tensor");
 	p.x_tiles = (p.X + SUR_TILE - 1) / SUR_TILE;
-	p.tiles = (long long)p.x_tiles * p.Y * p.Z * p.B;
+	// The planes of a block: deeper blocks stream fewer rows per output plane, shallower ones leave less
+	// of the last wave idle.  A block of c planes streams 32 (c + 2) + 24 c cycles of operands per tap
+	// pair and K step (sur_conv_kernel); the depth with the fewest cycles over all waves is taken.
+	const long long sms = sm_count_impl(device), pipes = sms * CONV_PIPES;
+	long long best = 0;
+	for (int c = 1; c <= std::min(CONV_PLANES, p.Z); c++)
+	{
+		const long long blocks = (long long)p.x_tiles * p.Y * p.B * ((p.Z + c - 1) / c);
+		const long long cycles = (blocks + pipes - 1) / pipes * (56 * c + 64);
+		if (best == 0 || cycles <= best)
+		{
+			best = cycles;
+			p.planes = c;
+		}
+	}
+	p.z_blocks = (p.Z + p.planes - 1) / p.planes;
+	p.tiles = (long long)p.x_tiles * p.Y * p.B * p.z_blocks;
 	if ((st = set_smem(sur_conv_kernel, CONV_SMEM)))
 		return st;
-	const long long grid =
-		std::min<long long>((p.tiles + CONV_PIPES - 1) / CONV_PIPES, (long long)sm_count_impl(device));
+	const long long grid = std::min<long long>((p.tiles + CONV_PIPES - 1) / CONV_PIPES, sms);
 	sur_conv_kernel<<<(unsigned)std::max(1LL, grid), CONV_THREADS, CONV_SMEM, stream>>>(act, wmap, p);
 	const cudaError_t e = cudaGetLastError();
 	return e == cudaSuccess ? BFVM_OK : cuda_fail(e, "sur_conv_kernel");

@@ -17,6 +17,7 @@ struct conv_params
 {
 	int X, Y, Z, B;
 	int x_tiles;	// set by the launcher
+	int planes, z_blocks; // output planes of a convolution's block, blocks along z (set by the launcher)
 	long long tiles; // set by the launcher
 	const float* bias;				// [32] added first, or null
 	const __nv_bfloat16* residual;	// [voxels][32] added next, or null
