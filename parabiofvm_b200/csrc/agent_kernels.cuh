@@ -46,6 +46,27 @@ __global__ void secrete_kernel(long long total, int S, float* __restrict__ dens,
 							   const float* __restrict__ red_fac, float* __restrict__ intern, int internalized,
 							   float voxel_volume);
 
+// The voxel of an agent; false outside the mesh.
+__device__ __forceinline__ bool voxel_of(const float* pos, int dims, int3 bmin, int3 vox, int3 grid, int3& c)
+{
+	// truncating (pos - min) / dx as in src/mesh.cpp:35-53; positions in (-dx, 0) truncate to 0 there
+	// too.  Anything outside the mesh is rejected instead of indexing out of bounds.
+	c = make_int3(0, 0, 0);
+	const int bm[3] = { bmin.x, bmin.y, bmin.z };
+	const int vx[3] = { vox.x, vox.y, vox.z };
+	const int gr[3] = { grid.x, grid.y, grid.z };
+	int out[3] = { 0, 0, 0 };
+	for (int d = 0; d < dims; d++)
+	{
+		const float t = __fdiv_rn(__fsub_rn(pos[d], (float)bm[d]), (float)vx[d]);
+		if (!(t > -1.0f && t < (float)gr[d]))
+			return false;
+		out[d] = (int)t;
+	}
+	c = make_int3(out[0], out[1], out[2]);
+	return true;
+}
+
 // One (voxel segment, substrate) pair of the secretion update; t < segments * S (secrete_kernel of
 // cell.cu, and the ensemble update of batch_kernels.cu).  See cell.cu for the formulas.  SORTED:
 // the per-agent rows num/den/fac/intern are in the binning's sorted order (row p is the agent at
@@ -165,9 +186,10 @@ __device__ __forceinline__ void secrete_sorted4_element(long long t, int S, floa
 __global__ void __launch_bounds__(SCAN_THREADS) scan_tile_kernel(const int* in, int* out, long long n, int* tile_sums);
 __global__ void scan_add_kernel(int* out, long long n, const int* tile_offsets);
 
-// cell.cu: keys, sort, segments, intermediates, reductions; `sorted`: also the sorted copies of the
-// per-agent terms (agent_state::snum ...), from which the reductions are then summed
-int rebuild_bins(bfvm_solver* s, bool sorted = false);
+// bins.cu: the agents' order by voxel (agent_state::keys, vals) and its segments, on the solver's
+// stream; the buffers this needs for `count` agents
+int launch_bins(bfvm_solver* s);
+int bins_alloc(bfvm_solver* s, int count);
 
 // number of 8-bit radix passes for keys in [0, V] (V marks agents outside the mesh)
 inline int sort_passes(long long V)

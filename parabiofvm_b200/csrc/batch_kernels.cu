@@ -835,9 +835,9 @@ int ensemble_build(ensemble_plan& plan, const std::vector<bfvm_solver*>& meshes,
 		const bool sorted = a.count > 0 && (rebinned ? s->internalized : a.sorted);
 		m.sorted = sorted ? 1 : 0;
 		m.vec4 = sorted && s->S % 4 == 0 ? 1 : 0;
-		m.num = sorted ? a.snum : a.num;
-		m.den = sorted ? a.sden : a.den;
-		m.fac = sorted ? a.sfac : a.fac;
+		m.num = a.num;
+		m.den = a.den;
+		m.fac = a.fac;
 		m.red_num = a.red_num;
 		m.red_den = a.red_den;
 		m.red_fac = a.red_fac;

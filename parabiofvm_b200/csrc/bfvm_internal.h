@@ -82,13 +82,6 @@ struct sweep_plan
 	} chunks;
 };
 
-// Radix-sort / scan scratch for the agent binning.
-struct scan_plan
-{
-	std::vector<long long> level_sizes; // element count at each level
-	std::vector<int*> level_sums;		// block sums per level (device)
-};
-
 // A Dirichlet overwrite list grouped by the tiles of one axis's staged sweep (dirichlet.cu): the
 // runs of four and single elements of tile w are [qoff[w], qoff[w + 1]) and [soff[w], soff[w + 1]).
 struct dirichlet_tiles
@@ -124,24 +117,20 @@ struct agent_state
 	// binning (rebuilt on recompute)
 	unsigned int *keys = nullptr, *keys_alt = nullptr;
 	int *vals = nullptr, *vals_alt = nullptr;
-	int* hist = nullptr;		 // [256][tiles]
-	int* flags = nullptr;		 // [A]
-	int* seg_id = nullptr;		 // [A]
+	unsigned char* bin_state = nullptr; // scratch of the multi-CTA binning (bins.cu); its first int is set when it gave up
+	size_t bin_state_bytes = 0;
 	int* seg_start = nullptr;	 // [A+1]
 	int* seg_count_dev = nullptr; // [2]: number of segments, number of valid agents
-	float *num = nullptr, *den = nullptr, *fac = nullptr;			 // [A][S]
+	float *num = nullptr, *den = nullptr, *fac = nullptr;			 // [A][S] in the sorted order
 	float *red_num = nullptr, *red_den = nullptr, *red_fac = nullptr; // [A][S] by segment
-	int tiles = 0;
-	scan_plan hist_scan, flag_scan;
 	bool binned = false;		 // a recompute has run since the last store
 
-	// A solver stepping alone with internalized substrates keeps its per-agent terms in the
-	// binning's sorted order (cell.cu): row p of snum/sden/sfac/sintern is row vals[p] of
-	// num/den/fac/intern, and rank[i] is agent i's row there, so the per-step update reads and
-	// writes contiguous rows.  While `sorted` is set, sintern holds the internalized amounts and
-	// intern is only a copy, refreshed when they are loaded.
-	float *snum = nullptr, *sden = nullptr, *sfac = nullptr, *sintern = nullptr; // [A][S] sorted
-	int* rank = nullptr;																// [A]
+	// Row p of num/den/fac is agent vals[p]'s.  With internalized substrates so is row p of sintern, so
+	// the per-step update reads and writes contiguous rows, and rank[i] is agent i's row there.  While
+	// `sorted` is set, sintern holds the internalized amounts and intern is only a copy, refreshed when
+	// they are loaded.
+	float* sintern = nullptr; // [A][S] sorted
+	int* rank = nullptr;	  // [A]
 	bool sorted = false;
 
 	int* move_idx = nullptr; // [2][moves]: destinations, then sources of bfvm_remove_agents
@@ -347,11 +336,6 @@ int launch_release(bfvm_solver* s, int index);
 // storage for `count` agents keeping the stored rows; the moves dst[k] <- src[k] of every agent row
 int cell_grow(bfvm_solver* s, int count);
 int launch_agent_moves(bfvm_solver* s, const std::vector<int>& dst, const std::vector<int>& src);
-
-// scan.cu
-int scan_plan_build(scan_plan& p, long long n);
-void scan_plan_free(scan_plan& p);
-int launch_exclusive_scan(bfvm_solver* s, scan_plan& p, const int* in, int* out, long long n);
 
 template <typename T>
 int device_alloc(T** ptr, size_t count)

@@ -1,0 +1,624 @@
+// Binning of the agents into voxels (recompute steps): agents ordered by voxel, agents of one voxel
+// by index, and the segments of the order that share a voxel.
+//
+// The order is a stable LSD radix sort of (voxel key, agent index); agents outside the mesh carry the
+// key V and sort to the end.  Two forms:
+//  - up to BIN_BLOCK_AGENTS agents, one CTA does all of it (keys, sort, segments) in shared memory: a
+//    launch costs more than its share of the work there, and the multi-CTA form needs 3 + passes of them;
+//  - beyond that, a kernel computes the keys and the digit histograms of every pass, one kernel per
+//    digit ranks and scatters (single-pass radix sort with decoupled look-back, after Adinets and
+//    Merrill, "Onesweep", 2022), and one finds the segments with the same look-back.
+// The sort was three or more launches per digit (histogram, scan, scatter) and five for the segments, 22 to
+// 28 in all.  One step with rebinning at 100^3 x 4 with 50,000 agents: 200 -> 145 us; ten steps (one
+// rebinning) at 50^3 x 4 with 5,000: 616 -> 571 us, at 128^3 x 4 with 200,000: 1179 -> 1109 us.
+// CTAs of the look-back kernels take their tiles from a counter, so a tile only ever waits for tiles
+// whose CTAs already run; the waits are bounded, and one that runs out raises DEVERR_TIMEOUT and the
+// scratch's abort word, after which the remaining kernels leave at once with no segments.  What is left
+// in keys and vals then are valid indices of some order (vals starts zeroed), so nothing indexes out of
+// the agents' arrays.
+
+#include <algorithm>
+
+#include "agent_kernels.cuh"
+#include "sm100_common.cuh"
+#include "sweep_common.cuh"
+
+namespace bfvm {
+
+static constexpr int BIN_BLOCK_AGENTS = 16384;
+static constexpr int BLOCK_THREADS = 1024;
+static constexpr int BLOCK_WARPS = BLOCK_THREADS / 32;
+static constexpr int BLOCK_ITEMS = BIN_BLOCK_AGENTS / BLOCK_THREADS;
+
+// ------------------------------------------------------------------------------------------------
+// one CTA
+
+struct bin_job
+{
+	const float* pos;
+	unsigned int* keys;
+	int* vals;
+	int* seg_start;
+	int* counts;
+	int* err;
+	int A, dims;
+	int3 bmin, vox, grid;
+	unsigned int invalid; // key of an agent outside the mesh
+	int passes, bits;	  // radix passes and bits per pass (at most 8)
+};
+
+static size_t block_smem(int A)
+{
+	const size_t rounds = (A + BLOCK_THREADS - 1) / BLOCK_THREADS;
+	return rounds * BLOCK_THREADS * (sizeof(unsigned int) + sizeof(unsigned short)) + BLOCK_WARPS * 256 * sizeof(unsigned short);
+}
+
+// Warp w holds agents (sorted positions) w * 32 * rounds + 32 r + lane for r < rounds, so the rounds of
+// a warp and then the warps follow the order, which makes the ranks stable.
+__global__ void __launch_bounds__(BLOCK_THREADS, 1) bin_block_kernel(const __grid_constant__ bin_job j)
+{
+	extern __shared__ __align__(16) unsigned char bin_smem[];
+	__shared__ int tot[256];
+	__shared__ int wsum[BLOCK_WARPS], wvalid[BLOCK_WARPS];
+	const int rounds = (j.A + BLOCK_THREADS - 1) / BLOCK_THREADS;
+	unsigned int* skey = reinterpret_cast<unsigned int*>(bin_smem);
+	unsigned short* cnt = reinterpret_cast<unsigned short*>(skey + rounds * BLOCK_THREADS); // [warps][256]
+	unsigned short* sval = cnt + BLOCK_WARPS * 256;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const int base = warp * 32 * rounds + lane;
+	const unsigned int below = (1u << lane) - 1u;
+
+	unsigned int key[BLOCK_ITEMS];
+	unsigned int vr[BLOCK_ITEMS]; // agent index << 16 | rank
+	bool outside = false;
+#pragma unroll
+	for (int r = 0; r < BLOCK_ITEMS; r++)
+		if (r < rounds)
+		{
+			const int i = base + 32 * r;
+			key[r] = j.invalid;
+			vr[r] = (unsigned int)i << 16;
+			int3 c;
+			if (i < j.A)
+			{
+				if (voxel_of(j.pos + (size_t)i * j.dims, j.dims, j.bmin, j.vox, j.grid, c))
+					key[r] = (unsigned int)c.x
+							 + (unsigned int)j.grid.x * ((unsigned int)c.y + (unsigned int)j.grid.y * (unsigned int)c.z);
+				else
+					outside = true;
+			}
+		}
+	if (outside)
+		atomicOr(j.err, DEVERR_AGENT_OUTSIDE);
+
+	// positions past A carry the key of agents outside the mesh and the largest indices: they sort last
+	const unsigned int mask = (1u << j.bits) - 1u;
+	for (int pass = 0; pass < j.passes; pass++)
+	{
+		const int shift = pass * j.bits;
+		for (int t = tid; t < BLOCK_WARPS * 128; t += BLOCK_THREADS)
+			reinterpret_cast<unsigned int*>(cnt)[t] = 0;
+		__syncthreads();
+		unsigned short* wc = cnt + warp * 256;
+#pragma unroll
+		for (int r = 0; r < BLOCK_ITEMS; r++)
+			if (r < rounds)
+			{
+				const unsigned int d = (key[r] >> shift) & mask;
+				const unsigned int peers = __match_any_sync(0xffffffffu, d);
+				const unsigned int before = wc[d];
+				__syncwarp();
+				if ((peers & below) == 0)
+					wc[d] = (unsigned short)(before + __popc(peers));
+				__syncwarp();
+				vr[r] = (vr[r] & 0xffff0000u) | (before + __popc(peers & below));
+			}
+		__syncthreads();
+		// exclusive offsets of (digit, warp): four threads a digit, eight warps each
+		{
+			const int d = tid >> 2, part = tid & 3;
+			int own = 0;
+#pragma unroll
+			for (int w = 0; w < BLOCK_WARPS / 4; w++)
+				own += cnt[(part * (BLOCK_WARPS / 4) + w) * 256 + d];
+			int incl = own;
+#pragma unroll
+			for (int o = 1; o < 4; o <<= 1)
+			{
+				const int up = __shfl_up_sync(0xffffffffu, incl, o, 4);
+				if (part >= o)
+					incl += up;
+			}
+			if (part == 3)
+				tot[d] = incl;
+			__syncthreads();
+			if (warp == 0)
+			{
+				int v[8], sum = 0;
+#pragma unroll
+				for (int k = 0; k < 8; k++)
+				{
+					v[k] = sum;
+					sum += tot[lane * 8 + k];
+				}
+				int run = sum;
+#pragma unroll
+				for (int o = 1; o < 32; o <<= 1)
+				{
+					const int up = __shfl_up_sync(0xffffffffu, run, o);
+					if (lane >= o)
+						run += up;
+				}
+#pragma unroll
+				for (int k = 0; k < 8; k++)
+					tot[lane * 8 + k] = run - sum + v[k];
+			}
+			__syncthreads();
+			int run = tot[d] + incl - own;
+#pragma unroll
+			for (int w = 0; w < BLOCK_WARPS / 4; w++)
+			{
+				unsigned short* c = cnt + (part * (BLOCK_WARPS / 4) + w) * 256 + d;
+				const int n = *c;
+				*c = (unsigned short)run;
+				run += n;
+			}
+		}
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < BLOCK_ITEMS; r++)
+			if (r < rounds)
+			{
+				const int at = wc[(key[r] >> shift) & mask] + (int)(vr[r] & 0xffffu);
+				skey[at] = key[r];
+				sval[at] = (unsigned short)(vr[r] >> 16);
+			}
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < BLOCK_ITEMS; r++)
+			if (r < rounds)
+			{
+				key[r] = skey[base + 32 * r];
+				vr[r] = (unsigned int)sval[base + 32 * r] << 16;
+			}
+	}
+
+	// segments: a position starts one when its key differs from the previous position's
+	int heads = 0, valid = 0;
+#pragma unroll
+	for (int r = 0; r < BLOCK_ITEMS; r++)
+		if (r < rounds)
+		{
+			const int p = base + 32 * r;
+			const bool in = key[r] != j.invalid;
+			const bool head = in && (p == 0 || skey[p - 1] != key[r]);
+			const unsigned int hb = __ballot_sync(0xffffffffu, head);
+			// segments that start before this position in the warp, and whether one starts here
+			vr[r] = (vr[r] & 0xffff0000u) | ((unsigned int)(heads + __popc(hb & below)) << 1) | (head ? 1u : 0u);
+			heads += __popc(hb);
+			valid += __popc(__ballot_sync(0xffffffffu, in));
+		}
+	if (lane == 0)
+	{
+		wsum[warp] = heads;
+		wvalid[warp] = valid;
+	}
+	__syncthreads();
+	int ahead = 0, segments = 0, agents = 0;
+	for (int w = 0; w < BLOCK_WARPS; w++)
+	{
+		if (w == warp)
+			ahead = segments;
+		segments += wsum[w];
+		agents += wvalid[w];
+	}
+#pragma unroll
+	for (int r = 0; r < BLOCK_ITEMS; r++)
+		if (r < rounds)
+		{
+			const int p = base + 32 * r;
+			if (p < j.A)
+			{
+				j.keys[p] = key[r];
+				j.vals[p] = (int)(vr[r] >> 16);
+				if (vr[r] & 1u)
+					j.seg_start[ahead + (int)((vr[r] & 0xffffu) >> 1)] = p;
+			}
+		}
+	if (tid == 0)
+	{
+		j.counts[0] = segments;
+		j.counts[1] = agents;
+		j.counts[2] = agents > segments ? 1 : 0;
+		j.seg_start[segments] = agents;
+	}
+}
+
+// ------------------------------------------------------------------------------------------------
+// many CTAs
+
+static constexpr int PASS_THREADS = 512;
+static constexpr int PASS_WARPS = PASS_THREADS / 32;
+static constexpr int MAX_PASSES = 4;
+// a tile's published count: a state in the high word, the count in the low
+static constexpr unsigned long long TILE_SUM = 1ull << 32;	 // of the tile alone
+static constexpr unsigned long long TILE_TOTAL = 2ull << 32; // of the tile and all before it
+
+// scratch of the multi-CTA form, zeroed before each binning
+struct bin_state
+{
+	int abort;
+	int ticket[MAX_PASSES + 1];
+	int hist[MAX_PASSES][256];
+};
+
+__device__ __forceinline__ unsigned long long tile_load(const unsigned long long* p)
+{
+	return *reinterpret_cast<const volatile unsigned long long*>(p);
+}
+
+__device__ __forceinline__ void tile_publish(unsigned long long* p, unsigned long long v)
+{
+	*reinterpret_cast<volatile unsigned long long*>(p) = v;
+}
+
+// The counts of the tiles before `tile`: state of tile t at state[t * stride], read LOOK tiles at a time
+// so that their latencies overlap.  False when a wait ran out or the binning was aborted.
+__device__ __forceinline__ bool look_back(const unsigned long long* state, long long stride, int tile,
+										  const volatile int* abort_word, int& sum)
+{
+	constexpr int LOOK = 8;
+	sum = 0;
+	const long long t0 = clock64();
+	int t = tile - 1;
+	while (t >= 0)
+	{
+		unsigned long long v[LOOK];
+#pragma unroll
+		for (int k = 0; k < LOOK; k++)
+			v[k] = t - k >= 0 ? tile_load(state + (t - k) * stride) : TILE_TOTAL;
+#pragma unroll
+		for (int k = 0; k < LOOK; k++)
+		{
+			if ((v[k] >> 32) == 0)
+				break;
+			sum += (int)(unsigned int)v[k];
+			t--;
+			if (v[k] & TILE_TOTAL)
+				return true;
+		}
+		if (clock64() - t0 > WAIT_LIMIT_CYCLES || *abort_word)
+			return false;
+	}
+	return true;
+}
+
+// keys of the agents, and the digit histograms of every pass
+__global__ void __launch_bounds__(PASS_THREADS) bin_keys_kernel(const float* __restrict__ pos, int A, int dims, int3 bmin,
+																 int3 vox, int3 grid, unsigned int* __restrict__ keys,
+																 unsigned int invalid, int passes, int bits,
+																 bin_state* __restrict__ st, int* __restrict__ err)
+{
+	__shared__ int h[MAX_PASSES][256];
+	for (int t = threadIdx.x; t < MAX_PASSES * 256; t += PASS_THREADS)
+		h[t >> 8][t & 255] = 0;
+	__syncthreads();
+	const unsigned int mask = (1u << bits) - 1u;
+	bool outside = false;
+	for (long long i = blockIdx.x * (long long)PASS_THREADS + threadIdx.x; i < A; i += (long long)gridDim.x * PASS_THREADS)
+	{
+		int3 c;
+		unsigned int k = invalid;
+		if (voxel_of(pos + (size_t)i * dims, dims, bmin, vox, grid, c))
+			k = (unsigned int)c.x + (unsigned int)grid.x * ((unsigned int)c.y + (unsigned int)grid.y * (unsigned int)c.z);
+		else
+			outside = true;
+		keys[i] = k;
+		for (int p = 0; p < passes; p++)
+			atomicAdd(&h[p][(k >> (p * bits)) & mask], 1);
+	}
+	if (outside)
+		atomicOr(err, DEVERR_AGENT_OUTSIDE);
+	__syncthreads();
+	for (int t = threadIdx.x; t < passes * 256; t += PASS_THREADS)
+	{
+		const int n = h[t >> 8][t & 255];
+		if (n)
+			atomicAdd(&st->hist[t >> 8][t & 255], n);
+	}
+}
+
+// One digit: a tile of PASS_THREADS * ITEMS keys is ranked within the CTA, its digit counts are joined
+// with those of the tiles before it, and its keys go to their places.  vin null: agent indices (the
+// first pass).
+template <int ITEMS>
+__global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned int* __restrict__ kin,
+																 const int* __restrict__ vin,
+																 unsigned int* __restrict__ kout, int* __restrict__ vout,
+																 int n, int pass, int bits, bin_state* st,
+																 unsigned long long* state, int* __restrict__ err)
+{
+	__shared__ int cnt[PASS_WARPS][256];
+	__shared__ int place[256]; // where the tile's first key of a digit goes
+	__shared__ int wtot[8];
+	__shared__ int tile_s, stop;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	if (tid == 0)
+	{
+		tile_s = atomicAdd(&st->ticket[pass], 1);
+		stop = *reinterpret_cast<volatile int*>(&st->abort);
+	}
+	for (int t = tid; t < PASS_WARPS * 256; t += PASS_THREADS)
+		cnt[t >> 8][t & 255] = 0;
+	__syncthreads();
+	if (stop)
+		return;
+	const int tile = tile_s;
+	const long long base = (long long)tile * (PASS_THREADS * ITEMS) + warp * 32 * ITEMS + lane;
+	const int shift = pass * bits;
+	const unsigned int mask = (1u << bits) - 1u, below = (1u << lane) - 1u;
+	unsigned int key[ITEMS];
+	int val[ITEMS], rank[ITEMS];
+#pragma unroll
+	for (int r = 0; r < ITEMS; r++)
+	{
+		const long long i = base + 32 * r;
+		key[r] = i < n ? kin[i] : 0u;
+		val[r] = i >= n ? 0 : vin ? vin[i] : (int)i;
+	}
+#pragma unroll
+	for (int r = 0; r < ITEMS; r++)
+	{
+		const bool in = base + 32 * r < n;
+		const unsigned int d = (key[r] >> shift) & mask;
+		const unsigned int peers = __match_any_sync(0xffffffffu, in ? d : 256u);
+		const int before = cnt[warp][d];
+		__syncwarp();
+		if (in && (peers & below) == 0)
+			cnt[warp][d] = before + __popc(peers);
+		__syncwarp();
+		rank[r] = before + __popc(peers & below);
+	}
+	__syncthreads();
+	int total = 0, gincl = 0, gown = 0;
+	if (tid < 256)
+	{
+#pragma unroll
+		for (int w = 0; w < PASS_WARPS; w++)
+		{
+			const int c = cnt[w][tid];
+			cnt[w][tid] = total;
+			total += c;
+		}
+		tile_publish(state + (long long)tile * 256 + tid, (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total);
+		// keys of smaller digits: exclusive scan of the pass's histogram
+		gown = st->hist[pass][tid];
+		gincl = gown;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1)
+		{
+			const int up = __shfl_up_sync(0xffffffffu, gincl, o);
+			if (lane >= o)
+				gincl += up;
+		}
+		if (lane == 31)
+			wtot[warp] = gincl;
+	}
+	__syncthreads();
+	if (tid < 256)
+	{
+		int smaller = gincl - gown;
+		for (int w = 0; w < warp; w++)
+			smaller += wtot[w];
+		int before = 0;
+		if (tile > 0)
+		{
+			if (!look_back(state + tid, 256, tile, &st->abort, before))
+			{
+				atomicOr(err, DEVERR_TIMEOUT);
+				atomicExch(&st->abort, 1);
+				stop = 1;
+			}
+			else
+				tile_publish(state + (long long)tile * 256 + tid, TILE_TOTAL | (unsigned int)(before + total));
+		}
+		place[tid] = smaller + before;
+	}
+	__syncthreads();
+	if (stop)
+		return;
+#pragma unroll
+	for (int r = 0; r < ITEMS; r++)
+		if (base + 32 * r < n)
+		{
+			const unsigned int d = (key[r] >> shift) & mask;
+			const int at = place[d] + cnt[warp][d] + rank[r];
+			kout[at] = key[r];
+			vout[at] = val[r];
+		}
+}
+
+// Segments of the sorted keys (the outputs of bin_block_kernel); counts starts zeroed.
+template <int ITEMS>
+__global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsigned int* __restrict__ keys, int n,
+																	 unsigned int invalid, int* __restrict__ seg_start,
+																	 int* __restrict__ counts, bin_state* st,
+																	 unsigned long long* state, int* __restrict__ err)
+{
+	__shared__ int wsum[PASS_WARPS];
+	__shared__ int tile_s, stop, before_s;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	if (tid == 0)
+	{
+		tile_s = atomicAdd(&st->ticket[MAX_PASSES], 1);
+		stop = *reinterpret_cast<volatile int*>(&st->abort);
+	}
+	__syncthreads();
+	if (stop)
+		return;
+	const int tile = tile_s;
+	const long long base = (long long)tile * (PASS_THREADS * ITEMS) + warp * 32 * ITEMS + lane;
+	const unsigned int below = (1u << lane) - 1u;
+	int id[ITEMS]; // segments that start before the position in the warp, or -1 - that where one starts
+	int heads = 0;
+	long long end = -1; // the position after the last agent inside the mesh, where this thread sees it
+	int end_segs = 0;
+#pragma unroll
+	for (int r = 0; r < ITEMS; r++)
+	{
+		const long long p = base + 32 * r;
+		const unsigned int k = p < n ? keys[p] : invalid;
+		const bool in = k != invalid;
+		const bool head = in && (p == 0 || keys[p - 1] != k);
+		const unsigned int hb = __ballot_sync(0xffffffffu, head);
+		const int prefix = heads + __popc(hb & below);
+		id[r] = head ? -1 - prefix : prefix;
+		if (in && (p == n - 1 || keys[p + 1] == invalid))
+		{
+			end = p + 1;
+			end_segs = prefix + (head ? 1 : 0);
+		}
+		heads += __popc(hb);
+	}
+	if (lane == 0)
+		wsum[warp] = heads;
+	__syncthreads();
+	int ahead = 0, total = 0;
+	for (int w = 0; w < PASS_WARPS; w++)
+	{
+		if (w == warp)
+			ahead = total;
+		total += wsum[w];
+	}
+	if (tid == 0)
+	{
+		tile_publish(state + tile, (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total);
+		int before = 0;
+		if (tile > 0)
+		{
+			if (!look_back(state, 1, tile, &st->abort, before))
+			{
+				atomicOr(err, DEVERR_TIMEOUT);
+				atomicExch(&st->abort, 1);
+				stop = 1;
+			}
+			else
+				tile_publish(state + tile, TILE_TOTAL | (unsigned int)(before + total));
+		}
+		before_s = before;
+	}
+	__syncthreads();
+	if (stop)
+		return;
+	ahead += before_s;
+#pragma unroll
+	for (int r = 0; r < ITEMS; r++)
+		if (id[r] < 0)
+			seg_start[ahead - 1 - id[r]] = (int)(base + 32 * r);
+	if (end >= 0)
+	{
+		const int segments = ahead + end_segs;
+		counts[0] = segments;
+		counts[1] = (int)end;
+		counts[2] = end > segments ? 1 : 0;
+		seg_start[segments] = (int)end;
+	}
+}
+
+// ------------------------------------------------------------------------------------------------
+// host side
+
+// keys per tile of the look-back kernels: small tiles spread few agents over more CTAs, large ones
+// shorten the chain of tiles
+static constexpr int SMALL_TILE_AGENTS = 1 << 18;
+static int tile_items(int A) { return A <= SMALL_TILE_AGENTS ? 2 : 8; }
+
+static long long state_tiles(int A)
+{
+	const int tile = PASS_THREADS * tile_items(A);
+	return (A + (long long)tile - 1) / tile;
+}
+
+int bins_alloc(bfvm_solver* s, int count)
+{
+	agent_state& a = s->ag;
+	int st;
+	if (count <= BIN_BLOCK_AGENTS)
+		return BFVM_OK;
+	// the most tiles of any count up to this one
+	const long long tiles = std::max(state_tiles(count), state_tiles(std::min(count, SMALL_TILE_AGENTS)));
+	a.bin_state_bytes = (sizeof(bin_state) + 255) / 256 * 256 + (size_t)tiles * (MAX_PASSES * 256 + 1) * sizeof(unsigned long long);
+	if ((st = device_alloc(&a.bin_state, a.bin_state_bytes)) || (st = device_alloc(&a.keys_alt, (size_t)count))
+		|| (st = device_alloc(&a.vals_alt, (size_t)count)))
+		return st;
+	BFVM_CUDA(cudaMemsetAsync(a.vals_alt, 0, (size_t)count * sizeof(int), s->stream));
+	return BFVM_OK;
+}
+
+template <int ITEMS>
+static int launch_tiles(bfvm_solver* s, bin_state* st, unsigned long long* tiles, unsigned int invalid, int passes, int bits)
+{
+	agent_state& a = s->ag;
+	const int A = a.count;
+	const unsigned grid = (unsigned)state_tiles(A);
+	int rc;
+	// the passes alternate between the two buffers and end in keys/vals
+	unsigned int* kin = passes % 2 ? a.keys_alt : a.keys;
+	unsigned int* kout = passes % 2 ? a.keys : a.keys_alt;
+	int* vin = passes % 2 ? a.vals_alt : a.vals;
+	int* vout = passes % 2 ? a.vals : a.vals_alt;
+	for (int p = 0; p < passes; p++)
+	{
+		bin_pass_kernel<ITEMS><<<grid, PASS_THREADS, 0, s->stream>>>(kin, p ? vin : nullptr, kout, vout, A, p, bits, st,
+																	 tiles + (size_t)p * 256 * grid, s->dev_error);
+		if ((rc = check_launch(s, "bin_pass_kernel")))
+			return rc;
+		std::swap(kin, kout);
+		std::swap(vin, vout);
+	}
+	bin_segments_kernel<ITEMS><<<grid, PASS_THREADS, 0, s->stream>>>(
+		a.keys, A, invalid, a.seg_start, a.seg_count_dev, st, tiles + (size_t)passes * 256 * grid, s->dev_error);
+	return check_launch(s, "bin_segments_kernel");
+}
+
+int launch_bins(bfvm_solver* s)
+{
+	agent_state& a = s->ag;
+	const int A = a.count;
+	const int3 bmin = make_int3(s->bbox_min[0], s->bbox_min[1], s->bbox_min[2]);
+	const int3 vox = make_int3(s->voxel[0], s->voxel[1], s->voxel[2]);
+	const int3 grid = make_int3(s->grid[0], s->grid[1], s->grid[2]);
+	const unsigned int invalid = (unsigned int)s->V;
+	// keys take the values 0 .. V: as few passes of at most 8 bits as they need, of equal width
+	const int passes = sort_passes(s->V);
+	int total = 1;
+	while (total < 32 && ((1ull << total) <= (unsigned long long)s->V))
+		total++;
+	const int bits = (total + passes - 1) / passes;
+	int st;
+	if (A <= BIN_BLOCK_AGENTS)
+	{
+		const bin_job j{ a.pos, a.keys, a.vals, a.seg_start, a.seg_count_dev, s->dev_error, A, s->dims,
+						 bmin, vox, grid, invalid, passes, bits };
+		const size_t smem = block_smem(A);
+		if ((st = set_smem(bin_block_kernel, block_smem(BIN_BLOCK_AGENTS))))
+			return st;
+		bin_block_kernel<<<1, BLOCK_THREADS, smem, s->stream>>>(j);
+		return check_launch(s, "bin_block_kernel");
+	}
+	BFVM_CUDA(cudaMemsetAsync(a.seg_count_dev, 0, 4 * sizeof(int), s->stream));
+	BFVM_CUDA(cudaMemsetAsync(a.bin_state, 0, a.bin_state_bytes, s->stream));
+	bin_state* bs = reinterpret_cast<bin_state*>(a.bin_state);
+	unsigned long long* tiles =
+		reinterpret_cast<unsigned long long*>(a.bin_state + (sizeof(bin_state) + 255) / 256 * 256);
+	const unsigned ctas = (unsigned)std::min<long long>((A + PASS_THREADS - 1) / PASS_THREADS, 2LL * sm_count_impl(s->device));
+	bin_keys_kernel<<<ctas, PASS_THREADS, 0, s->stream>>>(a.pos, A, s->dims, bmin, vox, grid,
+														   passes % 2 ? a.keys_alt : a.keys, invalid, passes, bits, bs,
+														   s->dev_error);
+	if ((st = check_launch(s, "bin_keys_kernel")))
+		return st;
+	return tile_items(A) == 2 ? launch_tiles<2>(s, bs, tiles, invalid, passes, bits)
+							  : launch_tiles<8>(s, bs, tiles, invalid, passes, bits);
+}
+
+} // namespace bfvm

@@ -28,26 +28,6 @@ namespace bfvm {
 // ---------------------------------------------------------------------------------------------
 // voxel keys
 
-__device__ __forceinline__ bool voxel_of(const float* pos, int dims, int3 bmin, int3 vox, int3 grid, int3& c)
-{
-	// truncating (pos - min) / dx as in src/mesh.cpp:35-53; positions in (-dx, 0) truncate to 0 there
-	// too.  Anything outside the mesh is rejected instead of indexing out of bounds.
-	c = make_int3(0, 0, 0);
-	const int bm[3] = { bmin.x, bmin.y, bmin.z };
-	const int vx[3] = { vox.x, vox.y, vox.z };
-	const int gr[3] = { grid.x, grid.y, grid.z };
-	int out[3] = { 0, 0, 0 };
-	for (int d = 0; d < dims; d++)
-	{
-		const float t = __fdiv_rn(__fsub_rn(pos[d], (float)bm[d]), (float)vx[d]);
-		if (!(t > -1.0f && t < (float)gr[d]))
-			return false;
-		out[d] = (int)t;
-	}
-	c = make_int3(out[0], out[1], out[2]);
-	return true;
-}
-
 __global__ void agent_keys_kernel(const float* __restrict__ pos, int A, int dims, int3 bmin, int3 vox, int3 grid,
 								  unsigned int* __restrict__ keys, int* __restrict__ vals, unsigned int invalid_key,
 								  int* err)
@@ -219,74 +199,171 @@ __global__ void reduce_kernel(long long total, int S, const int* __restrict__ co
 	red_fac[t] = rf;
 }
 
-// The same sums over rows in the binning's sorted order (row p is the agent at sorted position p).
-__global__ void reduce_sorted_kernel(long long total, int S, const int* __restrict__ counts,
-									 const int* __restrict__ seg_start, const float* __restrict__ num,
-									 const float* __restrict__ den, const float* __restrict__ fac,
-									 float* __restrict__ red_num, float* __restrict__ red_den,
-									 float* __restrict__ red_fac)
+// V consecutive substrates of a row: four as one 16-byte access (S % 4 == 0), else one.
+template <int V>
+struct lanes
 {
-	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= total)
-		return;
-	const int seg = (int)(t / S);
-	const int s = (int)(t % S);
-	if (seg >= counts[0])
-		return;
-	const int b = seg_start[seg], e = seg_start[seg + 1];
-	const size_t w = (size_t)b * S + s;
-	float rn = __fadd_rn(0.f, num[w]);
-	float rd = __fadd_rn(0.f, __fadd_rn(den[w], 1.f));
-	float rf = __fadd_rn(0.f, fac[w]);
-	for (int p = b + 1; p < e; p++)
+	float v[V];
+
+	__device__ __forceinline__ void load(const float* p)
 	{
-		const size_t k = (size_t)p * S + s;
-		rn = __fadd_rn(rn, num[k]);
-		rd = __fadd_rn(rd, den[k]);
-		rf = __fadd_rn(rf, fac[k]);
+		if constexpr (V == 4)
+		{
+			const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+			v[0] = t.x;
+			v[1] = t.y;
+			v[2] = t.z;
+			v[3] = t.w;
+		}
+		else
+			v[0] = __ldg(p);
 	}
-	red_num[t] = rn;
-	red_den[t] = rd;
-	red_fac[t] = rf;
+
+	__device__ __forceinline__ void store(float* p) const
+	{
+		if constexpr (V == 4)
+			*reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+		else
+			p[0] = v[0];
+	}
+};
+
+// t / n and t % n, in 32 bits where the range allows (a 64-bit division costs as much as the rest of
+// these kernels' arithmetic)
+__device__ __forceinline__ int split_index(long long t, int n, int& rem)
+{
+	if ((t >> 32) == 0)
+	{
+		const unsigned q = (unsigned)t / (unsigned)n;
+		rem = (int)((unsigned)t - q * (unsigned)n);
+		return (int)q;
+	}
+	const long long q = t / n;
+	rem = (int)(t - q * n);
+	return (int)q;
 }
 
-// Row p of the sorted copies takes row order[p] of the agent-order arrays, and rank[order[p]] = p
-// (t over A * S; every agent, those outside the mesh included, has a row).
-__global__ void sort_agent_terms_kernel(long long total, int S, const int* __restrict__ order,
-										const float* __restrict__ num, const float* __restrict__ den,
-										const float* __restrict__ fac, const float* __restrict__ intern,
-										float* __restrict__ snum, float* __restrict__ sden, float* __restrict__ sfac,
-										float* __restrict__ sintern, int* __restrict__ rank)
+// The agent terms in the binning's sorted order, and the internalized amounts with them: row p of
+// num/den/fac/sintern is agent order[p]'s, and rank[order[p]] = p (every agent, those outside the mesh
+// included, has a row).  Bound by memory, five gathered rows read and four written per agent: computing
+// the terms where they are needed, instead of in agent order and then sorting them, saves three arrays
+// written and read.
+template <int V>
+__global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int SV, const int* __restrict__ order,
+															const float* __restrict__ sec, const float* __restrict__ sat,
+															const float* __restrict__ upt, const float* __restrict__ nex,
+															const float* __restrict__ intern,
+															const float* __restrict__ vol, float voxel_volume, float dt,
+															float* __restrict__ num, float* __restrict__ den,
+															float* __restrict__ fac, float* __restrict__ sintern,
+															int* __restrict__ rank)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= total)
 		return;
-	const int p = (int)(t / S);
-	const int s = (int)(t - (long long)p * S);
-	const int i = order[p];
-	const size_t k = (size_t)i * S + s;
-	snum[t] = num[k];
-	sden[t] = den[k];
-	sfac[t] = fac[k];
-	sintern[t] = intern[k];
-	if (s == 0)
-		rank[i] = p;
+	int q;
+	const int p = split_index(t, SV, q);
+	const int i = __ldg(&order[p]);
+	const size_t k = ((size_t)i * SV + q) * V, o = (size_t)t * V;
+	lanes<V> se, sa, up, ne, in;
+	se.load(sec + k);
+	sa.load(sat + k);
+	up.load(upt + k);
+	ne.load(nex + k);
+	if (sintern)
+		in.load(intern + k);
+	const float v = __ldg(&vol[i]);
+	lanes<V> nu, de, fa;
+#pragma unroll
+	for (int c = 0; c < V; c++)
+	{
+		nu.v[c] = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(se.v[c], sa.v[c]), dt), v), voxel_volume);
+		de.v[c] = __fdiv_rn(__fmul_rn(__fmul_rn(__fadd_rn(up.v[c], se.v[c]), dt), v), voxel_volume);
+		fa.v[c] = __fdiv_rn(__fmul_rn(ne.v[c], dt), voxel_volume);
+	}
+	nu.store(num + o);
+	de.store(den + o);
+	fa.store(fac + o);
+	if (sintern)
+	{
+		in.store(sintern + o);
+		if (q == 0)
+			rank[i] = p;
+	}
+}
+
+// The per-voxel sums over the sorted rows (reduce_kernel's, in the same order).  A binning that gave up
+// (bins.cu) leaves no segments.
+template <int V>
+__global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int SV, int* counts,
+															 const int* __restrict__ seg_start,
+															 const float* __restrict__ num, const float* __restrict__ den,
+															 const float* __restrict__ fac, float* __restrict__ red_num,
+															 float* __restrict__ red_den, float* __restrict__ red_fac,
+															 const int* gave_up)
+{
+	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	if (gave_up && *gave_up)
+	{
+		if (t == 0)
+			counts[0] = 0;
+		return;
+	}
+	if (t >= total)
+		return;
+	int q;
+	const int seg = split_index(t, SV, q);
+	if (seg >= counts[0])
+		return;
+	const int b = __ldg(&seg_start[seg]), e = __ldg(&seg_start[seg + 1]);
+	const size_t w = ((size_t)b * SV + q) * V;
+	lanes<V> rn, rd, rf;
+	rn.load(num + w);
+	rd.load(den + w);
+	rf.load(fac + w);
+#pragma unroll
+	for (int c = 0; c < V; c++)
+	{
+		rn.v[c] = __fadd_rn(0.f, rn.v[c]);
+		rd.v[c] = __fadd_rn(0.f, __fadd_rn(rd.v[c], 1.f));
+		rf.v[c] = __fadd_rn(0.f, rf.v[c]);
+	}
+	for (int p = b + 1; p < e; p++)
+	{
+		const size_t k = ((size_t)p * SV + q) * V;
+		lanes<V> n1, d1, f1;
+		n1.load(num + k);
+		d1.load(den + k);
+		f1.load(fac + k);
+#pragma unroll
+		for (int c = 0; c < V; c++)
+		{
+			rn.v[c] = __fadd_rn(rn.v[c], n1.v[c]);
+			rd.v[c] = __fadd_rn(rd.v[c], d1.v[c]);
+			rf.v[c] = __fadd_rn(rf.v[c], f1.v[c]);
+		}
+	}
+	rn.store(red_num + (size_t)t * V);
+	rd.store(red_den + (size_t)t * V);
+	rf.store(red_fac + (size_t)t * V);
 }
 
 // One array between the two orders: to_sorted, row p of `sorted` takes row order[p] of `agent`;
 // otherwise row order[p] of `agent` takes row p of `sorted`.
-__global__ void permute_rows_kernel(long long total, int S, const int* __restrict__ order, float* __restrict__ agent,
-									float* __restrict__ sorted, int to_sorted)
+template <int V>
+__global__ void __launch_bounds__(256) permute_rows_kernel(long long total, int SV, const int* __restrict__ order,
+															float* __restrict__ agent, float* __restrict__ sorted,
+															int to_sorted)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= total)
 		return;
-	const int p = (int)(t / S);
-	const size_t k = (size_t)order[p] * S + (t - (long long)p * S);
-	if (to_sorted)
-		sorted[t] = agent[k];
-	else
-		agent[k] = sorted[t];
+	int q;
+	const int p = split_index(t, SV, q);
+	const size_t k = ((size_t)__ldg(&order[p]) * SV + q) * V, o = (size_t)t * V;
+	lanes<V> x;
+	x.load((to_sorted ? agent + k : sorted + o));
+	x.store((to_sorted ? sorted + o : agent + k));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -394,7 +471,7 @@ void cell_free(bfvm_solver* s)
 {
 	agent_state& a = s->ag;
 	for (float** p : { &a.sec, &a.sat, &a.upt, &a.nex, &a.intern, &a.frac, &a.vol, &a.pos, &a.num, &a.den, &a.fac,
-					   &a.red_num, &a.red_den, &a.red_fac, &a.snum, &a.sden, &a.sfac, &a.sintern })
+					   &a.red_num, &a.red_den, &a.red_fac, &a.sintern })
 		device_free(*p);
 	device_free(a.rank);
 	a.sorted = false;
@@ -402,13 +479,9 @@ void cell_free(bfvm_solver* s)
 	device_free(a.keys_alt);
 	device_free(a.vals);
 	device_free(a.vals_alt);
-	device_free(a.hist);
-	device_free(a.flags);
-	device_free(a.seg_id);
+	device_free(a.bin_state);
 	device_free(a.seg_start);
 	device_free(a.seg_count_dev);
-	scan_plan_free(a.hist_scan);
-	scan_plan_free(a.flag_scan);
 	device_free(a.move_idx);
 	a.move_capacity = 0;
 	a.capacity = 0;
@@ -435,101 +508,51 @@ int cell_alloc(bfvm_solver* s, int count)
 		return st;
 	if (s->internalized)
 	{
-		for (float** p : { &a.snum, &a.sden, &a.sfac, &a.sintern })
-			if ((st = device_alloc(p, AS)))
-				return st;
-		if ((st = device_alloc(&a.rank, (size_t)count)))
+		if ((st = device_alloc(&a.sintern, AS)) || (st = device_alloc(&a.rank, (size_t)count)))
 			return st;
 	}
-	a.tiles = (int)((count + SORT_TILE - 1) / SORT_TILE);
-	if ((st = device_alloc(&a.keys, (size_t)count)) || (st = device_alloc(&a.keys_alt, (size_t)count))
-		|| (st = device_alloc(&a.vals, (size_t)count)) || (st = device_alloc(&a.vals_alt, (size_t)count))
-		|| (st = device_alloc(&a.hist, (size_t)256 * a.tiles)) || (st = device_alloc(&a.flags, (size_t)count))
-		|| (st = device_alloc(&a.seg_id, (size_t)count)) || (st = device_alloc(&a.seg_start, (size_t)count + 1))
-		|| (st = device_alloc(&a.seg_count_dev, 4)))
+	if ((st = device_alloc(&a.keys, (size_t)count)) || (st = device_alloc(&a.vals, (size_t)count))
+		|| (st = device_alloc(&a.seg_start, (size_t)count + 1)) || (st = device_alloc(&a.seg_count_dev, 4))
+		|| (st = bins_alloc(s, count)))
 		return st;
-	if ((st = scan_plan_build(a.hist_scan, 256LL * a.tiles)) || (st = scan_plan_build(a.flag_scan, count)))
-		return st;
+	// indices of some agent, whatever a binning that gave up leaves of them (bins.cu)
+	BFVM_CUDA(cudaMemsetAsync(a.vals, 0, (size_t)count * sizeof(int), s->stream));
+	BFVM_CUDA(cudaMemsetAsync(a.seg_start, 0, ((size_t)count + 1) * sizeof(int), s->stream));
 	a.capacity = count;
 	a.count = count;
 	return BFVM_OK;
 }
 
-int rebuild_bins(bfvm_solver* s, bool sorted)
+// A kernel over the agents' [A][S] rows, four substrates per thread where S allows.
+#define LAUNCH_ROWS(s, kernel, ...)                                                                                     \
+	do                                                                                                                 \
+	{                                                                                                                  \
+		const int v_ = (s)->S % 4 == 0 ? 4 : 1, sv_ = (s)->S / v_;                                                     \
+		const long long rows_ = (long long)(s)->ag.count * sv_;                                                        \
+		const unsigned blocks_ = (unsigned)((rows_ + 255) / 256);                                                      \
+		if (v_ == 4)                                                                                                   \
+			kernel<4><<<blocks_, 256, 0, (s)->stream>>>(rows_, sv_, __VA_ARGS__);                                      \
+		else                                                                                                           \
+			kernel<1><<<blocks_, 256, 0, (s)->stream>>>(rows_, sv_, __VA_ARGS__);                                      \
+	} while (0)
+
+// The binning, the agent terms in its order and the per-voxel sums; with internalized substrates also
+// the amounts in that order.
+static int rebuild_bins(bfvm_solver* s)
 {
 	agent_state& a = s->ag;
-	const int A = a.count;
-	const int3 bmin = make_int3(s->bbox_min[0], s->bbox_min[1], s->bbox_min[2]);
-	const int3 vox = make_int3(s->voxel[0], s->voxel[1], s->voxel[2]);
-	const int3 grid = make_int3(s->grid[0], s->grid[1], s->grid[2]);
-	const unsigned int invalid = (unsigned int)s->V;
 	int st;
-
-	BFVM_CUDA(cudaMemsetAsync(a.seg_count_dev, 0, 4 * sizeof(int), s->stream));
-	// The sort ping-pongs between the two buffers once per pass; starting in the buffer that makes
-	// it end in keys/vals keeps those pointers fixed, so graphs and ensemble descriptors that hold
-	// them stay valid.
-	const int passes = sort_passes(s->V);
-	unsigned int* kin = (passes % 2) ? a.keys_alt : a.keys;
-	unsigned int* kout = (passes % 2) ? a.keys : a.keys_alt;
-	int* vin = (passes % 2) ? a.vals_alt : a.vals;
-	int* vout = (passes % 2) ? a.vals : a.vals_alt;
-	agent_keys_kernel<<<(A + 255) / 256, 256, 0, s->stream>>>(a.pos, A, s->dims, bmin, vox, grid, kin, vin, invalid,
-															   s->dev_error);
-	if ((st = check_launch(s, "agent_keys_kernel")))
+	if ((st = launch_bins(s)))
 		return st;
-
-	const int tiles = (A + SORT_TILE - 1) / SORT_TILE;
-	for (int pass = 0; pass < passes; pass++)
-	{
-		radix_hist_kernel<<<tiles, SORT_THREADS, 0, s->stream>>>(kin, A, 8 * pass, a.hist, tiles);
-		if ((st = check_launch(s, "radix_hist_kernel")))
-			return st;
-		if ((st = launch_exclusive_scan(s, a.hist_scan, a.hist, a.hist, 256LL * tiles)))
-			return st;
-		radix_scatter_kernel<<<tiles, SORT_THREADS, 0, s->stream>>>(kin, vin, kout, vout, A, 8 * pass, a.hist, tiles);
-		if ((st = check_launch(s, "radix_scatter_kernel")))
-			return st;
-		std::swap(kin, kout);
-		std::swap(vin, vout);
-	}
-	// the sorted result is in a.keys / a.vals now (kin == a.keys)
-
-	seg_flags_kernel<<<(A + 255) / 256, 256, 0, s->stream>>>(a.keys, A, invalid, a.flags);
-	if ((st = check_launch(s, "seg_flags_kernel")))
+	LAUNCH_ROWS(s, sorted_terms_kernel, a.vals, a.sec, a.sat, a.upt, a.nex, a.intern, a.vol,
+				(float)(s->voxel[0] * s->voxel[1] * s->voxel[2]), s->dt, a.num, a.den, a.fac,
+				s->internalized ? a.sintern : nullptr, a.rank);
+	if ((st = check_launch(s, "sorted_terms_kernel")))
 		return st;
-	if ((st = launch_exclusive_scan(s, a.flag_scan, a.flags, a.seg_id, A)))
+	LAUNCH_ROWS(s, reduce_sorted_kernel, a.seg_count_dev, a.seg_start, a.num, a.den, a.fac, a.red_num, a.red_den,
+				a.red_fac, reinterpret_cast<const int*>(a.bin_state));
+	if ((st = check_launch(s, "reduce_sorted_kernel")))
 		return st;
-	seg_finish_kernel<<<(A + 255) / 256, 256, 0, s->stream>>>(a.keys, a.flags, a.seg_id, A, invalid, a.seg_start,
-															   a.seg_count_dev);
-	if ((st = check_launch(s, "seg_finish_kernel")))
-		return st;
-
-	const long long AS = (long long)A * s->S;
-	const unsigned blocks = (unsigned)((AS + 255) / 256);
-	intermediates_kernel<<<blocks, 256, 0, s->stream>>>(AS, s->S, a.sec, a.sat, a.upt, a.nex, a.vol,
-														 (float)(s->voxel[0] * s->voxel[1] * s->voxel[2]), s->dt,
-														 a.num, a.den, a.fac);
-	if ((st = check_launch(s, "intermediates_kernel")))
-		return st;
-	if (sorted)
-	{
-		sort_agent_terms_kernel<<<blocks, 256, 0, s->stream>>>(AS, s->S, a.vals, a.num, a.den, a.fac, a.intern, a.snum,
-																a.sden, a.sfac, a.sintern, a.rank);
-		if ((st = check_launch(s, "sort_agent_terms_kernel")))
-			return st;
-		reduce_sorted_kernel<<<blocks, 256, 0, s->stream>>>(AS, s->S, a.seg_count_dev, a.seg_start, a.snum, a.sden,
-															 a.sfac, a.red_num, a.red_den, a.red_fac);
-		if ((st = check_launch(s, "reduce_sorted_kernel")))
-			return st;
-	}
-	else
-	{
-		reduce_kernel<<<blocks, 256, 0, s->stream>>>(AS, s->S, a.seg_count_dev, a.seg_start, a.vals, a.num, a.den,
-													 a.fac, a.red_num, a.red_den, a.red_fac);
-		if ((st = check_launch(s, "reduce_kernel")))
-			return st;
-	}
 	a.binned = true;
 	return BFVM_OK;
 }
@@ -537,9 +560,7 @@ int rebuild_bins(bfvm_solver* s, bool sorted)
 // One per-agent array between agent order and the binning's sorted order.
 static int permute_rows(bfvm_solver* s, float* agent, float* sorted, bool to_sorted)
 {
-	const long long AS = (long long)s->ag.count * s->S;
-	permute_rows_kernel<<<(unsigned)((AS + 255) / 256), 256, 0, s->stream>>>(AS, s->S, s->ag.vals, agent, sorted,
-																			  to_sorted ? 1 : 0);
+	LAUNCH_ROWS(s, permute_rows_kernel, s->ag.vals, agent, sorted, to_sorted ? 1 : 0);
 	return check_launch(s, "permute_rows_kernel");
 }
 
@@ -566,38 +587,18 @@ int agents_resort_internalized(bfvm_solver* s)
 	return permute_rows(s, a.intern, a.sintern, true);
 }
 
-// With internalized substrates the secretion runs on sorted agent terms, alone or in a batch: a
-// rebinning sorts them (after writing the internalized amounts back to agent order with the old
-// order), and a solver binned but not sorted (stored amounts of an unchanged count) sorts them
-// once.  Solvers without internalized substrates keep agent order (only the per-voxel sums are
-// read then).
+// The secretion runs on agent terms in the binning's sorted order, alone or in a batch.  With
+// internalized substrates a rebinning first writes the amounts back to agent order with the old order;
+// without, only the per-voxel sums are read afterwards.
 int prepare_agent_terms(bfvm_solver* s, bool recompute)
 {
 	agent_state& a = s->ag;
-	if (a.count == 0)
+	if (a.count == 0 || (!recompute && a.binned && a.sorted == s->internalized))
 		return BFVM_OK;
-	const bool use_sorted = s->internalized;
 	int st;
-	if (recompute || !a.binned || (a.sorted && !use_sorted))
-	{
-		if ((st = agents_unsort(s, false)))
-			return st;
-	}
-	if (recompute || !a.binned)
-	{
-		if ((st = rebuild_bins(s, use_sorted)))
-			return st;
-		a.sorted = use_sorted;
-	}
-	else if (use_sorted && !a.sorted)
-	{
-		const long long AS = (long long)a.count * s->S;
-		sort_agent_terms_kernel<<<(unsigned)((AS + 255) / 256), 256, 0, s->stream>>>(
-			AS, s->S, a.vals, a.num, a.den, a.fac, a.intern, a.snum, a.sden, a.sfac, a.sintern, a.rank);
-		if ((st = check_launch(s, "sort_agent_terms_kernel")))
-			return st;
-		a.sorted = true;
-	}
+	if ((st = agents_unsort(s, false)) || (st = rebuild_bins(s)))
+		return st;
+	a.sorted = s->internalized;
 	return BFVM_OK;
 }
 
@@ -618,14 +619,14 @@ int launch_secretion(bfvm_solver* s, bool recompute)
 		const unsigned grid = (unsigned)std::max<long long>(
 			1, std::min<long long>((threads + 255) / 256, (long long)sm_count_impl(s->device) * 8));
 		secrete_sorted4_kernel<<<grid, 256, 0, s->stream>>>(s->S, s->dens, a.seg_count_dev, a.seg_start, a.keys,
-															 a.snum, a.sden, a.sfac, a.red_num, a.red_den, a.red_fac,
+															 a.num, a.den, a.fac, a.red_num, a.red_den, a.red_fac,
 															 a.sintern, vv);
 		return check_launch(s, "secrete_sorted4_kernel");
 	}
 	if (a.sorted)
 	{
 		secrete_sorted_kernel<<<(unsigned)((AS + 255) / 256), 256, 0, s->stream>>>(
-			AS, s->S, s->dens, a.seg_count_dev, a.seg_start, a.keys, a.snum, a.sden, a.sfac, a.red_num, a.red_den,
+			AS, s->S, s->dens, a.seg_count_dev, a.seg_start, a.keys, a.num, a.den, a.fac, a.red_num, a.red_den,
 			a.red_fac, a.sintern, vv);
 		return check_launch(s, "secrete_sorted_kernel");
 	}

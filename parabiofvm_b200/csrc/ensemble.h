@@ -40,8 +40,8 @@ struct ens_inst
 	const long long* dir_iidx;
 	const float* dir_ival;
 	long long dir_icount;
-	// secretion (the binning of the mesh's cell solver).  sorted: num/den/fac/intern are the agent
-	// terms in the binning's sorted order (agent_state::snum ...), else in agent order; vec4: sorted
+	// secretion (the binning of the mesh's cell solver).  num/den/fac are the agent terms in the binning's
+	// sorted order; sorted: so are the internalized amounts, else in agent order; vec4: sorted
 	// with S % 4 == 0, a unit is 256 (segment, four substrates) pairs
 	long long AS; // agents * S (0 without agents)
 	int internalized;
