@@ -62,6 +62,7 @@ struct sweep_plan
 	int vP = 1;
 	int pad = 0;
 	float* vtab = nullptr; // padded_table_floats(vP, S) floats
+	float* ltab = nullptr; // small meshes: b' [S][32 vP], then (tg, G) pairs [S][32 vP], of vtab (small.cu)
 	// lines longer than the staged sweep takes, cut into chunks that it takes (chunks.cu): chunk k
 	// holds elements [bounds[k], bounds[k + 1]) of every line; count 0 when the axis is not chunked
 	struct chunks_t
@@ -185,6 +186,9 @@ struct bfvm_solver
 	float* face_vals_d = nullptr;		  // [6][S]
 	unsigned char* face_tiles[3] = {};	  // per staged tile of each axis: a line lies on a face of another axis
 	bfvm::overwrite_list dir_interior;	  // the interior elements of the list
+	float* dir_dense = nullptr;			  // small meshes: the conditions as an array over the field (small.cu)
+	unsigned int* dir_masks[3] = {};	  // ... and its elements as mask bits per axis
+	bool dir_dense_ok = false;			  // these hold the current list
 
 	bfvm::agent_state ag;
 
@@ -256,6 +260,9 @@ struct bfvm_solver
 	// on copy_stream, each ordered after the work queued on `stream` when it was called; the next
 	// call that touches agent data makes `stream` wait for them (order_after_copies)
 	cudaStream_t copy_stream = nullptr;
+	// inside a captured step the rebinning runs on this stream, beside the diffusion (one_step)
+	cudaStream_t bin_stream = nullptr;
+	cudaEvent_t bin_fork = nullptr, bin_done = nullptr;
 	cudaEvent_t copy_ready = nullptr, copy_done = nullptr;
 	bool copy_pending = false;
 };
@@ -313,7 +320,7 @@ int rebuild_dirichlet(bfvm_solver* s);
 void free_dirichlet(bfvm_solver* s);
 
 // gradient.cu
-int launch_gradient(bfvm_solver* s);
+int launch_gradient(bfvm_solver* s, bool overlap = false); // overlap: after a small mesh's sweeps (small.h)
 // the 3D gradient of rows [y0, y1) of every plane, when substrates % 4 == 0 (false: not this shape)
 bool gradient_rows_possible(const bfvm_solver* s);
 int launch_gradient_rows(bfvm_solver* s, int y0, int y1);
@@ -326,7 +333,9 @@ void free_bulk(bfvm_solver* s);
 // cell.cu
 int cell_alloc(bfvm_solver* s, int count);
 void cell_free(bfvm_solver* s);
-int launch_secretion(bfvm_solver* s, bool recompute);
+int launch_secretion(bfvm_solver* s, bool recompute, bool overlap = false);
+// whether the next secretion rebuilds the binning (prepare_agent_terms)
+bool agents_rebin(const bfvm_solver* s, bool recompute);
 // the binning and the agent terms' order a secretion update needs (a rebinning when `recompute`)
 int prepare_agent_terms(bfvm_solver* s, bool recompute);
 int agents_unsort(bfvm_solver* s, bool keep_sorted); // internalized amounts back to agent order (cell.cu)

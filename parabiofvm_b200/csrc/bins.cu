@@ -25,6 +25,20 @@
 
 namespace bfvm {
 
+// The lanes whose `d` agrees in its low `bits` bits (8 ballots at most: a match instruction over the whole
+// value took four times as long in the ranking loops).
+__device__ __forceinline__ unsigned int same_digit(unsigned int d, int bits)
+{
+	unsigned int peers = 0xffffffffu;
+	for (int b = 0; b < bits; b++)
+	{
+		const bool on = (d >> b) & 1;
+		const unsigned int v = __ballot_sync(0xffffffffu, on);
+		peers &= on ? v : ~v;
+	}
+	return peers;
+}
+
 static constexpr int BIN_BLOCK_AGENTS = 16384;
 static constexpr int BLOCK_THREADS = 1024;
 static constexpr int BLOCK_WARPS = BLOCK_THREADS / 32;
@@ -105,7 +119,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) bin_block_kernel(const __gri
 			if (r < rounds)
 			{
 				const unsigned int d = (key[r] >> shift) & mask;
-				const unsigned int peers = __match_any_sync(0xffffffffu, d);
+				const unsigned int peers = same_digit(d, j.bits);
 				const unsigned int before = wc[d];
 				__syncwarp();
 				if ((peers & below) == 0)
@@ -371,7 +385,7 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 	{
 		const bool in = base + 32 * r < n;
 		const unsigned int d = (key[r] >> shift) & mask;
-		const unsigned int peers = __match_any_sync(0xffffffffu, in ? d : 256u);
+		const unsigned int peers = same_digit(d, bits) & __ballot_sync(0xffffffffu, in);
 		const int before = cnt[warp][d];
 		__syncwarp();
 		if (in && (peers & below) == 0)

@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "agent_kernels.cuh"
+#include "small.h"
 #include "sweep_common.cuh"
 
 namespace bfvm {
@@ -378,6 +379,7 @@ __global__ void secrete_kernel(long long total, int S, float* __restrict__ dens,
 							   float voxel_volume)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	wait_previous();
 	if (t >= total)
 		return;
 	secrete_element(t, S, dens, counts, seg_start, order, keys, num, den, fac, red_num, red_den, red_fac, intern,
@@ -394,6 +396,7 @@ __global__ void secrete_sorted_kernel(long long total, int S, float* __restrict_
 									  float* __restrict__ sintern, float voxel_volume)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	wait_previous();
 	if (t >= total)
 		return;
 	secrete_element<true>(t, S, dens, counts, seg_start, nullptr, keys, snum, sden, sfac, red_num, red_den, red_fac,
@@ -435,6 +438,7 @@ __global__ void __launch_bounds__(256) secrete_sorted4_kernel(int S, float* __re
 															  const float* __restrict__ red_fac,
 															  float* __restrict__ sintern, float voxel_volume)
 {
+	wait_previous();
 	const long long n = (long long)counts[0] * (S >> 2);
 	for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
 		secrete_sorted4_element(t, S, dens, counts, seg_start, keys, snum, sden, sfac, red_num, red_den, red_fac, sintern,
@@ -590,10 +594,16 @@ int agents_resort_internalized(bfvm_solver* s)
 // The secretion runs on agent terms in the binning's sorted order, alone or in a batch.  With
 // internalized substrates a rebinning first writes the amounts back to agent order with the old order;
 // without, only the per-voxel sums are read afterwards.
+bool agents_rebin(const bfvm_solver* s, bool recompute)
+{
+	const agent_state& a = s->ag;
+	return a.count > 0 && (recompute || !a.binned || a.sorted != s->internalized);
+}
+
 int prepare_agent_terms(bfvm_solver* s, bool recompute)
 {
 	agent_state& a = s->ag;
-	if (a.count == 0 || (!recompute && a.binned && a.sorted == s->internalized))
+	if (!agents_rebin(s, recompute))
 		return BFVM_OK;
 	int st;
 	if ((st = agents_unsort(s, false)) || (st = rebuild_bins(s)))
@@ -602,12 +612,14 @@ int prepare_agent_terms(bfvm_solver* s, bool recompute)
 	return BFVM_OK;
 }
 
-int launch_secretion(bfvm_solver* s, bool recompute)
+// overlap: the launch may overlap the end of the kernel before it (launch_overlapped)
+int launch_secretion(bfvm_solver* s, bool recompute, bool overlap)
 {
 	agent_state& a = s->ag;
 	if (a.count == 0)
 		return BFVM_OK;
 	int st;
+	overlap = overlap && !agents_rebin(s, recompute);
 	if ((st = prepare_agent_terms(s, recompute)))
 		return st;
 	const long long AS = (long long)a.count * s->S;
@@ -618,22 +630,18 @@ int launch_secretion(bfvm_solver* s, bool recompute)
 		const long long threads = AS / 4;
 		const unsigned grid = (unsigned)std::max<long long>(
 			1, std::min<long long>((threads + 255) / 256, (long long)sm_count_impl(s->device) * 8));
-		secrete_sorted4_kernel<<<grid, 256, 0, s->stream>>>(s->S, s->dens, a.seg_count_dev, a.seg_start, a.keys,
-															 a.num, a.den, a.fac, a.red_num, a.red_den, a.red_fac,
-															 a.sintern, vv);
-		return check_launch(s, "secrete_sorted4_kernel");
+		return launch_overlapped(s, "secrete_sorted4_kernel", secrete_sorted4_kernel, dim3(grid), dim3(256), 0, overlap,
+								 s->S, s->dens, a.seg_count_dev, a.seg_start, a.keys, a.num, a.den, a.fac, a.red_num,
+								 a.red_den, a.red_fac, a.sintern, vv);
 	}
+	const dim3 grid((unsigned)((AS + 255) / 256));
 	if (a.sorted)
-	{
-		secrete_sorted_kernel<<<(unsigned)((AS + 255) / 256), 256, 0, s->stream>>>(
-			AS, s->S, s->dens, a.seg_count_dev, a.seg_start, a.keys, a.num, a.den, a.fac, a.red_num, a.red_den,
-			a.red_fac, a.sintern, vv);
-		return check_launch(s, "secrete_sorted_kernel");
-	}
-	secrete_kernel<<<(unsigned)((AS + 255) / 256), 256, 0, s->stream>>>(
-		AS, s->S, s->dens, a.seg_count_dev, a.seg_start, a.vals, a.keys, a.num, a.den, a.fac, a.red_num, a.red_den,
-		a.red_fac, a.intern, s->internalized ? 1 : 0, vv);
-	return check_launch(s, "secrete_kernel");
+		return launch_overlapped(s, "secrete_sorted_kernel", secrete_sorted_kernel, grid, dim3(256), 0, overlap, AS, s->S,
+								 s->dens, a.seg_count_dev, a.seg_start, a.keys, a.num, a.den, a.fac, a.red_num,
+								 a.red_den, a.red_fac, a.sintern, vv);
+	return launch_overlapped(s, "secrete_kernel", secrete_kernel, grid, dim3(256), 0, overlap, AS, s->S, s->dens,
+							 a.seg_count_dev, a.seg_start, a.vals, a.keys, a.num, a.den, a.fac, a.red_num, a.red_den,
+							 a.red_fac, a.intern, s->internalized ? 1 : 0, vv);
 }
 
 int launch_release(bfvm_solver* s, int index)

@@ -13,6 +13,7 @@
 #include <cstring>
 
 #include "bfvm_internal.h"
+#include "small.h"
 #include "sweep_common.cuh"
 
 namespace bfvm {
@@ -79,6 +80,7 @@ void free_dirichlet(bfvm_solver* s)
 	device_free(s->dir_val);
 	s->dir_qcount = 0;
 	s->dir_count = 0;
+	s->dir_dense_ok = false;
 	for (auto& t : s->dir_tiles)
 		free_tiles(t);
 	s->face_pos_ok = false;
@@ -298,6 +300,35 @@ static int build_tile_lists(bfvm_solver* s, const std::vector<long long>& qidx, 
 	return BFVM_OK;
 }
 
+// The list of a small mesh as an array over the field.  A condition whose value is the mark of "no
+// condition" leaves the mesh to the overwrite kernels.
+static int build_dense(bfvm_solver* s, const std::vector<float>& val)
+{
+	if (!small_mesh(s) || val.empty())
+		return BFVM_OK;
+	for (float v : val)
+	{
+		unsigned int bits;
+		std::memcpy(&bits, &v, sizeof(bits));
+		if (bits == SMALL_FREE)
+			return BFVM_OK;
+	}
+	const size_t n = (size_t)(s->V * s->S);
+	int st;
+	if (!s->dir_dense && (st = device_alloc(&s->dir_dense, n)))
+		return st;
+	BFVM_CUDA(cudaMemsetAsync(s->dir_dense, 0xff, n * sizeof(float), 0));
+	const long long entries = s->dir_qcount + s->dir_count;
+	dirichlet_scatter_kernel<<<(unsigned)std::min<long long>((entries + 255) / 256, 148LL * 16), 256>>>(
+		s->dir_dense, s->dir_qidx, s->dir_qval, s->dir_qcount, s->dir_idx, s->dir_val, s->dir_count);
+	BFVM_CUDA(cudaGetLastError());
+	if ((st = build_small_masks(s)))
+		return st;
+	BFVM_CUDA(cudaStreamSynchronize(0));
+	s->dir_dense_ok = true;
+	return BFVM_OK;
+}
+
 // Resolve the faces and interior voxels into the overwrite list and upload it.
 int rebuild_dirichlet(bfvm_solver* s)
 {
@@ -411,7 +442,9 @@ int rebuild_dirichlet(bfvm_solver* s)
 	s->dir_count = (long long)sidx.size();
 	if (s->slab_count > 1 || qidx.size() + sidx.size() == 0)
 		return BFVM_OK; // slabs step axis by axis through the unfused calls
-	int st2 = build_tile_lists(s, qidx, qval, sidx, sval);
+	int st2 = build_dense(s, val);
+	if (!st2)
+		st2 = build_tile_lists(s, qidx, qval, sidx, sval);
 	if (!st2 && by_position)
 		st2 = build_face_tables(s, iidx, ival);
 	if (st2)

@@ -8,6 +8,7 @@
 // 1D [x][s][1], 2D [y][x][s][2], 3D [3][z][y][x][s].  An axis of length 1 has gradient 0.
 
 #include "bfvm_internal.h"
+#include "small.h"
 
 namespace bfvm {
 
@@ -148,8 +149,10 @@ int launch_gradient_rows(bfvm_solver* st, int y0, int y1)
 	return check_launch(st, "gradient3d_vec4_kernel");
 }
 
-int launch_gradient(bfvm_solver* st)
+int launch_gradient(bfvm_solver* st, bool overlap)
 {
+	if (small_step(st))
+		return launch_small_gradient(st, overlap);
 	const long long total = st->V * st->S;
 	float f[6];
 	gradient_factors(st, f);

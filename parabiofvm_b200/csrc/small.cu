@@ -1,0 +1,601 @@
+// The step of a small mesh: sweeps and gradient for fields that stay in L2, where a step's time is not
+// bytes but the latency of its launches, one after another.
+//
+// The staged sweeps (sweep_tma.cu) need a launch's ramp before their first tile (tables staged in shared
+// memory, barriers, the copies of the first tiles), and each overwrite of Dirichlet elements is a launch
+// of its own.  Here
+//  - a warp holds a block of 32 elements of 32 lines in registers, read straight from the field together
+//    with the coefficients of its block: one round trip to L2, nothing staged;
+//  - the Dirichlet conditions are an array over the field and, per axis, a word of mask bits per block and
+//    line: a sweep reads one word per thread and, where that is not zero, the values, which replace what it
+//    stores (the x sweep also what it loaded), so the four overwrites of the LOD step need no launch;
+//  - each kernel lets the next one launch at once (programmatic dependent launch) and reads its
+//    coefficients before it waits for the kernel before it, so launch latency overlaps work.
+// The arithmetic is that of the staged sweeps on the same tables (front-padded blocks of 32, precompute.cpp),
+// element by element, so results are the same bits.
+// One step without rebinning, before and now: 20^3 x 1 41 -> 12 us, 50^3 x 4 53 -> 23, 400 x 300 x 3 35 -> 18,
+// 97 x 61 x 83 x 5 53 -> 47, 100^3 x 4 90 -> 61, 128^3 x 4 103 -> 85.
+
+#include "small.h"
+#include "sweep_common.cuh"
+
+namespace bfvm {
+
+struct small_sweep_args
+{
+	float* data;
+	const float* ltab;		   // b' [S][N], then (tg, G) pairs [S][N], of the padded tables (N = 32 P)
+	const float* vtab;		   // the padded tables: c and the per-block products
+	const unsigned int* masks; // per tile, block and lane: the elements with a condition; null: none
+	const float* conditions;   // [V * S]: their values
+	int P, pad, S, tiles;
+	int rows, R;			   // x: rows of the field, rows per tile
+	int cols, col_tiles;	   // y, z: columns of a plane
+	int XS, line_stride, outer_stride;
+};
+
+// Where a lane's line of a tile lies: AXIS 0, a tile is R = 32 / S whole rows, lane l substrate l % S of row
+// l / S; AXIS 1, 2, 32 adjacent columns of a plane.  Lanes without a line point at an existing one.
+template <int AXIS>
+struct small_line
+{
+	bool active;
+	int s, row0, rows, rl;
+	long long at;	// offset of the line's first element
+	int stride;
+
+	__device__ __forceinline__ small_line(const small_sweep_args& a, int tile, int lane, int S)
+	{
+		active = tile < a.tiles;
+		if (!active)
+			tile = 0;
+		if (AXIS == 0)
+		{
+			rl = lane / S;
+			s = lane - rl * S;
+			row0 = tile * a.R;
+			rows = active ? min(a.R, a.rows - row0) : 0;
+			active = rl < rows;
+			at = (long long)(row0 + (active ? rl : 0)) * a.XS + s;
+			stride = S;
+		}
+		else
+		{
+			const int outer = AXIS == 1 ? tile / a.col_tiles : 0;
+			const int q = (tile - outer * a.col_tiles) * 32 + lane;
+			active = active && q < a.cols;
+			const int qq = active ? q : 0;
+			s = qq % S;
+			at = (long long)outer * a.outer_stride + qq;
+			stride = a.line_stride;
+			row0 = rows = rl = 0;
+		}
+	}
+};
+
+// The coefficients of a block.  With few warps an SM, b' is read ahead of the wait and held in registers,
+// and the responses (tg, G) come from L1: the shortest path for one tile (128 registers a thread).  STAGED,
+// the CTA copies the tables to shared memory ahead of the wait, and 64 registers do: twice the warps, which
+// larger fields need to keep the memory busy.  Rows of a table lie 4 floats (8 for the pairs) apart in banks.
+template <bool STAGED>
+struct small_coefficients
+{
+	float b[STAGED ? 1 : 32];
+	const float* bs;
+	const float2* ts;
+
+	// floats of shared memory that the staged tables take
+	static __host__ __device__ __forceinline__ int floats(int S, int N) { return STAGED ? S * (3 * N + 12) : 0; }
+
+	__device__ __forceinline__ small_coefficients(const small_sweep_args& a, int S, int s, int p, float* tab)
+	{
+		const int N = 32 * a.P;
+		if constexpr (STAGED)
+		{
+			// rows of N floats: b' of each substrate, then two per row of pairs; a warp copies whole rows
+			float* pairs = tab + S * (N + 4);
+			const int warps = a.P * blockDim.z;
+			for (int row = threadIdx.y + a.P * threadIdx.z; row < 3 * S; row += warps)
+			{
+				const float4* from = reinterpret_cast<const float4*>(a.ltab + (size_t)row * N);
+				float* to = row < S ? tab + row * (N + 4) : pairs + ((row - S) >> 1) * (2 * N + 8) + ((row - S) & 1) * N;
+				for (int t = threadIdx.x; t < N / 4; t += 32)
+					reinterpret_cast<float4*>(to)[t] = __ldg(from + t);
+			}
+			bs = tab + s * (N + 4) + p;
+			ts = reinterpret_cast<const float2*>(pairs + s * (2 * N + 8)) + p;
+			__syncthreads();
+		}
+		else
+		{
+			const float4* at = reinterpret_cast<const float4*>(a.ltab + (size_t)s * N + p);
+#pragma unroll
+			for (int k = 0; k < 32; k += 4)
+			{
+				const float4 t = __ldg(at + k / 4);
+				b[k] = t.x;
+				b[k + 1] = t.y;
+				b[k + 2] = t.z;
+				b[k + 3] = t.w;
+			}
+			ts = reinterpret_cast<const float2*>(a.ltab + (size_t)S * N + 2 * ((size_t)s * N + p));
+		}
+	}
+
+	__device__ __forceinline__ float operator[](int k) const { return STAGED ? bs[k] : b[STAGED ? 0 : k]; }
+	__device__ __forceinline__ float2 response(int k) const { return STAGED ? ts[k] : __ldg(ts + k); }
+};
+
+// The recurrences and carry folds of one block, element by element those of sweep_tma.cu.  Every thread of
+// the CTA calls it (two barriers when P > 1).
+template <bool STAGED>
+__device__ __forceinline__ void small_solve(float (&d)[32], const small_coefficients<STAGED>& b, const small_sweep_args& a,
+											int S, int s, int j, int lane, float cs, float* carry_f, float* carry_t)
+{
+	constexpr int M = 32;
+	const int P = a.P, N = 32 * P;
+#pragma unroll
+	for (int k = 1; k < M; k++)
+		d[k] = __fsub_rn(d[k], __fmul_rn(__fmul_rn(cs, b[k - 1]), d[k - 1]));
+	carry_f[j * 32 + lane] = d[M - 1];
+	asm volatile("" ::: "memory"); // staged b' is read again, not kept in 32 registers
+	d[M - 1] = __fmul_rn(d[M - 1], b[M - 1]);
+#pragma unroll
+	for (int k = M - 2; k >= 0; k--)
+		d[k] = __fmul_rn(__fsub_rn(d[k], __fmul_rn(cs, d[k + 1])), b[k]);
+	if (P == 1)
+		return;
+	const float* gqtab = a.vtab + (size_t)3 * N * S + S;
+	const float* tgptab = gqtab + P * S;
+	const float* Gptab = tgptab + P * S;
+	__syncthreads();
+	float C = 0.f, Xc = 0.f;
+	if (j > 0)
+	{
+		C = carry_f[lane];
+		for (int k = 1; k < j; k++)
+			C = fmaf(__ldg(&gqtab[k * S + s]), C, carry_f[k * 32 + lane]);
+	}
+	carry_t[j * 32 + lane] = fmaf(C, __ldg(&tgptab[j * S + s]), d[0]);
+	__syncthreads();
+	if (j < P - 1)
+	{
+		Xc = carry_t[(P - 1) * 32 + lane];
+		for (int k = P - 2; k > j; k--)
+			Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
+	}
+#pragma unroll
+	for (int k = 0; k < M; k++)
+	{
+		const float2 t = b.response(k);
+		d[k] = fmaf(Xc, t.y, fmaf(C, t.x, d[k]));
+	}
+}
+
+// v = *p where `on` is not zero: straight into the register (a load into a temporary would need 32 more)
+__device__ __forceinline__ void replace_where(float& v, unsigned int on, const float* p)
+{
+	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p ld.global.nc.f32 %0, [%2];\n\t}" : "+f"(v) : "r"(on), "l"(p));
+}
+
+// y and z sweeps.  CTA = (32, P, T): T tiles, warp (j, t) block j of tile t.
+template <int AXIS, bool STAGED>
+__global__ void __launch_bounds__(512, STAGED ? 2 : 1) small_columns_kernel(const __grid_constant__ small_sweep_args a)
+{
+	extern __shared__ __align__(16) float small_smem[];
+	let_next_launch();
+	const int lane = threadIdx.x, j = threadIdx.y, P = a.P, p = 32 * j;
+	const int tile = blockIdx.x * blockDim.z + threadIdx.z;
+	float* carry_f = small_smem + threadIdx.z * 2 * P * 32; // [P][32], then carry_t
+	const small_line<AXIS> l(a, tile, lane, a.S);
+	// coefficients and masks: constant while the solver lives, so they are read ahead of the wait
+	float d[32];
+	const small_coefficients<STAGED> b(a, a.S, l.s, p, small_smem + blockDim.z * 2 * P * 32);
+	const float cs = __ldg(a.vtab + (size_t)96 * P * a.S + l.s);
+	unsigned int mask = a.masks && l.active ? __ldg(&a.masks[((size_t)tile * P + j) * 32 + lane]) : 0u;
+	const int stride = l.stride;
+	const int first = j == 0 ? a.pad : 0; // virtual elements before the line
+	const float* from = a.data + l.at + (long long)(p - a.pad) * stride; // element 0 of the block
+	wait_previous();
+	if (first == 0)
+	{
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			d[k] = from[(long long)k * stride];
+	}
+	else
+	{
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			d[k] = k >= first ? from[(long long)k * stride] : 0.f;
+	}
+	small_solve<STAGED>(d, b, a, a.S, l.s, j, lane, cs, carry_f, carry_f + P * 32);
+	// addresses from an opaque copy of the stride: none of the load phase's stay live across the solve
+	int stride2;
+	asm volatile("mov.b32 %0, %1;" : "=r"(stride2) : "r"(stride));
+	const long long block = l.at + (long long)(p - a.pad) * stride2;
+	if (mask)
+	{
+		const float* cond = a.conditions + block;
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			replace_where(d[k], mask & (1u << k), cond + (long long)k * stride2);
+	}
+	if (!l.active)
+		return;
+	float* to = a.data + block;
+	if (first == 0)
+	{
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			to[(long long)k * stride2] = d[k];
+	}
+	else
+	{
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			if (k >= first)
+				to[(long long)k * stride2] = d[k];
+	}
+}
+
+// x sweep: a tile's rows go through shared memory so that global accesses are contiguous.  A row's block is
+// S runs of 32 floats; run i of the tile is run i % S of row i / S, kept at i % S * 32 of row i / S, rows
+// 33 S floats apart so that the lanes' elements fall into distinct banks.  SC: the substrate count where
+// it is fixed at compile time (offsets become immediates), 0 otherwise.  The conditions apply to what is
+// loaded, too: the overwrite before the first sweep of the step.
+template <int SC, bool STAGED>
+__global__ void __launch_bounds__(512, STAGED ? 2 : 1) small_rows_kernel(const __grid_constant__ small_sweep_args a)
+{
+	extern __shared__ __align__(16) float small_smem[];
+	let_next_launch();
+	const int S = SC ? SC : a.S;
+	constexpr int RUNS = SC ? 32 / (SC ? SC : 1) * SC : 32;
+	const int lane = threadIdx.x, j = threadIdx.y, P = a.P, p = 32 * j;
+	const int tile = blockIdx.x * blockDim.z + threadIdx.z;
+	float* carry_f = small_smem + threadIdx.z * 2 * P * 32;
+	float* buf = small_smem + blockDim.z * 2 * P * 32 + (threadIdx.z * P + j) * (33 * 32);
+	const int pitch = 33 * S;
+	const small_line<0> l(a, tile, lane, S);
+	float d[32];
+	const small_coefficients<STAGED> b(a, S, l.s, p, small_smem + blockDim.z * P * (64 + 33 * 32));
+	const float cs = __ldg(a.vtab + (size_t)96 * P * S + l.s);
+	const unsigned int mask = a.masks && l.active ? __ldg(&a.masks[((size_t)tile * P + j) * 32 + lane]) : 0u;
+	const int skip = j == 0 ? a.pad * S : 0; // floats of a row's block before the line
+	float* base = a.data + (long long)l.row0 * a.XS + (p - a.pad) * S + lane;
+	float* mine = buf + (l.rl < a.R ? l.rl : 0) * pitch + l.s; // element k at mine[k * S]
+	const bool whole = skip == 0 && l.rows == a.R;			   // uniform
+	wait_previous();
+
+	// f(run, offset of the lane's float in the field, offset in the buffer, whether it exists)
+	auto runs = [&](auto&& f) {
+		int r = 0, q = 0;
+#pragma unroll
+		for (int i = 0; i < RUNS; i++)
+		{
+			if (SC)
+			{
+				r = i / (SC ? SC : 1);
+				q = i - r * SC;
+			}
+			f(i, (long long)r * a.XS + 32 * q, r * pitch + 32 * q + lane, r < l.rows && 32 * q + lane >= skip);
+			if (!SC && ++q == S)
+			{
+				q = 0;
+				r++;
+			}
+		}
+	};
+	if (SC && whole)
+		runs([&](int i, long long o, int, bool) { d[i] = base[o]; });
+	else
+		runs([&](int i, long long o, int, bool in) { d[i] = in ? base[o] : 0.f; });
+	if (SC)
+		runs([&](int i, long long, int t, bool) { buf[t] = d[i]; });
+	else
+		runs([&](int i, long long, int t, bool in) {
+			if (in || t < 33 * 32)
+				buf[t] = d[i];
+		});
+	__syncwarp();
+	const long long line = l.at + (long long)(p - a.pad) * S; // offset of the block's element 0
+#pragma unroll
+	for (int k = 0; k < 32; k++)
+		d[k] = mine[k * S];
+	auto overwrite = [&]() {
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			replace_where(d[k], mask & (1u << k), a.conditions + line + k * S);
+	};
+	if (mask)
+		overwrite();
+
+	small_solve<STAGED>(d, b, a, S, l.s, j, lane, cs, carry_f, carry_f + P * 32);
+
+	if (mask)
+		overwrite();
+	__syncwarp();
+	if (l.rl < a.R)
+	{
+#pragma unroll
+		for (int k = 0; k < 32; k++)
+			mine[k * S] = d[k];
+	}
+	__syncwarp();
+	if (SC && whole)
+		runs([&](int, long long o, int t, bool) { base[o] = buf[t]; });
+	else
+		runs([&](int, long long o, int t, bool in) {
+			if (in)
+				base[o] = buf[t];
+		});
+}
+
+// Bit k of word (tile, block, lane): element k of the lane's block has a condition.
+template <int AXIS>
+__global__ void __launch_bounds__(256) small_masks_kernel(const __grid_constant__ small_sweep_args a,
+														   unsigned int* __restrict__ masks)
+{
+	const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	if (w >= (long long)a.tiles * a.P * 32)
+		return;
+	const int lane = (int)(w & 31), j = (int)((w >> 5) % a.P), tile = (int)((w >> 5) / a.P);
+	const small_line<AXIS> l(a, tile, lane, a.S);
+	unsigned int m = 0;
+	if (l.active)
+		for (int k = 0; k < 32; k++)
+		{
+			const int r = 32 * j + k - a.pad;
+			if (r >= 0 && __float_as_uint(a.conditions[l.at + (long long)r * l.stride]) != SMALL_FREE)
+				m |= 1u << k;
+		}
+	masks[w] = m;
+}
+
+// The gradient (gradient.cu's arithmetic) of V substrates at a time (4 where S % 4 == 0, else 1): a thread
+// owns one column of the (y, x, s) plane over the planes z0 .. z0 + zc - 1 of its blockIdx.y.
+struct small_gradient_args
+{
+	const float* u;
+	float* g;
+	int X, Y, Z, SV, zc;
+	float b[3], c[3];
+};
+
+template <int V>
+struct small_vec
+{
+	float v[V];
+
+	__device__ __forceinline__ void load(const float* p)
+	{
+		if constexpr (V == 4)
+		{
+			const float4 t = *reinterpret_cast<const float4*>(p);
+			v[0] = t.x;
+			v[1] = t.y;
+			v[2] = t.z;
+			v[3] = t.w;
+		}
+		else
+			v[0] = *p;
+	}
+
+	__device__ __forceinline__ void difference(const small_vec& hi, const small_vec& lo, float f)
+	{
+#pragma unroll
+		for (int k = 0; k < V; k++)
+			v[k] = __fmul_rn(__fsub_rn(hi.v[k], lo.v[k]), f);
+	}
+
+	__device__ __forceinline__ void store(float* p) const
+	{
+		if constexpr (V == 4)
+			__stcs(reinterpret_cast<float4*>(p), make_float4(v[0], v[1], v[2], v[3]));
+		else
+			__stcs(p, v[0]);
+	}
+};
+
+template <int DIMS, int V>
+__global__ void __launch_bounds__(256) small_gradient_kernel(const __grid_constant__ small_gradient_args a)
+{
+	let_next_launch();
+	const int XS = a.X * a.SV, plane = XS * a.Y; // in units of V elements
+	const int c = blockIdx.x * blockDim.x + threadIdx.x;
+	const int y = c / XS, x = (c - y * XS) / a.SV;
+	// neighbour offsets and factors of x and y (the one-sided form at the ends)
+	const int xh = x == a.X - 1 ? 0 : a.SV, xl = x == 0 ? 0 : a.SV;
+	const int yh = y == a.Y - 1 ? 0 : XS, yl = y == 0 ? 0 : XS;
+	const float fx = (xh && xl) ? a.c[0] : a.b[0], fy = (yh && yl) ? a.c[1] : a.b[1];
+	const long long total = (long long)plane * a.Z * V;
+	wait_previous();
+	if (c >= plane)
+		return;
+	const int z0 = blockIdx.y * a.zc, z1 = min(a.Z, z0 + a.zc);
+	const float* u = a.u + ((long long)z0 * plane + c) * V;
+	float* g = a.g + ((long long)z0 * plane + c) * V * (DIMS == 3 ? 1 : DIMS);
+	small_vec<V> prev, cur;
+	cur.load(u);
+	prev = cur;
+	if (DIMS == 3 && z0 > 0)
+		prev.load(u - (long long)plane * V);
+#pragma unroll 2
+	for (int z = z0; z < z1; z++)
+	{
+		small_vec<V> hi, lo, gx, gy, gz, next;
+		next = cur;
+		if (DIMS == 3 && z + 1 < a.Z)
+			next.load(u + (long long)plane * V);
+		hi.load(u + xh * V);
+		lo.load(u - xl * V);
+		gx.difference(hi, lo, fx);
+		if (DIMS == 1)
+		{
+			g[0] = gx.v[0];
+			return;
+		}
+		hi.load(u + yh * V);
+		lo.load(u - yl * V);
+		gy.difference(hi, lo, fy);
+		if (DIMS == 2)
+		{
+			reinterpret_cast<float2*>(g)[0] = make_float2(gx.v[0], gy.v[0]);
+			return;
+		}
+		gz.difference(next, prev, (z == 0 || z == a.Z - 1) ? a.b[2] : a.c[2]);
+		gx.store(g);
+		gy.store(g + total);
+		gz.store(g + 2 * total);
+		prev = cur;
+		cur = next;
+		u += (long long)plane * V;
+		g += (long long)plane * V;
+	}
+}
+
+// ------------------------------------------------------------------------------------------------
+// host side
+
+bool small_mesh(const bfvm_solver* s)
+{
+	if (s->slab_count > 1 || s->S > 32 || s->V * s->S > SMALL_ELEMENTS)
+		return false;
+	for (int d = 0; d < s->dims; d++)
+		if (!s->plan[d].ltab || s->plan[d].vP > 16 || s->plan[d].chunks.count > 0)
+			return false;
+	return true;
+}
+
+// The options that name the staged sweeps, and the tests of their bounded waits, keep them.
+bool small_step(const bfvm_solver* s)
+{
+	return small_mesh(s) && s->use_tma && !s->tma_prefetch && !s->dir_fused && !s->grad_fused && !s->face_dirichlet
+		   && s->xy_band_planes == 0 && s->zg_band_rows == 0 && s->drop_tile_copy < 0
+		   && (s->dir_qcount + s->dir_count == 0 || s->dir_dense_ok);
+}
+
+template <int AXIS>
+static small_sweep_args sweep_args_of(const bfvm_solver* s)
+{
+	const sweep_plan& pl = s->plan[AXIS];
+	const int X = s->grid[0], Y = s->grid[1], Z = s->grid[2], S = s->S;
+	small_sweep_args a;
+	a.data = s->dens;
+	a.ltab = pl.ltab;
+	a.vtab = pl.vtab;
+	a.masks = s->dir_qcount + s->dir_count ? s->dir_masks[AXIS] : nullptr;
+	a.conditions = s->dir_dense;
+	a.P = pl.vP;
+	a.pad = pl.pad;
+	a.S = S;
+	a.XS = X * S;
+	a.R = 32 / S;
+	a.rows = Y * Z;
+	a.cols = AXIS == 1 ? a.XS : a.XS * Y;
+	a.col_tiles = (a.cols + 31) / 32;
+	a.line_stride = a.cols;
+	a.outer_stride = AXIS == 1 ? a.XS * Y : 0;
+	a.tiles = AXIS == 0 ? (a.rows + a.R - 1) / a.R : a.col_tiles * (AXIS == 1 ? Z : 1);
+	return a;
+}
+
+template <int AXIS, bool STAGED>
+static void (*small_kernel(int S))(const small_sweep_args)
+{
+	if constexpr (AXIS == 0)
+		return S == 1	 ? small_rows_kernel<1, STAGED>
+			   : S == 2	 ? small_rows_kernel<2, STAGED>
+			   : S == 3	 ? small_rows_kernel<3, STAGED>
+			   : S == 4	 ? small_rows_kernel<4, STAGED>
+			   : S == 5	 ? small_rows_kernel<5, STAGED>
+			   : S == 6	 ? small_rows_kernel<6, STAGED>
+			   : S == 8	 ? small_rows_kernel<8, STAGED>
+			   : S == 16 ? small_rows_kernel<16, STAGED>
+						 : small_rows_kernel<0, STAGED>;
+	else
+		return small_columns_kernel<AXIS, STAGED>;
+}
+
+template <int AXIS>
+static int launch_small_sweep(bfvm_solver* s, bool overlap)
+{
+	const small_sweep_args a = sweep_args_of<AXIS>(s);
+	// CTAs of about four warps: lines of few blocks share one
+	const int T = std::max(1, std::min(4 / a.P, (a.tiles + sm_count_impl(s->device) - 1) / sm_count_impl(s->device)));
+	// more warps than the registers of the fuller form let reside: the staged one
+	const bool staged = (long long)a.tiles * a.P > 16LL * sm_count_impl(s->device);
+	void (*kernel)(const small_sweep_args) = staged ? small_kernel<AXIS, true>(a.S) : small_kernel<AXIS, false>(a.S);
+	const size_t smem = ((size_t)T * a.P * (64 + (AXIS == 0 ? 33 * 32 : 0))
+						 + (staged ? small_coefficients<true>::floats(a.S, 32 * a.P) : 0)) * sizeof(float);
+	int st;
+	if ((st = set_smem(kernel, smem)))
+		return st;
+	return launch_overlapped(s, "small sweep", kernel, dim3((unsigned)((a.tiles + T - 1) / T)), dim3(32, a.P, T), smem,
+							 overlap, a);
+}
+
+template <int AXIS>
+static int build_masks(bfvm_solver* s)
+{
+	const small_sweep_args a = sweep_args_of<AXIS>(s);
+	const size_t words = (size_t)a.tiles * a.P * 32;
+	int st;
+	if (!s->dir_masks[AXIS] && (st = device_alloc(&s->dir_masks[AXIS], words)))
+		return st;
+	small_masks_kernel<AXIS><<<(unsigned)((words + 255) / 256), 256>>>(a, s->dir_masks[AXIS]);
+	BFVM_CUDA(cudaGetLastError());
+	return BFVM_OK;
+}
+
+int build_small_masks(bfvm_solver* s)
+{
+	int st = build_masks<0>(s);
+	if (!st && s->dims > 1)
+		st = build_masks<1>(s);
+	if (!st && s->dims > 2)
+		st = build_masks<2>(s);
+	return st;
+}
+
+int launch_small_diffusion(bfvm_solver* s)
+{
+	int st = launch_small_sweep<0>(s, false);
+	if (!st && s->dims > 1)
+		st = launch_small_sweep<1>(s, true);
+	if (!st && s->dims > 2)
+		st = launch_small_sweep<2>(s, true);
+	return st;
+}
+
+int launch_small_gradient(bfvm_solver* s, bool overlap)
+{
+	const bool vec = s->dims == 3 && s->S % 4 == 0;
+	small_gradient_args a;
+	a.u = s->dens;
+	a.g = s->grad;
+	a.X = s->grid[0];
+	a.Y = s->grid[1];
+	a.Z = s->grid[2];
+	a.SV = vec ? s->S / 4 : s->S;
+	for (int d = 0; d < 3; d++)
+	{
+		a.b[d] = d < s->dims ? 1.f / s->voxel[d] : 0.f;
+		a.c[d] = d < s->dims ? 1.f / (s->voxel[d] * 2) : 0.f;
+	}
+	const int cols = a.X * a.SV * a.Y, ctas = (cols + 255) / 256;
+	// planes per thread: as many as leave four CTAs per SM (each march re-reads the plane before it)
+	a.zc = 1;
+	while (a.zc < 8 && (long long)ctas * (a.Z / (2 * a.zc)) >= 4LL * sm_count_impl(s->device))
+		a.zc *= 2;
+	const dim3 grid((unsigned)ctas, (unsigned)((a.Z + a.zc - 1) / a.zc));
+	if (vec)
+		return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<3, 4>, grid, dim3(256), 0, overlap, a);
+	if (s->dims == 3)
+		return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<3, 1>, grid, dim3(256), 0, overlap, a);
+	if (s->dims == 2)
+		return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<2, 1>, grid, dim3(256), 0, overlap, a);
+	return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<1, 1>, grid, dim3(256), 0, overlap, a);
+}
+
+} // namespace bfvm

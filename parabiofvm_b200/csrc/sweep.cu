@@ -22,6 +22,7 @@
 //     substrate s = t % Sc of block j = (t / Sc) % P of row t / (Sc*P).
 
 #include "ensemble.h"
+#include "small.h"
 #include "sweep_common.cuh"
 
 namespace bfvm {
@@ -409,6 +410,8 @@ int launch_diffusion(bfvm_solver* st, bool gradient, bool* gradient_done)
 {
 	if (gradient_done)
 		*gradient_done = false;
+	if (small_step(st))
+		return launch_small_diffusion(st);
 	// the face conditions by position: each staged sweep writes them into the values it stores, and
 	// the scatter after it keeps the interior elements alone.  An axis whose sweep is not staged is
 	// followed by the whole list.
