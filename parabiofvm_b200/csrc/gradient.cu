@@ -1,135 +1,176 @@
 // Central-difference gradients of the field (paraBioFVM src/solver/host/gradient_solver.cpp:10-291).
 //
 // g = (u[i+1] - u[i-1]) * (1/(2h)) inside, (u[1] - u[0]) * (1/h) and (u[n-1] - u[n-2]) * (1/h) at
-// the ends, with both factors rounded to float as in the reference (:17-18).  A 3D grid walks the
-// field: blockIdx.y = y, blockIdx.z = z, and threads run along the contiguous x*s row, so every load
-// and store of a warp is coalesced and no per-element 64-bit division is needed; the x and y
-// neighbours hit L1/L2 and each plane is read from DRAM about once.  Output layouts (src/traits.h):
-// 1D [x][s][1], 2D [y][x][s][2], 3D [3][z][y][x][s].  An axis of length 1 has gradient 0.
+// the ends, with both factors rounded to float as in the reference (:17-18).  An axis of length 1 has
+// gradient 0.  Output layouts (src/traits.h): 1D [x][s][1], 2D [y][x][s][2], 3D [3][z][y][x][s].
+//
+// Bound by memory: an element read and one written per dimension.  A thread owns V substrates (four where
+// S % 4 == 0, 16-byte accesses) of one column of the (y, x, s) plane and marches over zc planes, u(z-1),
+// u(z) and u(z+1) in registers, so each plane comes from memory once; the x and y neighbours hit L1 or L2.
+// Columns are counted over the whole plane, so that short rows leave no threads idle, and zc follows the
+// mesh (planes_per_thread).  At 250^3 x 4 185 -> 168 us (6.0 TB/s), 640 x 160 x 128 x 4
+// 160 -> 141 us, 320^3 x 16 1.41 -> 1.37 ms, against rows of CTAs that march 32 planes whatever the mesh.
 
 #include "bfvm_internal.h"
 #include "small.h"
+#include "sweep_common.cuh"
 
 namespace bfvm {
 
-__device__ __forceinline__ float axis_grad(const float* __restrict__ u, long long i, int pos, int n, long long stride,
-										   float border, float center)
+struct gradient_args
 {
-	if (n == 1)
-		return 0.f;
-	if (pos == 0)
-		return __fmul_rn(__fsub_rn(__ldg(&u[i + stride]), __ldg(&u[i])), border);
-	if (pos == n - 1)
-		return __fmul_rn(__fsub_rn(__ldg(&u[i]), __ldg(&u[i - stride])), border);
-	return __fmul_rn(__fsub_rn(__ldg(&u[i + stride]), __ldg(&u[i - stride])), center);
-}
+	const float* u;
+	float* g;
+	int X, Y, Z, SV, zc;
+	long long c0, c1;	// columns of this launch, in units of V elements
+	float b[3], c[3];	// 1/h and 1/(2h) per axis
+};
 
-template <int DIMS>
-__global__ void __launch_bounds__(256) gradient_kernel(const float* __restrict__ u, float* __restrict__ g,
-													   long long total, int S, int X, int Y, int Z, float bx, float cx,
-													   float by, float cy, float bz, float cz)
+template <int V>
+struct grad_vec
 {
-	const int XS = X * S;
-	const int q = blockIdx.x * blockDim.x + threadIdx.x;
-	if (q >= XS)
-		return;
-	const int y = blockIdx.y, z = blockIdx.z;
-	const long long i = ((long long)z * Y + y) * XS + q;
-	const int x = q / S;
-	const float gx = axis_grad(u, i, x, X, S, bx, cx);
-	if (DIMS == 1)
+	float v[V];
+
+	__device__ __forceinline__ void load(const float* p)
 	{
-		g[i] = gx;
-		return;
+		if constexpr (V == 4)
+		{
+			const float4 t = *reinterpret_cast<const float4*>(p);
+			v[0] = t.x;
+			v[1] = t.y;
+			v[2] = t.z;
+			v[3] = t.w;
+		}
+		else
+			v[0] = *p;
 	}
-	const float gy = axis_grad(u, i, y, Y, XS, by, cy);
-	if (DIMS == 2)
+
+	// (hi - lo) * f, and 0 on an axis of one voxel
+	__device__ __forceinline__ void difference(const grad_vec& hi, const grad_vec& lo, float f, int n)
 	{
-		reinterpret_cast<float2*>(g)[i] = make_float2(gx, gy);
-		return;
+#pragma unroll
+		for (int k = 0; k < V; k++)
+			v[k] = n == 1 ? 0.f : __fmul_rn(__fsub_rn(hi.v[k], lo.v[k]), f);
 	}
-	const float gz = axis_grad(u, i, z, Z, (long long)XS * Y, bz, cz);
-	g[i] = gx;
-	g[total + i] = gy;
-	g[2 * total + i] = gz;
-}
 
-// 3D gradients when S % 4 == 0: a thread owns a float4 of four consecutive substrates of one voxel
-// column (x, y) and walks ZC planes of z, keeping u(z-1), u(z), u(z+1) in registers, so each
-// element costs one streamed 16-byte load of u(z+1) plus the x and y neighbours (L1/L2 hits) and
-// three 16-byte stores.  All four substrates share x, so the border logic is per thread.
-static constexpr int GRAD_ZC = 32;
+	__device__ __forceinline__ void store(float* p) const
+	{
+		if constexpr (V == 4)
+			__stcs(reinterpret_cast<float4*>(p), make_float4(v[0], v[1], v[2], v[3]));
+		else
+			__stcs(p, v[0]);
+	}
+};
 
-__device__ __forceinline__ float4 f4sub_mul(float4 a, float4 b, float f)
+// The field is read with ordinary loads: the launch may overlap the end of the kernel that writes it (small.h).
+template <int DIMS, int V>
+__global__ void __launch_bounds__(256) gradient_kernel(const __grid_constant__ gradient_args a)
 {
-	return make_float4(__fmul_rn(__fsub_rn(a.x, b.x), f), __fmul_rn(__fsub_rn(a.y, b.y), f),
-					   __fmul_rn(__fsub_rn(a.z, b.z), f), __fmul_rn(__fsub_rn(a.w, b.w), f));
-}
-
-__global__ void __launch_bounds__(256) gradient3d_vec4_kernel(const float4* __restrict__ u, float4* __restrict__ g,
-															   long long total4, int S4, int X, int Y, int Z, float bx,
-															   float cx, float by, float cy, float bz, float cz, int y0)
-{
-	const int XS4 = X * S4;
-	const int q4 = blockIdx.x * blockDim.x + threadIdx.x;
-	if (q4 >= XS4)
+	let_next_launch();
+	const long long XS = (long long)a.X * a.SV, plane = XS * a.Y; // in units of V elements
+	const long long c = a.c0 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
+	int y, x;
+	if ((plane >> 31) == 0)
+	{
+		y = (int)((unsigned)c / (unsigned)XS);
+		x = (int)(((unsigned)c - (unsigned)y * (unsigned)XS) / (unsigned)a.SV);
+	}
+	else
+	{
+		y = (int)(c / XS);
+		x = (int)((c - y * XS) / a.SV);
+	}
+	// neighbour offsets and factors of x and y (the one-sided form at the ends)
+	const long long xh = x == a.X - 1 ? 0 : a.SV, xl = x == 0 ? 0 : a.SV;
+	const long long yh = y == a.Y - 1 ? 0 : XS, yl = y == 0 ? 0 : XS;
+	const float fx = (xh && xl) ? a.c[0] : a.b[0], fy = (yh && yl) ? a.c[1] : a.b[1];
+	const long long total = plane * a.Z * V;
+	wait_previous();
+	if (c >= a.c1)
 		return;
-	const int y = y0 + blockIdx.y;
-	const int z0 = blockIdx.z * GRAD_ZC;
-	const int z1 = min(Z, z0 + GRAD_ZC);
-	const int x = q4 / S4;
-	const long long plane = (long long)Y * XS4;
-	const long long row = (long long)y * XS4 + q4;
-
-	// x neighbours: +-S4 float4s; y neighbours: +-XS4
-	const int xo_hi = x == X - 1 ? 0 : S4, xo_lo = x == 0 ? 0 : S4;
-	const float fx = (x == 0 || x == X - 1) ? bx : cx;
-	const int yo_hi = y == Y - 1 ? 0 : XS4, yo_lo = y == 0 ? 0 : XS4;
-	const float fy = (y == 0 || y == Y - 1) ? by : cy;
-
-	float4 prev = z0 > 0 ? __ldg(&u[(long long)(z0 - 1) * plane + row]) : make_float4(0, 0, 0, 0);
-	float4 cur = __ldg(&u[(long long)z0 * plane + row]);
+	const int z0 = blockIdx.y * a.zc, z1 = min(a.Z, z0 + a.zc);
+	const float* u = a.u + (z0 * plane + c) * V;
+	float* g = a.g + (z0 * plane + c) * V * (DIMS == 3 ? 1 : DIMS);
+	grad_vec<V> prev, cur;
+	cur.load(u);
+	prev = cur;
+	if (DIMS == 3 && z0 > 0)
+		prev.load(u - plane * V);
 	for (int z = z0; z < z1; z++)
 	{
-		const long long i = (long long)z * plane + row;
-		const float4 next = z + 1 < Z ? __ldg(&u[i + plane]) : cur;
-		float4 gx, gy, gz;
-		if (X == 1)
-			gx = make_float4(0, 0, 0, 0);
-		else
-			gx = f4sub_mul(__ldg(&u[i + xo_hi]), __ldg(&u[i - xo_lo]), fx);
-		if (Y == 1)
-			gy = make_float4(0, 0, 0, 0);
-		else
-			gy = f4sub_mul(__ldg(&u[i + yo_hi]), __ldg(&u[i - yo_lo]), fy);
-		if (Z == 1)
-			gz = make_float4(0, 0, 0, 0);
-		else if (z == 0)
-			gz = f4sub_mul(next, cur, bz);
-		else if (z == Z - 1)
-			gz = f4sub_mul(cur, prev, bz);
-		else
-			gz = f4sub_mul(next, prev, cz);
-		__stcs(&g[i], gx);
-		__stcs(&g[total4 + i], gy);
-		__stcs(&g[2 * total4 + i], gz);
+		grad_vec<V> hi, lo, gx, gy, gz, next;
+		next = cur;
+		if (DIMS == 3 && z + 1 < a.Z)
+			next.load(u + plane * V);
+		hi.load(u + xh * V);
+		lo.load(u - xl * V);
+		gx.difference(hi, lo, fx, a.X);
+		if (DIMS == 1)
+		{
+			g[0] = gx.v[0];
+			return;
+		}
+		hi.load(u + yh * V);
+		lo.load(u - yl * V);
+		gy.difference(hi, lo, fy, a.Y);
+		if (DIMS == 2)
+		{
+			reinterpret_cast<float2*>(g)[0] = make_float2(gx.v[0], gy.v[0]);
+			return;
+		}
+		gz.difference(next, prev, (z == 0 || z == a.Z - 1) ? a.b[2] : a.c[2], a.Z);
+		gx.store(g);
+		gy.store(g + total);
+		gz.store(g + 2 * total);
 		prev = cur;
 		cur = next;
+		u += plane * V;
+		g += plane * V;
 	}
 }
 
-static void gradient_factors(const bfvm_solver* st, float (&f)[6])
+// Planes per thread.  A march re-reads the planes at its ends and sets its addresses up once, so up to 8 as
+// long as every SM has four CTAs; longer marches only where they still leave 16 CTAs an SM, as six are
+// resident and a last wave of few costs more (250^3 x 4: 16 planes 168 us, 32 planes 181 us; 97 x 61 x 83 x 5:
+// 8 planes 10.6 us, 2 planes 14.4 us).
+static int planes_per_thread(const bfvm_solver* s, long long ctas)
 {
-	for (int d = 0; d < 6; d++)
-		f[d] = 0.f;
-	for (int d = 0; d < st->dims; d++)
-	{
-		f[2 * d] = 1.f / st->voxel[d];
-		f[2 * d + 1] = 1.f / (st->voxel[d] * 2);
-	}
+	int zc = 1;
+	while (zc < 32 && ctas * (s->grid[2] / (2 * zc)) >= (zc < 8 ? 4LL : 16LL) * sm_count_impl(s->device))
+		zc *= 2;
+	while ((s->grid[2] + zc - 1) / zc > 65535)
+		zc *= 2; // blockIdx.y
+	return zc;
 }
 
 bool gradient_rows_possible(const bfvm_solver* st) { return st->dims == 3 && st->S % 4 == 0; }
+
+static int launch_gradient_columns(bfvm_solver* s, int y0, int y1, bool overlap)
+{
+	const bool vec = gradient_rows_possible(s);
+	gradient_args a;
+	a.u = s->dens;
+	a.g = s->grad;
+	a.X = s->grid[0];
+	a.Y = s->grid[1];
+	a.Z = s->grid[2];
+	a.SV = vec ? s->S / 4 : s->S;
+	a.c0 = (long long)y0 * a.X * a.SV;
+	a.c1 = (long long)y1 * a.X * a.SV;
+	for (int d = 0; d < 3; d++)
+	{
+		a.b[d] = d < s->dims ? 1.f / s->voxel[d] : 0.f;
+		a.c[d] = d < s->dims ? 1.f / (s->voxel[d] * 2) : 0.f;
+	}
+	const long long ctas = (a.c1 - a.c0 + 255) / 256;
+	a.zc = planes_per_thread(s, ctas);
+	const dim3 grid((unsigned)ctas, (unsigned)((a.Z + a.zc - 1) / a.zc));
+	void (*kernel)(const gradient_args) = vec			 ? gradient_kernel<3, 4>
+										  : s->dims == 3 ? gradient_kernel<3, 1>
+										  : s->dims == 2 ? gradient_kernel<2, 1>
+														 : gradient_kernel<1, 1>;
+	return launch_overlapped(s, "gradient_kernel", kernel, grid, dim3(256), 0, overlap, a);
+}
 
 int launch_gradient_rows(bfvm_solver* st, int y0, int y1)
 {
@@ -137,40 +178,9 @@ int launch_gradient_rows(bfvm_solver* st, int y0, int y1)
 		return fail(BFVM_ERR_INVALID_ARGUMENT, "gradient rows outside the mesh or not a 3D mesh of 4k substrates");
 	if (y0 == y1)
 		return BFVM_OK;
-	float f[6];
-	gradient_factors(st, f);
-	const int threads = 256;
-	const int S = st->S, X = st->grid[0], Y = st->grid[1], Z = st->grid[2];
-	const int XS4 = X * (S / 4);
-	const dim3 blocks((unsigned)((XS4 + threads - 1) / threads), (unsigned)(y1 - y0), (unsigned)((Z + GRAD_ZC - 1) / GRAD_ZC));
-	gradient3d_vec4_kernel<<<blocks, threads, 0, st->stream>>>(reinterpret_cast<const float4*>(st->dens),
-															   reinterpret_cast<float4*>(st->grad), st->V * S / 4, S / 4,
-															   X, Y, Z, f[0], f[1], f[2], f[3], f[4], f[5], y0);
-	return check_launch(st, "gradient3d_vec4_kernel");
+	return launch_gradient_columns(st, y0, y1, false);
 }
 
-int launch_gradient(bfvm_solver* st, bool overlap)
-{
-	if (small_step(st))
-		return launch_small_gradient(st, overlap);
-	const long long total = st->V * st->S;
-	float f[6];
-	gradient_factors(st, f);
-	const int threads = 256;
-	const int S = st->S, X = st->grid[0], Y = st->grid[1], Z = st->grid[2];
-	if (gradient_rows_possible(st))
-		return launch_gradient_rows(st, 0, Y);
-	const dim3 blocks((unsigned)((X * S + threads - 1) / threads), (unsigned)Y, (unsigned)Z);
-	if (st->dims == 1)
-		gradient_kernel<1><<<blocks, threads, 0, st->stream>>>(st->dens, st->grad, total, S, X, Y, Z, f[0], f[1], f[2],
-															   f[3], f[4], f[5]);
-	else if (st->dims == 2)
-		gradient_kernel<2><<<blocks, threads, 0, st->stream>>>(st->dens, st->grad, total, S, X, Y, Z, f[0], f[1], f[2],
-															   f[3], f[4], f[5]);
-	else
-		gradient_kernel<3><<<blocks, threads, 0, st->stream>>>(st->dens, st->grad, total, S, X, Y, Z, f[0], f[1], f[2],
-															   f[3], f[4], f[5]);
-	return check_launch(st, "gradient_kernel");
-}
+int launch_gradient(bfvm_solver* st, bool overlap) { return launch_gradient_columns(st, 0, st->grid[1], overlap); }
 
 } // namespace bfvm

@@ -352,108 +352,6 @@ __global__ void __launch_bounds__(256) small_masks_kernel(const __grid_constant_
 	masks[w] = m;
 }
 
-// The gradient (gradient.cu's arithmetic) of V substrates at a time (4 where S % 4 == 0, else 1): a thread
-// owns one column of the (y, x, s) plane over the planes z0 .. z0 + zc - 1 of its blockIdx.y.
-struct small_gradient_args
-{
-	const float* u;
-	float* g;
-	int X, Y, Z, SV, zc;
-	float b[3], c[3];
-};
-
-template <int V>
-struct small_vec
-{
-	float v[V];
-
-	__device__ __forceinline__ void load(const float* p)
-	{
-		if constexpr (V == 4)
-		{
-			const float4 t = *reinterpret_cast<const float4*>(p);
-			v[0] = t.x;
-			v[1] = t.y;
-			v[2] = t.z;
-			v[3] = t.w;
-		}
-		else
-			v[0] = *p;
-	}
-
-	__device__ __forceinline__ void difference(const small_vec& hi, const small_vec& lo, float f)
-	{
-#pragma unroll
-		for (int k = 0; k < V; k++)
-			v[k] = __fmul_rn(__fsub_rn(hi.v[k], lo.v[k]), f);
-	}
-
-	__device__ __forceinline__ void store(float* p) const
-	{
-		if constexpr (V == 4)
-			__stcs(reinterpret_cast<float4*>(p), make_float4(v[0], v[1], v[2], v[3]));
-		else
-			__stcs(p, v[0]);
-	}
-};
-
-template <int DIMS, int V>
-__global__ void __launch_bounds__(256) small_gradient_kernel(const __grid_constant__ small_gradient_args a)
-{
-	let_next_launch();
-	const int XS = a.X * a.SV, plane = XS * a.Y; // in units of V elements
-	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	const int y = c / XS, x = (c - y * XS) / a.SV;
-	// neighbour offsets and factors of x and y (the one-sided form at the ends)
-	const int xh = x == a.X - 1 ? 0 : a.SV, xl = x == 0 ? 0 : a.SV;
-	const int yh = y == a.Y - 1 ? 0 : XS, yl = y == 0 ? 0 : XS;
-	const float fx = (xh && xl) ? a.c[0] : a.b[0], fy = (yh && yl) ? a.c[1] : a.b[1];
-	const long long total = (long long)plane * a.Z * V;
-	wait_previous();
-	if (c >= plane)
-		return;
-	const int z0 = blockIdx.y * a.zc, z1 = min(a.Z, z0 + a.zc);
-	const float* u = a.u + ((long long)z0 * plane + c) * V;
-	float* g = a.g + ((long long)z0 * plane + c) * V * (DIMS == 3 ? 1 : DIMS);
-	small_vec<V> prev, cur;
-	cur.load(u);
-	prev = cur;
-	if (DIMS == 3 && z0 > 0)
-		prev.load(u - (long long)plane * V);
-#pragma unroll 2
-	for (int z = z0; z < z1; z++)
-	{
-		small_vec<V> hi, lo, gx, gy, gz, next;
-		next = cur;
-		if (DIMS == 3 && z + 1 < a.Z)
-			next.load(u + (long long)plane * V);
-		hi.load(u + xh * V);
-		lo.load(u - xl * V);
-		gx.difference(hi, lo, fx);
-		if (DIMS == 1)
-		{
-			g[0] = gx.v[0];
-			return;
-		}
-		hi.load(u + yh * V);
-		lo.load(u - yl * V);
-		gy.difference(hi, lo, fy);
-		if (DIMS == 2)
-		{
-			reinterpret_cast<float2*>(g)[0] = make_float2(gx.v[0], gy.v[0]);
-			return;
-		}
-		gz.difference(next, prev, (z == 0 || z == a.Z - 1) ? a.b[2] : a.c[2]);
-		gx.store(g);
-		gy.store(g + total);
-		gz.store(g + 2 * total);
-		prev = cur;
-		cur = next;
-		u += (long long)plane * V;
-		g += (long long)plane * V;
-	}
-}
-
 // ------------------------------------------------------------------------------------------------
 // host side
 
@@ -566,36 +464,6 @@ int launch_small_diffusion(bfvm_solver* s)
 	if (!st && s->dims > 2)
 		st = launch_small_sweep<2>(s, true);
 	return st;
-}
-
-int launch_small_gradient(bfvm_solver* s, bool overlap)
-{
-	const bool vec = s->dims == 3 && s->S % 4 == 0;
-	small_gradient_args a;
-	a.u = s->dens;
-	a.g = s->grad;
-	a.X = s->grid[0];
-	a.Y = s->grid[1];
-	a.Z = s->grid[2];
-	a.SV = vec ? s->S / 4 : s->S;
-	for (int d = 0; d < 3; d++)
-	{
-		a.b[d] = d < s->dims ? 1.f / s->voxel[d] : 0.f;
-		a.c[d] = d < s->dims ? 1.f / (s->voxel[d] * 2) : 0.f;
-	}
-	const int cols = a.X * a.SV * a.Y, ctas = (cols + 255) / 256;
-	// planes per thread: as many as leave four CTAs per SM (each march re-reads the plane before it)
-	a.zc = 1;
-	while (a.zc < 8 && (long long)ctas * (a.Z / (2 * a.zc)) >= 4LL * sm_count_impl(s->device))
-		a.zc *= 2;
-	const dim3 grid((unsigned)ctas, (unsigned)((a.Z + a.zc - 1) / a.zc));
-	if (vec)
-		return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<3, 4>, grid, dim3(256), 0, overlap, a);
-	if (s->dims == 3)
-		return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<3, 1>, grid, dim3(256), 0, overlap, a);
-	if (s->dims == 2)
-		return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<2, 1>, grid, dim3(256), 0, overlap, a);
-	return launch_overlapped(s, "small_gradient_kernel", small_gradient_kernel<1, 1>, grid, dim3(256), 0, overlap, a);
 }
 
 } // namespace bfvm

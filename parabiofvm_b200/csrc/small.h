@@ -16,10 +16,9 @@ static constexpr unsigned int SMALL_FREE = 0xffffffffu; // no condition in bfvm_
 // the mesh's shape is one that small.cu takes; its step runs there (no option names the other kernels)
 bool small_mesh(const bfvm_solver* s);
 bool small_step(const bfvm_solver* s);
-// the overwrites and sweeps of the LOD step; the gradient (overlap: launched after them, launch_overlapped)
+// the overwrites and sweeps of the LOD step
 int launch_small_diffusion(bfvm_solver* s);
 int build_small_masks(bfvm_solver* s); // the sweeps' mask words from bfvm_solver::dir_dense, on the legacy stream
-int launch_small_gradient(bfvm_solver* s, bool overlap);
 
 // Let the next kernel of the stream launch, and wait for the one before to finish (no-ops in launches
 // without the programmatic attribute).  Field data is read only after the wait, with ordinary loads: a
