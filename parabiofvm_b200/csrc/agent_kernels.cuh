@@ -145,7 +145,7 @@ __device__ __forceinline__ void secrete_sorted4_element(long long t, int S, floa
 	const int S4 = S >> 2;
 	const int seg = (int)(t / S4);
 	const int s0 = (int)(t - (long long)seg * S4) * 4;
-	const int b = seg_start[seg];
+	const int b = seg_start[seg], e = seg_start[seg + 1];
 	const size_t dv = (size_t)keys[b] * S + s0;
 	const size_t r = (size_t)seg * S + s0;
 	const float4 D = ld4(dens + dv);
@@ -163,12 +163,14 @@ __device__ __forceinline__ void secrete_sorted4_element(long long t, int S, floa
 	}
 	else
 	{
-		// compute_internalized for every agent of the voxel, with its own intermediates
-		const int e = seg_start[seg + 1];
+		// compute_internalized for every agent of the voxel, with its own intermediates.  Alone in its voxel,
+		// an agent's num and fac are the voxel's sums (0 + num, 0 + fac): two of the five rows less
+		// (250^3 x 4 with two million agents: a step 612 -> 602 us)
 		for (int p = b; p < e; p++)
 		{
 			const size_t k = (size_t)p * S + s0;
-			const float4 nu = ld4(snum + k), de = ld4(sden + k), fa = ld4(sfac + k);
+			const float4 de = ld4(sden + k);
+			const float4 nu = e == b + 1 ? rn : ld4(snum + k), fa = e == b + 1 ? rf : ld4(sfac + k);
 			float4 I = ld4(sintern + k);
 			I.x = __fsub_rn(I.x, __fmul_rn(voxel_volume, agent_term(D.x, nu.x, de.x, fa.x)));
 			I.y = __fsub_rn(I.y, __fmul_rn(voxel_volume, agent_term(D.y, nu.y, de.y, fa.y)));
