@@ -47,24 +47,39 @@ __global__ void secrete_kernel(long long total, int S, float* __restrict__ dens,
 							   float voxel_volume);
 
 // The voxel of an agent; false outside the mesh.
-__device__ __forceinline__ bool voxel_of(const float* pos, int dims, int3 bmin, int3 vox, int3 grid, int3& c)
+__device__ __forceinline__ bool voxel_of(const float (&pos)[3], int dims, int3 bmin, int3 vox, int3 grid, int3& c)
 {
 	// truncating (pos - min) / dx as in src/mesh.cpp:35-53; positions in (-dx, 0) truncate to 0 there
 	// too.  Anything outside the mesh is rejected instead of indexing out of bounds.
-	c = make_int3(0, 0, 0);
 	const int bm[3] = { bmin.x, bmin.y, bmin.z };
 	const int vx[3] = { vox.x, vox.y, vox.z };
 	const int gr[3] = { grid.x, grid.y, grid.z };
 	int out[3] = { 0, 0, 0 };
-	for (int d = 0; d < dims; d++)
-	{
-		const float t = __fdiv_rn(__fsub_rn(pos[d], (float)bm[d]), (float)vx[d]);
-		if (!(t > -1.0f && t < (float)gr[d]))
-			return false;
-		out[d] = (int)t;
-	}
+	bool in = true;
+#pragma unroll
+	for (int d = 0; d < 3; d++)
+		if (d < dims)
+		{
+			const float t = __fdiv_rn(__fsub_rn(pos[d], (float)bm[d]), (float)vx[d]);
+			in = in && t > -1.0f && t < (float)gr[d];
+			out[d] = in ? (int)t : 0;
+		}
 	c = make_int3(out[0], out[1], out[2]);
-	return true;
+	return in;
+}
+
+__device__ __forceinline__ void load_position(const float* __restrict__ pos, long long i, int dims, float (&x)[3])
+{
+#pragma unroll
+	for (int d = 0; d < 3; d++)
+		x[d] = d < dims ? pos[i * dims + d] : 0.f;
+}
+
+__device__ __forceinline__ bool voxel_of(const float* __restrict__ pos, int dims, int3 bmin, int3 vox, int3 grid, int3& c)
+{
+	float x[3];
+	load_position(pos, 0, dims, x);
+	return voxel_of(x, dims, bmin, vox, grid, c);
 }
 
 // One (voxel segment, substrate) pair of the secretion update; t < segments * S (secrete_kernel of
@@ -187,6 +202,9 @@ __device__ __forceinline__ void secrete_sorted4_element(long long t, int S, floa
 
 __global__ void __launch_bounds__(SCAN_THREADS) scan_tile_kernel(const int* in, int* out, long long n, int* tile_sums);
 __global__ void scan_add_kernel(int* out, long long n, const int* tile_offsets);
+
+// most agents that one CTA bins
+static constexpr int BIN_BLOCK_AGENTS = 16384;
 
 // bins.cu: the agents' order by voxel (agent_state::keys, vals) and its segments, on the solver's
 // stream; the buffers this needs for `count` agents

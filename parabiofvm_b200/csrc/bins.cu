@@ -39,11 +39,6 @@ __device__ __forceinline__ unsigned int same_digit(unsigned int d, int bits)
 	return peers;
 }
 
-static constexpr int BIN_BLOCK_AGENTS = 16384;
-static constexpr int BLOCK_THREADS = 1024;
-static constexpr int BLOCK_WARPS = BLOCK_THREADS / 32;
-static constexpr int BLOCK_ITEMS = BIN_BLOCK_AGENTS / BLOCK_THREADS;
-
 // ------------------------------------------------------------------------------------------------
 // one CTA
 
@@ -58,26 +53,41 @@ struct bin_job
 	int A, dims;
 	int3 bmin, vox, grid;
 	unsigned int invalid; // key of an agent outside the mesh
-	int passes, bits;	  // radix passes and bits per pass (at most 8)
+	int passes, bits;	  // radix passes and bits per pass (at most BLOCK_BITS)
 };
 
-static size_t block_smem(int A)
+// The CTA's shape: 256 threads for up to 1,024 agents (its barriers are the larger part there), else 1,024.
+// Digits have as many bits as threads can count them (10: two passes for a million voxels); per digit the
+// counts of the warps lie as 16-bit halves in an odd number of words, so that neighbouring digits fall into
+// distinct banks.
+template <int THREADS>
+struct block_shape
 {
-	const size_t rounds = (A + BLOCK_THREADS - 1) / BLOCK_THREADS;
-	return rounds * BLOCK_THREADS * (sizeof(unsigned int) + sizeof(unsigned short)) + BLOCK_WARPS * 256 * sizeof(unsigned short);
-}
+	static constexpr int WARPS = THREADS / 32;
+	static constexpr int ITEMS = THREADS == 1024 ? BIN_BLOCK_AGENTS / 1024 : 4;
+	static constexpr int BITS = THREADS == 1024 ? 10 : 8;
+	static constexpr int WORDS = WARPS / 2 + 1;
+
+	static size_t smem(int A, int bits)
+	{
+		const size_t rounds = (A + THREADS - 1) / THREADS;
+		return rounds * THREADS * (sizeof(unsigned int) + sizeof(unsigned short)) + ((size_t)WORDS << bits) * sizeof(unsigned int);
+	}
+};
 
 // Warp w holds agents (sorted positions) w * 32 * rounds + 32 r + lane for r < rounds, so the rounds of
 // a warp and then the warps follow the order, which makes the ranks stable.
-__global__ void __launch_bounds__(BLOCK_THREADS, 1) bin_block_kernel(const __grid_constant__ bin_job j)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) bin_block_kernel(const __grid_constant__ bin_job j)
 {
+	constexpr int BLOCK_THREADS = THREADS, BLOCK_WARPS = block_shape<THREADS>::WARPS;
+	constexpr int BLOCK_ITEMS = block_shape<THREADS>::ITEMS, DIGIT_WORDS = block_shape<THREADS>::WORDS;
 	extern __shared__ __align__(16) unsigned char bin_smem[];
-	__shared__ int tot[256];
 	__shared__ int wsum[BLOCK_WARPS], wvalid[BLOCK_WARPS];
 	const int rounds = (j.A + BLOCK_THREADS - 1) / BLOCK_THREADS;
 	unsigned int* skey = reinterpret_cast<unsigned int*>(bin_smem);
-	unsigned short* cnt = reinterpret_cast<unsigned short*>(skey + rounds * BLOCK_THREADS); // [warps][256]
-	unsigned short* sval = cnt + BLOCK_WARPS * 256;
+	unsigned int* cnt = skey + rounds * BLOCK_THREADS; // [digits][DIGIT_WORDS]
+	unsigned short* sval = reinterpret_cast<unsigned short*>(cnt + (DIGIT_WORDS << j.bits));
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int base = warp * 32 * rounds + lane;
 	const unsigned int below = (1u << lane) - 1u;
@@ -85,21 +95,34 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) bin_block_kernel(const __gri
 	unsigned int key[BLOCK_ITEMS];
 	unsigned int vr[BLOCK_ITEMS]; // agent index << 16 | rank
 	bool outside = false;
+	// the positions of four rounds are loaded before any is used
 #pragma unroll
-	for (int r = 0; r < BLOCK_ITEMS; r++)
-		if (r < rounds)
+	for (int r0 = 0; r0 < BLOCK_ITEMS; r0 += 4)
+		if (r0 < rounds)
 		{
-			const int i = base + 32 * r;
-			key[r] = j.invalid;
-			vr[r] = (unsigned int)i << 16;
-			int3 c;
-			if (i < j.A)
+			float x[4][3];
+#pragma unroll
+			for (int r = 0; r < 4; r++)
 			{
-				if (voxel_of(j.pos + (size_t)i * j.dims, j.dims, j.bmin, j.vox, j.grid, c))
-					key[r] = (unsigned int)c.x
-							 + (unsigned int)j.grid.x * ((unsigned int)c.y + (unsigned int)j.grid.y * (unsigned int)c.z);
-				else
-					outside = true;
+				const int i = base + 32 * (r0 + r);
+				if (r0 + r < rounds && i < j.A)
+					load_position(j.pos, i, j.dims, x[r]);
+			}
+#pragma unroll
+			for (int r = 0; r < 4; r++)
+			{
+				const int i = base + 32 * (r0 + r);
+				key[r0 + r] = j.invalid;
+				vr[r0 + r] = (unsigned int)i << 16;
+				if (r0 + r < rounds && i < j.A)
+				{
+					int3 c;
+					if (voxel_of(x[r], j.dims, j.bmin, j.vox, j.grid, c))
+						key[r0 + r] = (unsigned int)c.x
+									  + (unsigned int)j.grid.x * ((unsigned int)c.y + (unsigned int)j.grid.y * (unsigned int)c.z);
+					else
+						outside = true;
+				}
 			}
 		}
 	if (outside)
@@ -110,80 +133,67 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) bin_block_kernel(const __gri
 	for (int pass = 0; pass < j.passes; pass++)
 	{
 		const int shift = pass * j.bits;
-		for (int t = tid; t < BLOCK_WARPS * 128; t += BLOCK_THREADS)
-			reinterpret_cast<unsigned int*>(cnt)[t] = 0;
+		for (int t = tid; t < DIGIT_WORDS << j.bits; t += BLOCK_THREADS)
+			cnt[t] = 0;
 		__syncthreads();
-		unsigned short* wc = cnt + warp * 256;
+		unsigned short* wc = reinterpret_cast<unsigned short*>(cnt) + warp; // this warp's count of digit d: wc[2 DIGIT_WORDS d]
 #pragma unroll
 		for (int r = 0; r < BLOCK_ITEMS; r++)
 			if (r < rounds)
 			{
 				const unsigned int d = (key[r] >> shift) & mask;
 				const unsigned int peers = same_digit(d, j.bits);
-				const unsigned int before = wc[d];
+				const unsigned int before = wc[2 * DIGIT_WORDS * d];
 				__syncwarp();
 				if ((peers & below) == 0)
-					wc[d] = (unsigned short)(before + __popc(peers));
+					wc[2 * DIGIT_WORDS * d] = (unsigned short)(before + __popc(peers));
 				__syncwarp();
 				vr[r] = (vr[r] & 0xffff0000u) | (before + __popc(peers & below));
 			}
 		__syncthreads();
-		// exclusive offsets of (digit, warp): four threads a digit, eight warps each
+		// exclusive offsets of (digit, warp): a thread a digit
 		{
-			const int d = tid >> 2, part = tid & 3;
-			int own = 0;
+			unsigned int* own = cnt + DIGIT_WORDS * tid;
+			const bool digit = tid <= (int)mask;
+			unsigned int c[BLOCK_WARPS / 2];
+			int total = 0;
 #pragma unroll
-			for (int w = 0; w < BLOCK_WARPS / 4; w++)
-				own += cnt[(part * (BLOCK_WARPS / 4) + w) * 256 + d];
-			int incl = own;
-#pragma unroll
-			for (int o = 1; o < 4; o <<= 1)
+			for (int w = 0; w < BLOCK_WARPS / 2; w++)
 			{
-				const int up = __shfl_up_sync(0xffffffffu, incl, o, 4);
-				if (part >= o)
+				c[w] = digit ? own[w] : 0u;
+				total += (int)(c[w] & 0xffffu) + (int)(c[w] >> 16);
+			}
+			int incl = total;
+#pragma unroll
+			for (int o = 1; o < 32; o <<= 1)
+			{
+				const int up = __shfl_up_sync(0xffffffffu, incl, o);
+				if (lane >= o)
 					incl += up;
 			}
-			if (part == 3)
-				tot[d] = incl;
+			if (lane == 31)
+				wsum[warp] = incl;
 			__syncthreads();
-			if (warp == 0)
-			{
-				int v[8], sum = 0;
+			int ws = lane < warp ? wsum[lane] : 0;
 #pragma unroll
-				for (int k = 0; k < 8; k++)
+			for (int o = 16; o > 0; o >>= 1)
+				ws += __shfl_xor_sync(0xffffffffu, ws, o);
+			unsigned int run = (unsigned int)(ws + incl - total);
+			if (digit)
+#pragma unroll
+				for (int w = 0; w < BLOCK_WARPS / 2; w++)
 				{
-					v[k] = sum;
-					sum += tot[lane * 8 + k];
+					const unsigned int lo = run, hi = run + (c[w] & 0xffffu);
+					own[w] = lo | (hi << 16);
+					run = hi + (c[w] >> 16);
 				}
-				int run = sum;
-#pragma unroll
-				for (int o = 1; o < 32; o <<= 1)
-				{
-					const int up = __shfl_up_sync(0xffffffffu, run, o);
-					if (lane >= o)
-						run += up;
-				}
-#pragma unroll
-				for (int k = 0; k < 8; k++)
-					tot[lane * 8 + k] = run - sum + v[k];
-			}
-			__syncthreads();
-			int run = tot[d] + incl - own;
-#pragma unroll
-			for (int w = 0; w < BLOCK_WARPS / 4; w++)
-			{
-				unsigned short* c = cnt + (part * (BLOCK_WARPS / 4) + w) * 256 + d;
-				const int n = *c;
-				*c = (unsigned short)run;
-				run += n;
-			}
 		}
 		__syncthreads();
 #pragma unroll
 		for (int r = 0; r < BLOCK_ITEMS; r++)
 			if (r < rounds)
 			{
-				const int at = wc[(key[r] >> shift) & mask] + (int)(vr[r] & 0xffffu);
+				const int at = wc[2 * DIGIT_WORDS * ((key[r] >> shift) & mask)] + (int)(vr[r] & 0xffffu);
 				skey[at] = key[r];
 				sval[at] = (unsigned short)(vr[r] >> 16);
 			}
@@ -603,23 +613,26 @@ int launch_bins(bfvm_solver* s)
 	const int3 vox = make_int3(s->voxel[0], s->voxel[1], s->voxel[2]);
 	const int3 grid = make_int3(s->grid[0], s->grid[1], s->grid[2]);
 	const unsigned int invalid = (unsigned int)s->V;
-	// keys take the values 0 .. V: as few passes of at most 8 bits as they need, of equal width
-	const int passes = sort_passes(s->V);
+	// keys take the values 0 .. V: as few passes as they need, of equal width
 	int total = 1;
 	while (total < 32 && ((1ull << total) <= (unsigned long long)s->V))
 		total++;
-	const int bits = (total + passes - 1) / passes;
 	int st;
 	if (A <= BIN_BLOCK_AGENTS)
 	{
-		const bin_job j{ a.pos, a.keys, a.vals, a.seg_start, a.seg_count_dev, s->dev_error, A, s->dims,
-						 bmin, vox, grid, invalid, passes, bits };
-		const size_t smem = block_smem(A);
-		if ((st = set_smem(bin_block_kernel, block_smem(BIN_BLOCK_AGENTS))))
-			return st;
-		bin_block_kernel<<<1, BLOCK_THREADS, smem, s->stream>>>(j);
-		return check_launch(s, "bin_block_kernel");
+		auto launch = [&](auto shape, auto kernel) {
+			constexpr int THREADS = 32 * decltype(shape)::WARPS;
+			const int passes = (total + shape.BITS - 1) / shape.BITS, bits = (total + passes - 1) / passes;
+			const bin_job j{ a.pos, a.keys, a.vals, a.seg_start, a.seg_count_dev, s->dev_error, A, s->dims,
+							 bmin, vox, grid, invalid, passes, bits };
+			if ((st = set_smem(kernel, shape.smem(BIN_BLOCK_AGENTS, shape.BITS))))
+				return st;
+			kernel<<<1, THREADS, shape.smem(A, bits), s->stream>>>(j);
+			return check_launch(s, "bin_block_kernel");
+		};
+		return A <= 1024 ? launch(block_shape<256>(), bin_block_kernel<256>) : launch(block_shape<1024>(), bin_block_kernel<1024>);
 	}
+	const int passes = sort_passes(s->V), bits = (total + passes - 1) / passes;
 	BFVM_CUDA(cudaMemsetAsync(a.seg_count_dev, 0, 4 * sizeof(int), s->stream));
 	BFVM_CUDA(cudaMemsetAsync(a.bin_state, 0, a.bin_state_bytes, s->stream));
 	bin_state* bs = reinterpret_cast<bin_state*>(a.bin_state);

@@ -244,6 +244,46 @@ __device__ __forceinline__ int split_index(long long t, int n, int& rem)
 	return (int)q;
 }
 
+// The terms of the agent at sorted position p, V substrates from V q, written to row p; with internalized
+// substrates also the amounts and the agent's rank.
+template <int V>
+__device__ __forceinline__ void agent_terms(int p, int q, int SV, const int* __restrict__ order,
+											const float* __restrict__ sec, const float* __restrict__ sat,
+											const float* __restrict__ upt, const float* __restrict__ nex,
+											const float* __restrict__ intern, const float* __restrict__ vol,
+											float voxel_volume, float dt, float* __restrict__ num,
+											float* __restrict__ den, float* __restrict__ fac,
+											float* __restrict__ sintern, int* __restrict__ rank, lanes<V>& nu,
+											lanes<V>& de, lanes<V>& fa)
+{
+	const int i = __ldg(&order[p]);
+	const size_t k = ((size_t)i * SV + q) * V, o = ((size_t)p * SV + q) * V;
+	lanes<V> se, sa, up, ne, in;
+	se.load(sec + k);
+	sa.load(sat + k);
+	up.load(upt + k);
+	ne.load(nex + k);
+	if (sintern)
+		in.load(intern + k);
+	const float v = __ldg(&vol[i]);
+#pragma unroll
+	for (int c = 0; c < V; c++)
+	{
+		nu.v[c] = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(se.v[c], sa.v[c]), dt), v), voxel_volume);
+		de.v[c] = __fdiv_rn(__fmul_rn(__fmul_rn(__fadd_rn(up.v[c], se.v[c]), dt), v), voxel_volume);
+		fa.v[c] = __fdiv_rn(__fmul_rn(ne.v[c], dt), voxel_volume);
+	}
+	nu.store(num + o);
+	de.store(den + o);
+	fa.store(fac + o);
+	if (sintern)
+	{
+		in.store(sintern + o);
+		if (q == 0)
+			rank[i] = p;
+	}
+}
+
 // The agent terms in the binning's sorted order, and the internalized amounts with them: row p of
 // num/den/fac/sintern is agent order[p]'s, and rank[order[p]] = p (every agent, those outside the mesh
 // included, has a row).  Bound by memory, five gathered rows read and four written per agent: computing
@@ -264,33 +304,9 @@ __global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int 
 		return;
 	int q;
 	const int p = split_index(t, SV, q);
-	const int i = __ldg(&order[p]);
-	const size_t k = ((size_t)i * SV + q) * V, o = (size_t)t * V;
-	lanes<V> se, sa, up, ne, in;
-	se.load(sec + k);
-	sa.load(sat + k);
-	up.load(upt + k);
-	ne.load(nex + k);
-	if (sintern)
-		in.load(intern + k);
-	const float v = __ldg(&vol[i]);
 	lanes<V> nu, de, fa;
-#pragma unroll
-	for (int c = 0; c < V; c++)
-	{
-		nu.v[c] = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(se.v[c], sa.v[c]), dt), v), voxel_volume);
-		de.v[c] = __fdiv_rn(__fmul_rn(__fmul_rn(__fadd_rn(up.v[c], se.v[c]), dt), v), voxel_volume);
-		fa.v[c] = __fdiv_rn(__fmul_rn(ne.v[c], dt), voxel_volume);
-	}
-	nu.store(num + o);
-	de.store(den + o);
-	fa.store(fac + o);
-	if (sintern)
-	{
-		in.store(sintern + o);
-		if (q == 0)
-			rank[i] = p;
-	}
+	agent_terms(p, q, SV, order, sec, sat, upt, nex, intern, vol, voxel_volume, dt, num, den, fac, sintern, rank, nu, de,
+				fa);
 }
 
 // The per-voxel sums over the sorted rows (reduce_kernel's, in the same order).  A binning that gave up
@@ -347,6 +363,49 @@ __global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int
 	rn.store(red_num + (size_t)t * V);
 	rd.store(red_den + (size_t)t * V);
 	rf.store(red_fac + (size_t)t * V);
+}
+
+// Both of the above at once, for agents that one CTA bins (launches count there, not bytes): a thread owns a
+// segment, or an agent outside the mesh, and walks its agents.
+template <int V>
+__global__ void __launch_bounds__(256) segment_terms_kernel(
+	long long total, int SV, int A, const int* __restrict__ counts, const int* __restrict__ seg_start,
+	const int* __restrict__ order, const float* __restrict__ sec, const float* __restrict__ sat,
+	const float* __restrict__ upt, const float* __restrict__ nex, const float* __restrict__ intern,
+	const float* __restrict__ vol, float voxel_volume, float dt, float* __restrict__ num, float* __restrict__ den,
+	float* __restrict__ fac, float* __restrict__ sintern, int* __restrict__ rank, float* __restrict__ red_num,
+	float* __restrict__ red_den, float* __restrict__ red_fac)
+{
+	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	if (t >= total)
+		return;
+	int q;
+	const int item = split_index(t, SV, q);
+	const int segments = counts[0], inside = counts[1];
+	if (item >= segments + A - inside)
+		return;
+	const bool in = item < segments;
+	const int b = in ? seg_start[item] : inside + item - segments, e = in ? seg_start[item + 1] : b + 1;
+	lanes<V> rn, rd, rf;
+	for (int p = b; p < e; p++)
+	{
+		lanes<V> nu, de, fa;
+		agent_terms(p, q, SV, order, sec, sat, upt, nex, intern, vol, voxel_volume, dt, num, den, fac, sintern, rank, nu,
+					de, fa);
+#pragma unroll
+		for (int c = 0; c < V; c++)
+		{
+			rn.v[c] = __fadd_rn(p == b ? 0.f : rn.v[c], nu.v[c]);
+			rd.v[c] = __fadd_rn(p == b ? 0.f : rd.v[c], p == b ? __fadd_rn(de.v[c], 1.f) : de.v[c]);
+			rf.v[c] = __fadd_rn(p == b ? 0.f : rf.v[c], fa.v[c]);
+		}
+	}
+	if (in)
+	{
+		rn.store(red_num + (size_t)t * V);
+		rd.store(red_den + (size_t)t * V);
+		rf.store(red_fac + (size_t)t * V);
+	}
 }
 
 // One array between the two orders: to_sorted, row p of `sorted` takes row order[p] of `agent`;
@@ -548,6 +607,14 @@ static int rebuild_bins(bfvm_solver* s)
 	int st;
 	if ((st = launch_bins(s)))
 		return st;
+	if (a.count <= BIN_BLOCK_AGENTS)
+	{
+		LAUNCH_ROWS(s, segment_terms_kernel, a.count, a.seg_count_dev, a.seg_start, a.vals, a.sec, a.sat, a.upt, a.nex,
+					a.intern, a.vol, (float)(s->voxel[0] * s->voxel[1] * s->voxel[2]), s->dt, a.num, a.den, a.fac,
+					s->internalized ? a.sintern : nullptr, a.rank, a.red_num, a.red_den, a.red_fac);
+		a.binned = true;
+		return check_launch(s, "segment_terms_kernel");
+	}
 	LAUNCH_ROWS(s, sorted_terms_kernel, a.vals, a.sec, a.sat, a.upt, a.nex, a.intern, a.vol,
 				(float)(s->voxel[0] * s->voxel[1] * s->voxel[2]), s->dt, a.num, a.den, a.fac,
 				s->internalized ? a.sintern : nullptr, a.rank);
