@@ -26,26 +26,33 @@ int build_small_masks(bfvm_solver* s); // the sweeps' mask words from bfvm_solve
 __device__ __forceinline__ void let_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launch `kernel` on the solver's stream; `overlap`: it may start before the kernel before it ends (that
-// kernel and every one before it in the step waits for its own predecessor).
+// Launch `kernel` on the stream; `overlap`: it may start before the kernel before it ends (which must itself
+// wait for its predecessor: wait_previous).
 template <typename... A, typename... B>
-int launch_overlapped(bfvm_solver* s, const char* what, void (*kernel)(A...), dim3 grid, dim3 block, size_t smem,
-						bool overlap, B&&... args)
+int launch_overlapped(cudaStream_t stream, const char* what, void (*kernel)(A...), dim3 grid, dim3 block, size_t smem,
+					  bool overlap, B&&... args)
 {
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid;
 	cfg.blockDim = block;
 	cfg.dynamicSmemBytes = smem;
-	cfg.stream = s->stream;
+	cfg.stream = stream;
 	cudaLaunchAttribute attr[1];
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	attr[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = overlap ? 1 : 0;
 	const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<B>(args)...);
-	if (e != cudaSuccess)
-		return cuda_fail(e, what);
-	return check_launch(s, what);
+	return e == cudaSuccess ? BFVM_OK : cuda_fail(e, what);
+}
+
+// ... on the solver's, counted
+template <typename... A, typename... B>
+int launch_overlapped(bfvm_solver* s, const char* what, void (*kernel)(A...), dim3 grid, dim3 block, size_t smem,
+					  bool overlap, B&&... args)
+{
+	const int st = launch_overlapped(s->stream, what, kernel, grid, block, smem, overlap, std::forward<B>(args)...);
+	return st ? st : check_launch(s, what);
 }
 
 } // namespace bfvm
