@@ -14,7 +14,8 @@
 // The arithmetic is that of the staged sweeps on the same tables (front-padded blocks of 32, precompute.cpp),
 // element by element, so results are the same bits.
 // One step without rebinning, before and now: 20^3 x 1 41 -> 12 us, 50^3 x 4 53 -> 23, 400 x 300 x 3 35 -> 18,
-// 97 x 61 x 83 x 5 53 -> 47, 100^3 x 4 90 -> 61, 128^3 x 4 103 -> 85.
+// 97 x 61 x 83 x 5 53 -> 47, 100^3 x 4 90 -> 61, 128^3 x 4 103 -> 85; lines beyond 512:
+// 800 x 600 x 4 61 -> 33, 40 x 900 x 3 33 -> 18, 600 x 600 x 20 x 1 162 -> 95.
 
 #include "small.h"
 #include "sweep_common.cuh"
@@ -178,9 +179,10 @@ __device__ __forceinline__ void replace_where(float& v, unsigned int on, const f
 	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p ld.global.nc.f32 %0, [%2];\n\t}" : "+f"(v) : "r"(on), "l"(p));
 }
 
-// y and z sweeps.  CTA = (32, P, T): T tiles, warp (j, t) block j of tile t.
-template <int AXIS, bool STAGED>
-__global__ void __launch_bounds__(512, STAGED ? 2 : 1) small_columns_kernel(const __grid_constant__ small_sweep_args a)
+// y and z sweeps.  CTA = (32, P, T): T tiles, warp (j, t) block j of tile t; at most THREADS threads (1024
+// for lines of 17 to 32 blocks, staged).
+template <int AXIS, bool STAGED, int THREADS>
+__global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) small_columns_kernel(const __grid_constant__ small_sweep_args a)
 {
 	extern __shared__ __align__(16) float small_smem[];
 	let_next_launch();
@@ -244,8 +246,8 @@ __global__ void __launch_bounds__(512, STAGED ? 2 : 1) small_columns_kernel(cons
 // 33 S floats apart so that the lanes' elements fall into distinct banks.  SC: the substrate count where
 // it is fixed at compile time (offsets become immediates), 0 otherwise.  The conditions apply to what is
 // loaded, too: the overwrite before the first sweep of the step.
-template <int SC, bool STAGED>
-__global__ void __launch_bounds__(512, STAGED ? 2 : 1) small_rows_kernel(const __grid_constant__ small_sweep_args a)
+template <int SC, bool STAGED, int THREADS>
+__global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) small_rows_kernel(const __grid_constant__ small_sweep_args a)
 {
 	extern __shared__ __align__(16) float small_smem[];
 	let_next_launch();
@@ -355,12 +357,21 @@ __global__ void __launch_bounds__(256) small_masks_kernel(const __grid_constant_
 // ------------------------------------------------------------------------------------------------
 // host side
 
+// shared memory of a CTA of T tiles
+static size_t sweep_smem(int axis, int P, int S, int T, bool staged)
+{
+	return ((size_t)T * P * (64 + (axis == 0 ? 33 * 32 : 0)) + (staged ? small_coefficients<true>::floats(S, 32 * P) : 0))
+		   * sizeof(float);
+}
+
 bool small_mesh(const bfvm_solver* s)
 {
 	if (s->slab_count > 1 || s->S > 32 || s->V * s->S > SMALL_ELEMENTS)
 		return false;
+	// lines of up to 32 blocks, in CTAs of up to 1024 threads, whose buffers and tables fit a CTA's 227 KB
 	for (int d = 0; d < s->dims; d++)
-		if (!s->plan[d].ltab || s->plan[d].vP > 16 || s->plan[d].chunks.count > 0)
+		if (!s->plan[d].ltab || s->plan[d].vP > 32
+			|| sweep_smem(d, s->plan[d].vP, s->S, std::max(1, 4 / s->plan[d].vP), true) > 227 * 1024)
 			return false;
 	return true;
 }
@@ -369,7 +380,7 @@ bool small_mesh(const bfvm_solver* s)
 bool small_step(const bfvm_solver* s)
 {
 	return small_mesh(s) && s->use_tma && !s->tma_prefetch && !s->dir_fused && !s->grad_fused && !s->face_dirichlet
-		   && s->xy_band_planes == 0 && s->zg_band_rows == 0 && s->drop_tile_copy < 0
+		   && s->xy_band_planes == 0 && s->zg_band_rows == 0 && s->chunk_elements == 0 && s->drop_tile_copy < 0
 		   && (s->dir_qcount + s->dir_count == 0 || s->dir_dense_ok);
 }
 
@@ -398,21 +409,21 @@ static small_sweep_args sweep_args_of(const bfvm_solver* s)
 	return a;
 }
 
-template <int AXIS, bool STAGED>
+template <int AXIS, bool STAGED, int THREADS>
 static void (*small_kernel(int S))(const small_sweep_args)
 {
 	if constexpr (AXIS == 0)
-		return S == 1	 ? small_rows_kernel<1, STAGED>
-			   : S == 2	 ? small_rows_kernel<2, STAGED>
-			   : S == 3	 ? small_rows_kernel<3, STAGED>
-			   : S == 4	 ? small_rows_kernel<4, STAGED>
-			   : S == 5	 ? small_rows_kernel<5, STAGED>
-			   : S == 6	 ? small_rows_kernel<6, STAGED>
-			   : S == 8	 ? small_rows_kernel<8, STAGED>
-			   : S == 16 ? small_rows_kernel<16, STAGED>
-						 : small_rows_kernel<0, STAGED>;
+		return S == 1	 ? small_rows_kernel<1, STAGED, THREADS>
+			   : S == 2	 ? small_rows_kernel<2, STAGED, THREADS>
+			   : S == 3	 ? small_rows_kernel<3, STAGED, THREADS>
+			   : S == 4	 ? small_rows_kernel<4, STAGED, THREADS>
+			   : S == 5	 ? small_rows_kernel<5, STAGED, THREADS>
+			   : S == 6	 ? small_rows_kernel<6, STAGED, THREADS>
+			   : S == 8	 ? small_rows_kernel<8, STAGED, THREADS>
+			   : S == 16 ? small_rows_kernel<16, STAGED, THREADS>
+						 : small_rows_kernel<0, STAGED, THREADS>;
 	else
-		return small_columns_kernel<AXIS, STAGED>;
+		return small_columns_kernel<AXIS, STAGED, THREADS>;
 }
 
 template <int AXIS>
@@ -421,11 +432,12 @@ static int launch_small_sweep(bfvm_solver* s, bool overlap)
 	const small_sweep_args a = sweep_args_of<AXIS>(s);
 	// CTAs of about four warps: lines of few blocks share one
 	const int T = std::max(1, std::min(4 / a.P, (a.tiles + sm_count_impl(s->device) - 1) / sm_count_impl(s->device)));
-	// more warps than the registers of the fuller form let reside: the staged one
-	const bool staged = (long long)a.tiles * a.P > 16LL * sm_count_impl(s->device);
-	void (*kernel)(const small_sweep_args) = staged ? small_kernel<AXIS, true>(a.S) : small_kernel<AXIS, false>(a.S);
-	const size_t smem = ((size_t)T * a.P * (64 + (AXIS == 0 ? 33 * 32 : 0))
-						 + (staged ? small_coefficients<true>::floats(a.S, 32 * a.P) : 0)) * sizeof(float);
+	// more warps than the registers of the fuller form let reside, or lines that need 1024 threads
+	const bool staged = a.P > 16 || (long long)a.tiles * a.P > 16LL * sm_count_impl(s->device);
+	void (*kernel)(const small_sweep_args) = a.P > 16 ? small_kernel<AXIS, true, 1024>(a.S)
+											 : staged ? small_kernel<AXIS, true, 512>(a.S)
+													  : small_kernel<AXIS, false, 512>(a.S);
+	const size_t smem = sweep_smem(AXIS, a.P, a.S, T, staged);
 	int st;
 	if ((st = set_smem(kernel, smem)))
 		return st;

@@ -1,6 +1,6 @@
 """The small-mesh kernels against the staged sweeps, the scattered overwrites and the plain gradient and
 secretion launches (any option that names those selects them; results are the same bits): line lengths at
-the edges of a block of 32, one to sixteen blocks, every substrate count that has an instance of its own
+the edges of a block of 32, one to 32 blocks, every substrate count that has an instance of its own
 and others, tiles with rows or columns missing, 1-D to 3-D, face and interior conditions that meet, and
 agents; two steps, so that one of them rebins beside the diffusion."""
 
@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 SHAPES = [((2, 2, 2), 1), ((31, 5, 3), 2), ((32, 33, 2), 3), ((33, 32, 31), 4), ((64, 65, 3), 5), ((3, 64, 65), 6),
           ((97, 9, 34), 7), ((40, 41, 42), 8), ((65, 4, 40), 12), ((34, 33, 20), 16), ((36, 10, 7), 17),
           ((33, 6, 5), 32), ((512, 5, 4), 1), ((4, 512, 3), 4), ((3, 4, 500), 3), ((300, 257), 3), ((20, 700), 2),
-          ((45, 31), 16), ((500,), 4), ((2,), 32), ((128, 100, 80), 8)]
+          ((45, 31), 16), ((500,), 4), ((2,), 32), ((128, 100, 80), 8),
+          ((513, 4, 3), 3), ((3, 700, 5), 4), ((4, 3, 1024), 2), ((1000, 30), 5), ((30, 999), 1), ((1024,), 6)]
 
 
 @pytest.mark.parametrize("grid,S", SHAPES)
@@ -38,6 +39,8 @@ def test_small_mesh_same_bits_as_staged(grid, S, conditions):
         s = Solver(dims, (0,) * 3, tuple(g * dx for g in grid), (dx,) * 3, D, lam, 0.05, compute_internalized=True)
         if staged:
             s.set_option("tma_prefetch", 1)
+            if max(grid) > 512:  # lines that the staged sweep takes in chunks, which agree to rounding only
+                s.set_option("tma_sweeps", 0)
         if conditions != "none":
             for d, m, v, c in faces:
                 s.set_boundary_dirichlet(d, m, v, c)
