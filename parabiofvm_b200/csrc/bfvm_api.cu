@@ -70,7 +70,7 @@ static int upload_plan(bfvm_solver* s, int axis)
 		if ((st = device_alloc(&p.vtab, vt.size())))
 			return st;
 		BFVM_CUDA(cudaMemcpy(p.vtab, vt.data(), vt.size() * sizeof(float), cudaMemcpyHostToDevice));
-		if (s->V * s->S <= SMALL_ELEMENTS)
+		if (s->V * s->S <= small_elements(s->S))
 		{
 			// the per-element tables with a substrate's values side by side
 			const size_t N = (size_t)32 * p.vP, S = (size_t)s->S;

@@ -13,9 +13,9 @@
 //    coefficients before it waits for the kernel before it, so launch latency overlaps work.
 // The arithmetic is that of the staged sweeps on the same tables (front-padded blocks of 32, precompute.cpp),
 // element by element, so results are the same bits.
-// One step without rebinning, before and now: 20^3 x 1 41 -> 12 us, 50^3 x 4 53 -> 23, 400 x 300 x 3 35 -> 18,
-// 97 x 61 x 83 x 5 53 -> 47, 100^3 x 4 90 -> 61, 128^3 x 4 103 -> 85; lines beyond 512:
-// 800 x 600 x 4 61 -> 33, 40 x 900 x 3 33 -> 18, 600 x 600 x 20 x 1 162 -> 95.
+// One step without rebinning, before and now, us: 20^3 x 1 41 -> 12, 50^3 x 4 53 -> 23, 400 x 300 x 3 35 -> 18,
+// 97 x 61 x 83 x 5 53 -> 45, 100^3 x 4 90 -> 62, 128^3 x 4 103 -> 80; lines beyond 512: 800 x 600 x 4 61 -> 33,
+// 40 x 900 x 3 33 -> 18, 60 x 60 x 900 x 2 129 -> 74.
 
 #include "small.h"
 #include "sweep_common.cuh"
@@ -33,6 +33,7 @@ struct small_sweep_args
 	int rows, R;			   // x: rows of the field, rows per tile
 	int cols, col_tiles;	   // y, z: columns of a plane
 	int XS, line_stride, outer_stride;
+	int passes;				   // staged: tiles that each warp of a CTA sweeps in turn
 };
 
 // Where a lane's line of a tile lies: AXIS 0, a tile is R = 32 / S whole rows, lane l substrate l % S of row
@@ -74,6 +75,24 @@ struct small_line
 	}
 };
 
+// The staged tables of S substrates and lines of N padded elements: floats, and their copy (rows of N floats:
+// b' of each substrate, then two per row of pairs; a warp copies whole rows).
+__host__ __device__ __forceinline__ int staged_floats(int S, int N) { return S * (3 * N + 12); }
+
+__device__ __forceinline__ void stage_tables(const small_sweep_args& a, float* tab, int warp, int warps)
+{
+	const int N = 32 * a.P, S = a.S;
+	float* pairs = tab + S * (N + 4);
+	for (int row = warp; row < 3 * S; row += warps)
+	{
+		const float4* from = reinterpret_cast<const float4*>(a.ltab + (size_t)row * N);
+		float* to = row < S ? tab + row * (N + 4) : pairs + ((row - S) >> 1) * (2 * N + 8) + ((row - S) & 1) * N;
+		for (int t = threadIdx.x; t < N / 4; t += 32)
+			reinterpret_cast<float4*>(to)[t] = __ldg(from + t);
+	}
+	__syncthreads();
+}
+
 // The coefficients of a block.  With few warps an SM, b' is read ahead of the wait and held in registers,
 // and the responses (tg, G) come from L1: the shortest path for one tile (128 registers a thread).  STAGED,
 // the CTA copies the tables to shared memory ahead of the wait, and 64 registers do: twice the warps, which
@@ -85,27 +104,13 @@ struct small_coefficients
 	const float* bs;
 	const float2* ts;
 
-	// floats of shared memory that the staged tables take
-	static __host__ __device__ __forceinline__ int floats(int S, int N) { return STAGED ? S * (3 * N + 12) : 0; }
-
-	__device__ __forceinline__ small_coefficients(const small_sweep_args& a, int S, int s, int p, float* tab)
+	__device__ __forceinline__ small_coefficients(const small_sweep_args& a, int S, int s, int p, const float* tab)
 	{
 		const int N = 32 * a.P;
 		if constexpr (STAGED)
 		{
-			// rows of N floats: b' of each substrate, then two per row of pairs; a warp copies whole rows
-			float* pairs = tab + S * (N + 4);
-			const int warps = a.P * blockDim.z;
-			for (int row = threadIdx.y + a.P * threadIdx.z; row < 3 * S; row += warps)
-			{
-				const float4* from = reinterpret_cast<const float4*>(a.ltab + (size_t)row * N);
-				float* to = row < S ? tab + row * (N + 4) : pairs + ((row - S) >> 1) * (2 * N + 8) + ((row - S) & 1) * N;
-				for (int t = threadIdx.x; t < N / 4; t += 32)
-					reinterpret_cast<float4*>(to)[t] = __ldg(from + t);
-			}
 			bs = tab + s * (N + 4) + p;
-			ts = reinterpret_cast<const float2*>(pairs + s * (2 * N + 8)) + p;
-			__syncthreads();
+			ts = reinterpret_cast<const float2*>(tab + S * (N + 4) + s * (2 * N + 8)) + p;
 		}
 		else
 		{
@@ -179,20 +184,16 @@ __device__ __forceinline__ void replace_where(float& v, unsigned int on, const f
 	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p ld.global.nc.f32 %0, [%2];\n\t}" : "+f"(v) : "r"(on), "l"(p));
 }
 
-// y and z sweeps.  CTA = (32, P, T): T tiles, warp (j, t) block j of tile t; at most THREADS threads (1024
-// for lines of 17 to 32 blocks, staged).
-template <int AXIS, bool STAGED, int THREADS>
-__global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) small_columns_kernel(const __grid_constant__ small_sweep_args a)
+// One tile of a y or z sweep: block j of its lines by this warp.  tab: the staged tables.
+template <int AXIS, bool STAGED>
+__device__ __forceinline__ void columns_tile(const small_sweep_args& a, int tile, int lane, int j, float* carry_f,
+											 const float* tab)
 {
-	extern __shared__ __align__(16) float small_smem[];
-	let_next_launch();
-	const int lane = threadIdx.x, j = threadIdx.y, P = a.P, p = 32 * j;
-	const int tile = blockIdx.x * blockDim.z + threadIdx.z;
-	float* carry_f = small_smem + threadIdx.z * 2 * P * 32; // [P][32], then carry_t
+	const int P = a.P, p = 32 * j;
 	const small_line<AXIS> l(a, tile, lane, a.S);
 	// coefficients and masks: constant while the solver lives, so they are read ahead of the wait
 	float d[32];
-	const small_coefficients<STAGED> b(a, a.S, l.s, p, small_smem + blockDim.z * 2 * P * 32);
+	const small_coefficients<STAGED> b(a, a.S, l.s, p, tab);
 	const float cs = __ldg(a.vtab + (size_t)96 * P * a.S + l.s);
 	unsigned int mask = a.masks && l.active ? __ldg(&a.masks[((size_t)tile * P + j) * 32 + lane]) : 0u;
 	const int stride = l.stride;
@@ -241,26 +242,38 @@ __global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) sma
 	}
 }
 
-// x sweep: a tile's rows go through shared memory so that global accesses are contiguous.  A row's block is
-// S runs of 32 floats; run i of the tile is run i % S of row i / S, kept at i % S * 32 of row i / S, rows
-// 33 S floats apart so that the lanes' elements fall into distinct banks.  SC: the substrate count where
-// it is fixed at compile time (offsets become immediates), 0 otherwise.  The conditions apply to what is
-// loaded, too: the overwrite before the first sweep of the step.
-template <int SC, bool STAGED, int THREADS>
-__global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) small_rows_kernel(const __grid_constant__ small_sweep_args a)
+// CTA = (32, P, T): T tiles, warp (j, t) block j of tile t; at most THREADS threads (1024 for lines of 17 to
+// 32 blocks, staged).
+template <int AXIS, bool STAGED, int THREADS>
+__global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1)
+	small_columns_kernel(const __grid_constant__ small_sweep_args a)
 {
 	extern __shared__ __align__(16) float small_smem[];
 	let_next_launch();
+	float* tab = small_smem + blockDim.z * a.P * 64;
+	if (STAGED)
+		stage_tables(a, tab, threadIdx.y + a.P * threadIdx.z, a.P * blockDim.z);
+	for (int k = 0; k < (STAGED ? a.passes : 1); k++)
+		columns_tile<AXIS, STAGED>(a, (blockIdx.x * (STAGED ? a.passes : 1) + k) * blockDim.z + threadIdx.z, threadIdx.x,
+								   threadIdx.y, small_smem + threadIdx.z * a.P * 64, tab);
+}
+
+// One tile of an x sweep: its rows go through shared memory (buf, 33 * 32 floats of this warp) so that global
+// accesses are contiguous.  A row's block is S runs of 32 floats; run i of the tile is run i % S of row i / S,
+// kept at i % S * 32 of row i / S, rows 33 S floats apart so that the lanes' elements fall into distinct banks.
+// SC: the substrate count (so that offsets are immediates), or 0 for 17 to 32 of them, one row per tile.  The
+// conditions apply to what is loaded, too: the overwrite before the first sweep of the step.
+template <int SC, bool STAGED>
+__device__ __forceinline__ void rows_tile(const small_sweep_args& a, int tile, int lane, int j, float* carry_f, float* buf,
+										  const float* tab)
+{
 	const int S = SC ? SC : a.S;
 	constexpr int RUNS = SC ? 32 / (SC ? SC : 1) * SC : 32;
-	const int lane = threadIdx.x, j = threadIdx.y, P = a.P, p = 32 * j;
-	const int tile = blockIdx.x * blockDim.z + threadIdx.z;
-	float* carry_f = small_smem + threadIdx.z * 2 * P * 32;
-	float* buf = small_smem + blockDim.z * 2 * P * 32 + (threadIdx.z * P + j) * (33 * 32);
+	const int P = a.P, p = 32 * j;
 	const int pitch = 33 * S;
 	const small_line<0> l(a, tile, lane, S);
 	float d[32];
-	const small_coefficients<STAGED> b(a, S, l.s, p, small_smem + blockDim.z * P * (64 + 33 * 32));
+	const small_coefficients<STAGED> b(a, S, l.s, p, tab);
 	const float cs = __ldg(a.vtab + (size_t)96 * P * S + l.s);
 	const unsigned int mask = a.masks && l.active ? __ldg(&a.masks[((size_t)tile * P + j) * 32 + lane]) : 0u;
 	const int skip = j == 0 ? a.pad * S : 0; // floats of a row's block before the line
@@ -271,34 +284,18 @@ __global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) sma
 
 	// f(run, offset of the lane's float in the field, offset in the buffer, whether it exists)
 	auto runs = [&](auto&& f) {
-		int r = 0, q = 0;
 #pragma unroll
 		for (int i = 0; i < RUNS; i++)
 		{
-			if (SC)
-			{
-				r = i / (SC ? SC : 1);
-				q = i - r * SC;
-			}
-			f(i, (long long)r * a.XS + 32 * q, r * pitch + 32 * q + lane, r < l.rows && 32 * q + lane >= skip);
-			if (!SC && ++q == S)
-			{
-				q = 0;
-				r++;
-			}
+			const int r = SC ? i / (SC ? SC : 1) : 0, q = SC ? i - r * SC : i;
+			f(i, (long long)r * a.XS + 32 * q, r * pitch + 32 * q + lane, r < l.rows && q < S && 32 * q + lane >= skip);
 		}
 	};
 	if (SC && whole)
 		runs([&](int i, long long o, int, bool) { d[i] = base[o]; });
 	else
 		runs([&](int i, long long o, int, bool in) { d[i] = in ? base[o] : 0.f; });
-	if (SC)
-		runs([&](int i, long long, int t, bool) { buf[t] = d[i]; });
-	else
-		runs([&](int i, long long, int t, bool in) {
-			if (in || t < 33 * 32)
-				buf[t] = d[i];
-		});
+	runs([&](int i, long long, int t, bool) { buf[t] = d[i]; });
 	__syncwarp();
 	const long long line = l.at + (long long)(p - a.pad) * S; // offset of the block's element 0
 #pragma unroll
@@ -333,6 +330,24 @@ __global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1) sma
 		});
 }
 
+template <int SC, bool STAGED, int THREADS>
+__global__ void __launch_bounds__(THREADS, STAGED && THREADS <= 512 ? 2 : 1)
+	small_rows_kernel(const __grid_constant__ small_sweep_args a)
+{
+	extern __shared__ __align__(16) float small_smem[];
+	let_next_launch();
+	float* bufs = small_smem + blockDim.z * a.P * 64;
+	float* tab = bufs + blockDim.z * a.P * (33 * 32);
+	if (STAGED)
+		stage_tables(a, tab, threadIdx.y + a.P * threadIdx.z, a.P * blockDim.z);
+	for (int k = 0; k < (STAGED ? a.passes : 1); k++)
+	{
+		rows_tile<SC, STAGED>(a, (blockIdx.x * (STAGED ? a.passes : 1) + k) * blockDim.z + threadIdx.z, threadIdx.x, threadIdx.y,
+							  small_smem + threadIdx.z * a.P * 64, bufs + (threadIdx.z * a.P + threadIdx.y) * (33 * 32), tab);
+		__syncwarp(); // the next tile's rows go to the same buffer
+	}
+}
+
 // Bit k of word (tile, block, lane): element k of the lane's block has a condition.
 template <int AXIS>
 __global__ void __launch_bounds__(256) small_masks_kernel(const __grid_constant__ small_sweep_args a,
@@ -360,13 +375,13 @@ __global__ void __launch_bounds__(256) small_masks_kernel(const __grid_constant_
 // shared memory of a CTA of T tiles
 static size_t sweep_smem(int axis, int P, int S, int T, bool staged)
 {
-	return ((size_t)T * P * (64 + (axis == 0 ? 33 * 32 : 0)) + (staged ? small_coefficients<true>::floats(S, 32 * P) : 0))
+	return ((size_t)T * P * (64 + (axis == 0 ? 33 * 32 : 0)) + (staged ? staged_floats(S, 32 * P) : 0))
 		   * sizeof(float);
 }
 
 bool small_mesh(const bfvm_solver* s)
 {
-	if (s->slab_count > 1 || s->S > 32 || s->V * s->S > SMALL_ELEMENTS)
+	if (s->slab_count > 1 || s->S > 32 || s->V * s->S > small_elements(s->S))
 		return false;
 	// lines of up to 32 blocks, in CTAs of up to 1024 threads, whose buffers and tables fit a CTA's 227 KB
 	for (int d = 0; d < s->dims; d++)
@@ -405,6 +420,7 @@ static small_sweep_args sweep_args_of(const bfvm_solver* s)
 	a.col_tiles = (a.cols + 31) / 32;
 	a.line_stride = a.cols;
 	a.outer_stride = AXIS == 1 ? a.XS * Y : 0;
+	a.passes = 1;
 	a.tiles = AXIS == 0 ? (a.rows + a.R - 1) / a.R : a.col_tiles * (AXIS == 1 ? Z : 1);
 	return a;
 }
@@ -413,15 +429,28 @@ template <int AXIS, bool STAGED, int THREADS>
 static void (*small_kernel(int S))(const small_sweep_args)
 {
 	if constexpr (AXIS == 0)
-		return S == 1	 ? small_rows_kernel<1, STAGED, THREADS>
-			   : S == 2	 ? small_rows_kernel<2, STAGED, THREADS>
-			   : S == 3	 ? small_rows_kernel<3, STAGED, THREADS>
-			   : S == 4	 ? small_rows_kernel<4, STAGED, THREADS>
-			   : S == 5	 ? small_rows_kernel<5, STAGED, THREADS>
-			   : S == 6	 ? small_rows_kernel<6, STAGED, THREADS>
-			   : S == 8	 ? small_rows_kernel<8, STAGED, THREADS>
-			   : S == 16 ? small_rows_kernel<16, STAGED, THREADS>
-						 : small_rows_kernel<0, STAGED, THREADS>;
+	{
+		switch (S)
+		{
+		case 1: return small_rows_kernel<1, STAGED, THREADS>;
+		case 2: return small_rows_kernel<2, STAGED, THREADS>;
+		case 3: return small_rows_kernel<3, STAGED, THREADS>;
+		case 4: return small_rows_kernel<4, STAGED, THREADS>;
+		case 5: return small_rows_kernel<5, STAGED, THREADS>;
+		case 6: return small_rows_kernel<6, STAGED, THREADS>;
+		case 7: return small_rows_kernel<7, STAGED, THREADS>;
+		case 8: return small_rows_kernel<8, STAGED, THREADS>;
+		case 9: return small_rows_kernel<9, STAGED, THREADS>;
+		case 10: return small_rows_kernel<10, STAGED, THREADS>;
+		case 11: return small_rows_kernel<11, STAGED, THREADS>;
+		case 12: return small_rows_kernel<12, STAGED, THREADS>;
+		case 13: return small_rows_kernel<13, STAGED, THREADS>;
+		case 14: return small_rows_kernel<14, STAGED, THREADS>;
+		case 15: return small_rows_kernel<15, STAGED, THREADS>;
+		case 16: return small_rows_kernel<16, STAGED, THREADS>;
+		default: return small_rows_kernel<0, STAGED, THREADS>;
+		}
+	}
 	else
 		return small_columns_kernel<AXIS, STAGED, THREADS>;
 }
@@ -429,7 +458,7 @@ static void (*small_kernel(int S))(const small_sweep_args)
 template <int AXIS>
 static int launch_small_sweep(bfvm_solver* s, bool overlap)
 {
-	const small_sweep_args a = sweep_args_of<AXIS>(s);
+	small_sweep_args a = sweep_args_of<AXIS>(s);
 	// CTAs of about four warps: lines of few blocks share one
 	const int T = std::max(1, std::min(4 / a.P, (a.tiles + sm_count_impl(s->device) - 1) / sm_count_impl(s->device)));
 	// more warps than the registers of the fuller form let reside, or lines that need 1024 threads
@@ -438,10 +467,20 @@ static int launch_small_sweep(bfvm_solver* s, bool overlap)
 											 : staged ? small_kernel<AXIS, true, 512>(a.S)
 													  : small_kernel<AXIS, false, 512>(a.S);
 	const size_t smem = sweep_smem(AXIS, a.P, a.S, T, staged);
+	// staged, the CTAs that are resident together sweep all tiles, so that the tables (as large as a tile at
+	// 16 substrates) are staged once
+	const long long groups = (a.tiles + T - 1) / T;
+	a.passes = 1;
+	if (staged)
+	{
+		const long long slots =
+			(long long)sm_count_impl(s->device) * std::max<long long>(1, std::min<long long>(32 / (T * a.P), 225 * 1024 / (long long)(smem + 1024)));
+		a.passes = (int)((groups + slots - 1) / slots);
+	}
 	int st;
 	if ((st = set_smem(kernel, smem)))
 		return st;
-	return launch_overlapped(s, "small sweep", kernel, dim3((unsigned)((a.tiles + T - 1) / T)), dim3(32, a.P, T), smem,
+	return launch_overlapped(s, "small sweep", kernel, dim3((unsigned)((groups + a.passes - 1) / a.passes)), dim3(32, a.P, T), smem,
 							 overlap, a);
 }
 

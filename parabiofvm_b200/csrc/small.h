@@ -7,10 +7,15 @@
 
 namespace bfvm {
 
-// Fields of at most this many elements take the kernels of small.cu.  At this size (128^3 x 4) a sweep here
-// takes 18 to 22 us against 24 staged; the staged sweeps stream larger fields from HBM faster (109 to 124 us
-// at 250^3 x 4, where 128^3's rate would make 136).
-static constexpr long long SMALL_ELEMENTS = 1LL << 23;
+// The kernels of small.cu take fields of at most this many elements: beyond, the staged sweeps, which copy
+// ahead of the solve, stream faster, the sooner the more a warp's 32 lines spread over substrates (their
+// tables are staged for each CTA).  A step staged and here, us: 220^3 x 1 186 / 110, 200^3 x 2 221 / 187;
+// 128^3 x 4 96 / 80, 160^3 x 4 157 / 160; 72^3 x 12 84 / 72, 91^3 x 8 84 / 73, 90^3 x 7 72 / 78, 101 x 103 x
+// 97 x 6 80 / 86, 80^3 x 16 98 / 109; 40^3 x 24 58 / 51, 50^3 x 32 78 / 83.
+inline long long small_elements(int S)
+{
+	return S <= 2 ? 1LL << 24 : S <= 4 ? 1LL << 23 : S <= 16 ? 9LL << 19 : 1LL << 21;
+}
 static constexpr unsigned int SMALL_FREE = 0xffffffffu; // no condition in bfvm_solver::dir_dense (a NaN)
 
 // the mesh's shape is one that small.cu takes; its step runs there (no option names the other kernels)

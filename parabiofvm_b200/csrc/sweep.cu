@@ -259,8 +259,9 @@ static int sweep_axis(bfvm_solver* st, int axis, const sweep_args& a, bool& stag
 	staged = false;
 	// lines longer than the chunk length (chunk_elements; always beyond 512): the staged sweep of
 	// their chunks with their carries (chunks.cu).  Not `staged` for the caller: the chunks write no
-	// per-tile overwrite, face condition or gradient.
-	if (st->use_tma && pl.chunks.count > 0)
+	// per-tile overwrite, face condition or gradient.  Small meshes sweep whole lines whatever the
+	// options, as their step does (small.cu), unless a chunk length is asked for.
+	if (st->use_tma && pl.chunks.count > 0 && !(st->chunk_elements == 0 && small_mesh(st)))
 	{
 		rc = launch_chunked_sweep(st, axis, handled);
 		if (rc || handled)

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 SHAPES = [((2, 2, 2), 1), ((31, 5, 3), 2), ((32, 33, 2), 3), ((33, 32, 31), 4), ((64, 65, 3), 5), ((3, 64, 65), 6),
           ((97, 9, 34), 7), ((40, 41, 42), 8), ((65, 4, 40), 12), ((34, 33, 20), 16), ((36, 10, 7), 17),
           ((33, 6, 5), 32), ((512, 5, 4), 1), ((4, 512, 3), 4), ((3, 4, 500), 3), ((300, 257), 3), ((20, 700), 2),
-          ((45, 31), 16), ((500,), 4), ((2,), 32), ((128, 100, 80), 8),
+          ((45, 31), 16), ((33, 5, 34), 9), ((21, 40, 9), 11), ((500,), 4), ((2,), 32), ((128, 100, 80), 8),
           ((513, 4, 3), 3), ((3, 700, 5), 4), ((4, 3, 1024), 2), ((1000, 30), 5), ((30, 999), 1), ((1024,), 6)]
 
 
