@@ -207,8 +207,11 @@ __global__ void scan_add_kernel(int* out, long long n, const int* tile_offsets);
 static constexpr int BIN_BLOCK_AGENTS = 16384;
 
 // bins.cu: the agents' order by voxel (agent_state::keys, vals) and its segments, on the solver's
-// stream; the buffers this needs for `count` agents
-int launch_bins(bfvm_solver* s);
+// stream (follows: launched ahead of the end of a kernel of small.h's kind); the buffers this needs for
+// `count` agents; the 16-byte units of scratch that the last kernel of a binning clears, and the scratch
+// after a wait that ran out
+int launch_bins(bfvm_solver* s, bool follows);
+long long bins_dirty(const bfvm_solver* s);
 int bins_alloc(bfvm_solver* s, int count);
 
 // number of 8-bit radix passes for keys in [0, V] (V marks agents outside the mesh)

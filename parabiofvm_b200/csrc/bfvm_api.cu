@@ -179,6 +179,9 @@ int check_device_errors(bfvm_solver* s)
 	if (e)
 	{
 		BFVM_CUDA(cudaMemsetAsync(s->dev_error, 0, sizeof(int), s->stream));
+		int st;
+		if ((e & DEVERR_TIMEOUT) && (st = bins_reset(s)))
+			return st;
 		if (e & DEVERR_TIMEOUT)
 			return fail(BFVM_ERR_TIMEOUT, "a sweep kernel timed out waiting for a tile copy; the field is not valid");
 		if (e & DEVERR_AGENT_OUTSIDE)

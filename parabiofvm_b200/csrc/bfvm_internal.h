@@ -339,6 +339,7 @@ bool agents_rebin(const bfvm_solver* s, bool recompute);
 // the binning and the agent terms' order a secretion update needs (a rebinning when `recompute`)
 int prepare_agent_terms(bfvm_solver* s, bool recompute);
 int agents_unsort(bfvm_solver* s, bool keep_sorted); // internalized amounts back to agent order (cell.cu)
+int bins_reset(bfvm_solver* s); // the binning's scratch after a wait that ran out (bins.cu)
 int solver_drop_graphs(bfvm_solver* s);			  // after queued work, drop the step graphs (bfvm_api.cu)
 int agents_resort_internalized(bfvm_solver* s);	  // stored internalized amounts into sorted order
 int launch_release(bfvm_solver* s, int index);

@@ -4,13 +4,16 @@
 // The order is a stable LSD radix sort of (voxel key, agent index); agents outside the mesh carry the
 // key V and sort to the end.  Two forms:
 //  - up to BIN_BLOCK_AGENTS agents, one CTA does all of it (keys, sort, segments) in shared memory: a
-//    launch costs more than its share of the work there, and the multi-CTA form needs 3 + passes of them;
+//    launch costs more than its share of the work there, and the multi-CTA form needs 2 + passes of them;
 //  - beyond that, a kernel computes the keys and the digit histograms of every pass, one kernel per
 //    digit ranks and scatters (single-pass radix sort with decoupled look-back, after Adinets and
 //    Merrill, "Onesweep", 2022), and one finds the segments with the same look-back.
 // The sort was three or more launches per digit (histogram, scan, scatter) and five for the segments, 22 to
 // 28 in all.  One step with rebinning at 100^3 x 4 with 50,000 agents: 200 -> 145 us; ten steps (one
 // rebinning) at 50^3 x 4 with 5,000: 616 -> 571 us, at 128^3 x 4 with 200,000: 1179 -> 1109 us.
+// The one-CTA form and what follows it launch ahead of their predecessors' ends (small.h), so what one writes
+// the next reads with ordinary loads.  The multi-CTA form does not: beside a captured step's diffusion, CTAs
+// that wait hold the registers that the sweeps need (250^3 x 4, a step with rebinning: 1198 us against 1006).
 // CTAs of the look-back kernels take their tiles from a counter, so a tile only ever waits for tiles
 // whose CTAs already run; the waits are bounded, and one that runs out raises DEVERR_TIMEOUT and the
 // scratch's abort word, after which the remaining kernels leave at once with no segments.  What is left
@@ -21,6 +24,7 @@
 
 #include "agent_kernels.cuh"
 #include "sm100_common.cuh"
+#include "small.h"
 #include "sweep_common.cuh"
 
 namespace bfvm {
@@ -95,6 +99,8 @@ __global__ void __launch_bounds__(THREADS, 1) bin_block_kernel(const __grid_cons
 	unsigned int key[BLOCK_ITEMS];
 	unsigned int vr[BLOCK_ITEMS]; // agent index << 16 | rank
 	bool outside = false;
+	let_next_launch();
+	wait_previous();
 	// the positions of four rounds are loaded before any is used
 #pragma unroll
 	for (int r0 = 0; r0 < BLOCK_ITEMS; r0 += 4)
@@ -264,16 +270,19 @@ __global__ void __launch_bounds__(THREADS, 1) bin_block_kernel(const __grid_cons
 static constexpr int PASS_THREADS = 512;
 static constexpr int PASS_WARPS = PASS_THREADS / 32;
 static constexpr int MAX_PASSES = 4;
+static constexpr int PASS_BITS = 10; // of a digit, at most: two passes for a million voxels
+static constexpr int DIGITS = 1 << PASS_BITS;
 // a tile's published count: a state in the high word, the count in the low
 static constexpr unsigned long long TILE_SUM = 1ull << 32;	 // of the tile alone
 static constexpr unsigned long long TILE_TOTAL = 2ull << 32; // of the tile and all before it
 
-// scratch of the multi-CTA form, zeroed before each binning
+// Scratch of the multi-CTA form, followed by the tiles' states.  It is zero before each binning: allocated so,
+// and cleared by the last kernel of each (bins_clear), which saves two memory-set nodes in front of the next.
 struct bin_state
 {
 	int abort;
 	int ticket[MAX_PASSES + 1];
-	int hist[MAX_PASSES][256];
+	int hist[MAX_PASSES][DIGITS];
 };
 
 __device__ __forceinline__ unsigned long long tile_load(const unsigned long long* p)
@@ -317,23 +326,61 @@ __device__ __forceinline__ bool look_back(const unsigned long long* state, long 
 	return true;
 }
 
-// keys of the agents, and the digit histograms of every pass
-__global__ void __launch_bounds__(PASS_THREADS) bin_keys_kernel(const float* __restrict__ pos, int A, int dims, int3 bmin,
-																 int3 vox, int3 grid, unsigned int* __restrict__ keys,
-																 unsigned int invalid, int passes, int bits,
-																 bin_state* __restrict__ st, int* __restrict__ err)
+// The same for one count per tile, by a warp: 32 tiles at a time.
+__device__ __forceinline__ bool warp_look_back(const unsigned long long* state, int tile, int lane, const volatile int* abort_word,
+											   int& sum)
 {
-	__shared__ int h[MAX_PASSES][256];
-	for (int t = threadIdx.x; t < MAX_PASSES * 256; t += PASS_THREADS)
-		h[t >> 8][t & 255] = 0;
+	sum = 0;
+	const long long t0 = clock64();
+	int t = tile - 1; // the nearest tile not yet counted
+	for (;;)
+	{
+		const unsigned long long v = t - lane >= 0 ? tile_load(state + t - lane) : TILE_TOTAL;
+		const unsigned int ready = __ballot_sync(0xffffffffu, (v >> 32) != 0);
+		const unsigned int totals = __ballot_sync(0xffffffffu, (v & TILE_TOTAL) != 0);
+		// count up to the nearest total, if every tile before it is ready, or all 32
+		const int upto = totals ? __ffs(totals) - 1 : 31;
+		const unsigned int need = upto == 31 ? 0xffffffffu : (2u << upto) - 1u;
+		if ((ready & need) == need)
+		{
+			int n = lane <= upto ? (int)(unsigned int)v : 0;
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1)
+				n += __shfl_xor_sync(0xffffffffu, n, o);
+			sum += n;
+			if (totals)
+				return true;
+			t -= 32;
+			continue;
+		}
+		const bool give_up = clock64() - t0 > WAIT_LIMIT_CYCLES || *abort_word;
+		if (__any_sync(0xffffffffu, give_up))
+			return false;
+	}
+}
+
+// keys of the agents, and the digit histograms of every pass
+__global__ void __launch_bounds__(PASS_THREADS) bin_keys_kernel(const float* pos, int A, int dims, int3 bmin, int3 vox,
+																 int3 grid, unsigned int* keys, unsigned int invalid, int passes,
+																 int bits, bin_state* st, int* counts, int* err)
+{
+	__shared__ int h[MAX_PASSES][DIGITS];
+	let_next_launch();
+	for (int t = threadIdx.x; t < MAX_PASSES * DIGITS; t += PASS_THREADS)
+		h[t / DIGITS][t % DIGITS] = 0;
 	__syncthreads();
+	wait_previous();
+	if (blockIdx.x == 0 && threadIdx.x < 3)
+		counts[threadIdx.x] = 0; // no segments, should no agent be inside
 	const unsigned int mask = (1u << bits) - 1u;
 	bool outside = false;
 	for (long long i = blockIdx.x * (long long)PASS_THREADS + threadIdx.x; i < A; i += (long long)gridDim.x * PASS_THREADS)
 	{
+		float x[3];
 		int3 c;
 		unsigned int k = invalid;
-		if (voxel_of(pos + (size_t)i * dims, dims, bmin, vox, grid, c))
+		load_position(pos, i, dims, x);
+		if (voxel_of(x, dims, bmin, vox, grid, c))
 			k = (unsigned int)c.x + (unsigned int)grid.x * ((unsigned int)c.y + (unsigned int)grid.y * (unsigned int)c.z);
 		else
 			outside = true;
@@ -344,36 +391,34 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_keys_kernel(const float* __r
 	if (outside)
 		atomicOr(err, DEVERR_AGENT_OUTSIDE);
 	__syncthreads();
-	for (int t = threadIdx.x; t < passes * 256; t += PASS_THREADS)
-	{
-		const int n = h[t >> 8][t & 255];
-		if (n)
-			atomicAdd(&st->hist[t >> 8][t & 255], n);
-	}
+	for (int p = 0; p < passes; p++)
+		for (int t = threadIdx.x; t <= (int)mask; t += PASS_THREADS)
+			if (h[p][t])
+				atomicAdd(&st->hist[p][t], h[p][t]);
 }
 
 // One digit: a tile of PASS_THREADS * ITEMS keys is ranked within the CTA, its digit counts are joined
 // with those of the tiles before it, and its keys go to their places.  vin null: agent indices (the
 // first pass).
 template <int ITEMS>
-__global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned int* __restrict__ kin,
-																 const int* __restrict__ vin,
-																 unsigned int* __restrict__ kout, int* __restrict__ vout,
-																 int n, int pass, int bits, bin_state* st,
-																 unsigned long long* state, int* __restrict__ err)
+__global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned int* kin, const int* vin, unsigned int* kout,
+																 int* vout, int n, int pass, int bits, bin_state* st,
+																 unsigned long long* state, int* err)
 {
-	__shared__ int cnt[PASS_WARPS][256];
-	__shared__ int place[256]; // where the tile's first key of a digit goes
-	__shared__ int wtot[8];
+	__shared__ unsigned short cnt[PASS_WARPS][DIGITS];
+	__shared__ int place[DIGITS]; // where the tile's first key of a digit goes
+	__shared__ int wtot[PASS_WARPS];
 	__shared__ int tile_s, stop;
+	let_next_launch();
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	for (int t = tid; t < PASS_WARPS * DIGITS / 2; t += PASS_THREADS)
+		reinterpret_cast<unsigned int*>(&cnt[0][0])[t] = 0;
+	wait_previous();
 	if (tid == 0)
 	{
 		tile_s = atomicAdd(&st->ticket[pass], 1);
 		stop = *reinterpret_cast<volatile int*>(&st->abort);
 	}
-	for (int t = tid; t < PASS_WARPS * 256; t += PASS_THREADS)
-		cnt[t >> 8][t & 255] = 0;
 	__syncthreads();
 	if (stop)
 		return;
@@ -399,54 +444,62 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 		const int before = cnt[warp][d];
 		__syncwarp();
 		if (in && (peers & below) == 0)
-			cnt[warp][d] = before + __popc(peers);
+			cnt[warp][d] = (unsigned short)(before + __popc(peers));
 		__syncwarp();
 		rank[r] = before + __popc(peers & below);
 	}
 	__syncthreads();
-	int total = 0, gincl = 0, gown = 0;
-	if (tid < 256)
+	// thread t counts and places `per` digits from t per
+	const int per = mask >= PASS_THREADS ? 2 : 1, d0 = tid * per;
+	const bool mine = d0 <= (int)mask;
+	int total[2] = { 0, 0 }, own[2] = { 0, 0 }, incl = 0;
+	if (mine)
+		for (int k = 0; k < per; k++)
+		{
+#pragma unroll
+			for (int w = 0; w < PASS_WARPS; w++)
+			{
+				const int c = cnt[w][d0 + k];
+				cnt[w][d0 + k] = (unsigned short)total[k];
+				total[k] += c;
+			}
+			tile_publish(state + (((long long)tile << bits) + d0 + k), (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total[k]);
+			own[k] = st->hist[pass][d0 + k];
+		}
+	// keys of smaller digits: exclusive scan of the pass's histogram
+	incl = own[0] + own[1];
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1)
 	{
-#pragma unroll
-		for (int w = 0; w < PASS_WARPS; w++)
-		{
-			const int c = cnt[w][tid];
-			cnt[w][tid] = total;
-			total += c;
-		}
-		tile_publish(state + (long long)tile * 256 + tid, (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total);
-		// keys of smaller digits: exclusive scan of the pass's histogram
-		gown = st->hist[pass][tid];
-		gincl = gown;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1)
-		{
-			const int up = __shfl_up_sync(0xffffffffu, gincl, o);
-			if (lane >= o)
-				gincl += up;
-		}
-		if (lane == 31)
-			wtot[warp] = gincl;
+		const int up = __shfl_up_sync(0xffffffffu, incl, o);
+		if (lane >= o)
+			incl += up;
 	}
+	if (lane == 31)
+		wtot[warp] = incl;
 	__syncthreads();
-	if (tid < 256)
+	if (mine)
 	{
-		int smaller = gincl - gown;
+		int smaller = incl - own[0] - own[1];
 		for (int w = 0; w < warp; w++)
 			smaller += wtot[w];
-		int before = 0;
-		if (tile > 0)
+		for (int k = 0; k < per; k++)
 		{
-			if (!look_back(state + tid, 256, tile, &st->abort, before))
+			int before = 0;
+			if (tile > 0)
 			{
-				atomicOr(err, DEVERR_TIMEOUT);
-				atomicExch(&st->abort, 1);
-				stop = 1;
+				if (!look_back(state + d0 + k, 1LL << bits, tile, &st->abort, before))
+				{
+					atomicOr(err, DEVERR_TIMEOUT);
+					atomicExch(&st->abort, 1);
+					stop = 1;
+				}
+				else
+					tile_publish(state + (((long long)tile << bits) + d0 + k), TILE_TOTAL | (unsigned int)(before + total[k]));
 			}
-			else
-				tile_publish(state + (long long)tile * 256 + tid, TILE_TOTAL | (unsigned int)(before + total));
+			place[d0 + k] = smaller + before;
+			smaller += own[k];
 		}
-		place[tid] = smaller + before;
 	}
 	__syncthreads();
 	if (stop)
@@ -464,14 +517,15 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 
 // Segments of the sorted keys (the outputs of bin_block_kernel); counts starts zeroed.
 template <int ITEMS>
-__global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsigned int* __restrict__ keys, int n,
-																	 unsigned int invalid, int* __restrict__ seg_start,
-																	 int* __restrict__ counts, bin_state* st,
-																	 unsigned long long* state, int* __restrict__ err)
+__global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsigned int* keys, int n, unsigned int invalid,
+																	 int* seg_start, int* counts, bin_state* st,
+																	 unsigned long long* state, int* err)
 {
 	__shared__ int wsum[PASS_WARPS];
 	__shared__ int tile_s, stop, before_s;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	let_next_launch();
+	wait_previous();
 	if (tid == 0)
 	{
 		tile_s = atomicAdd(&st->ticket[MAX_PASSES], 1);
@@ -514,22 +568,24 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsign
 			ahead = total;
 		total += wsum[w];
 	}
-	if (tid == 0)
+	if (warp == 0)
 	{
-		tile_publish(state + tile, (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total);
+		if (lane == 0)
+			tile_publish(state + tile, (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total);
 		int before = 0;
-		if (tile > 0)
+		const bool found = tile == 0 || warp_look_back(state, tile, lane, &st->abort, before);
+		if (lane == 0)
 		{
-			if (!look_back(state, 1, tile, &st->abort, before))
+			if (!found)
 			{
 				atomicOr(err, DEVERR_TIMEOUT);
 				atomicExch(&st->abort, 1);
 				stop = 1;
 			}
-			else
+			else if (tile > 0)
 				tile_publish(state + tile, TILE_TOTAL | (unsigned int)(before + total));
+			before_s = before;
 		}
-		before_s = before;
 	}
 	__syncthreads();
 	if (stop)
@@ -571,11 +627,40 @@ int bins_alloc(bfvm_solver* s, int count)
 		return BFVM_OK;
 	// the most tiles of any count up to this one
 	const long long tiles = std::max(state_tiles(count), state_tiles(std::min(count, SMALL_TILE_AGENTS)));
-	a.bin_state_bytes = (sizeof(bin_state) + 255) / 256 * 256 + (size_t)tiles * (MAX_PASSES * 256 + 1) * sizeof(unsigned long long);
+	a.bin_state_bytes = (sizeof(bin_state) + 255) / 256 * 256 + (size_t)tiles * (MAX_PASSES * DIGITS + 1) * sizeof(unsigned long long);
 	if ((st = device_alloc(&a.bin_state, a.bin_state_bytes)) || (st = device_alloc(&a.keys_alt, (size_t)count))
 		|| (st = device_alloc(&a.vals_alt, (size_t)count)))
 		return st;
 	BFVM_CUDA(cudaMemsetAsync(a.vals_alt, 0, (size_t)count * sizeof(int), s->stream));
+	BFVM_CUDA(cudaMemsetAsync(a.bin_state, 0, a.bin_state_bytes, s->stream));
+	return BFVM_OK;
+}
+
+// radix passes of the multi-CTA form and their bits
+static int pass_count(const bfvm_solver* s, int& bits)
+{
+	int total = 1; // keys take the values 0 .. V
+	while (total < 32 && ((1ull << total) <= (unsigned long long)s->V))
+		total++;
+	const int passes = (total + PASS_BITS - 1) / PASS_BITS;
+	bits = (total + passes - 1) / passes;
+	return passes;
+}
+
+// What a binning of the present agents leaves in its scratch, in 16-byte units: cleared by the kernel that ends
+// it (whose abort word is zero then).
+long long bins_dirty(const bfvm_solver* s)
+{
+	int bits;
+	const long long passes = pass_count(s, bits), states = state_tiles(s->ag.count) * ((passes << bits) + 1);
+	return ((long long)(sizeof(bin_state) + 255) / 256 * 256 + states * (long long)sizeof(unsigned long long) + 15) / 16;
+}
+
+// After a wait that ran out: the scratch as it was when allocated.
+int bins_reset(bfvm_solver* s)
+{
+	if (s->ag.bin_state)
+		BFVM_CUDA(cudaMemsetAsync(s->ag.bin_state, 0, s->ag.bin_state_bytes, s->stream));
 	return BFVM_OK;
 }
 
@@ -593,19 +678,17 @@ static int launch_tiles(bfvm_solver* s, bin_state* st, unsigned long long* tiles
 	int* vout = passes % 2 ? a.vals : a.vals_alt;
 	for (int p = 0; p < passes; p++)
 	{
-		bin_pass_kernel<ITEMS><<<grid, PASS_THREADS, 0, s->stream>>>(kin, p ? vin : nullptr, kout, vout, A, p, bits, st,
-																	 tiles + (size_t)p * 256 * grid, s->dev_error);
-		if ((rc = check_launch(s, "bin_pass_kernel")))
+		if ((rc = launch_overlapped(s, "bin_pass_kernel", bin_pass_kernel<ITEMS>, dim3(grid), dim3(PASS_THREADS), 0, false, kin,
+									p ? vin : nullptr, kout, vout, A, p, bits, st, tiles + ((size_t)p << bits) * grid, s->dev_error)))
 			return rc;
 		std::swap(kin, kout);
 		std::swap(vin, vout);
 	}
-	bin_segments_kernel<ITEMS><<<grid, PASS_THREADS, 0, s->stream>>>(
-		a.keys, A, invalid, a.seg_start, a.seg_count_dev, st, tiles + (size_t)passes * 256 * grid, s->dev_error);
-	return check_launch(s, "bin_segments_kernel");
+	return launch_overlapped(s, "bin_segments_kernel", bin_segments_kernel<ITEMS>, dim3(grid), dim3(PASS_THREADS), 0, false, a.keys,
+							 A, invalid, a.seg_start, a.seg_count_dev, st, tiles + ((size_t)passes << bits) * grid, s->dev_error);
 }
 
-int launch_bins(bfvm_solver* s)
+int launch_bins(bfvm_solver* s, bool follows)
 {
 	agent_state& a = s->ag;
 	const int A = a.count;
@@ -627,22 +710,19 @@ int launch_bins(bfvm_solver* s)
 							 bmin, vox, grid, invalid, passes, bits };
 			if ((st = set_smem(kernel, shape.smem(BIN_BLOCK_AGENTS, shape.BITS))))
 				return st;
-			kernel<<<1, THREADS, shape.smem(A, bits), s->stream>>>(j);
-			return check_launch(s, "bin_block_kernel");
+			return launch_overlapped(s, "bin_block_kernel", kernel, dim3(1), dim3(THREADS), shape.smem(A, bits), follows, j);
 		};
 		return A <= 1024 ? launch(block_shape<256>(), bin_block_kernel<256>) : launch(block_shape<1024>(), bin_block_kernel<1024>);
 	}
-	const int passes = sort_passes(s->V), bits = (total + passes - 1) / passes;
-	BFVM_CUDA(cudaMemsetAsync(a.seg_count_dev, 0, 4 * sizeof(int), s->stream));
-	BFVM_CUDA(cudaMemsetAsync(a.bin_state, 0, a.bin_state_bytes, s->stream));
+	int bits;
+	const int passes = pass_count(s, bits);
 	bin_state* bs = reinterpret_cast<bin_state*>(a.bin_state);
 	unsigned long long* tiles =
 		reinterpret_cast<unsigned long long*>(a.bin_state + (sizeof(bin_state) + 255) / 256 * 256);
 	const unsigned ctas = (unsigned)std::min<long long>((A + PASS_THREADS - 1) / PASS_THREADS, 2LL * sm_count_impl(s->device));
-	bin_keys_kernel<<<ctas, PASS_THREADS, 0, s->stream>>>(a.pos, A, s->dims, bmin, vox, grid,
-														   passes % 2 ? a.keys_alt : a.keys, invalid, passes, bits, bs,
-														   s->dev_error);
-	if ((st = check_launch(s, "bin_keys_kernel")))
+	if ((st = launch_overlapped(s, "bin_keys_kernel", bin_keys_kernel, dim3(ctas), dim3(PASS_THREADS), 0, false, a.pos, A,
+								s->dims, bmin, vox, grid, passes % 2 ? a.keys_alt : a.keys, invalid, passes, bits, bs,
+								a.seg_count_dev, s->dev_error)))
 		return st;
 	return tile_items(A) == 2 ? launch_tiles<2>(s, bs, tiles, invalid, passes, bits)
 							  : launch_tiles<8>(s, bs, tiles, invalid, passes, bits);

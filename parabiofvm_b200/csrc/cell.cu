@@ -200,7 +200,8 @@ __global__ void reduce_kernel(long long total, int S, const int* __restrict__ co
 	red_fac[t] = rf;
 }
 
-// V consecutive substrates of a row: four as one 16-byte access (S % 4 == 0), else one.
+// V consecutive substrates of a row: four as one 16-byte access (S % 4 == 0), else one.  The kernels below
+// launch ahead of their predecessors' ends (small.h): ordinary loads.
 template <int V>
 struct lanes
 {
@@ -210,14 +211,14 @@ struct lanes
 	{
 		if constexpr (V == 4)
 		{
-			const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+			const float4 t = *reinterpret_cast<const float4*>(p);
 			v[0] = t.x;
 			v[1] = t.y;
 			v[2] = t.z;
 			v[3] = t.w;
 		}
 		else
-			v[0] = __ldg(p);
+			v[0] = *p;
 	}
 
 	__device__ __forceinline__ void store(float* p) const
@@ -247,16 +248,16 @@ __device__ __forceinline__ int split_index(long long t, int n, int& rem)
 // The terms of the agent at sorted position p, V substrates from V q, written to row p; with internalized
 // substrates also the amounts and the agent's rank.
 template <int V>
-__device__ __forceinline__ void agent_terms(int p, int q, int SV, const int* __restrict__ order,
-											const float* __restrict__ sec, const float* __restrict__ sat,
-											const float* __restrict__ upt, const float* __restrict__ nex,
-											const float* __restrict__ intern, const float* __restrict__ vol,
-											float voxel_volume, float dt, float* __restrict__ num,
-											float* __restrict__ den, float* __restrict__ fac,
-											float* __restrict__ sintern, int* __restrict__ rank, lanes<V>& nu,
+__device__ __forceinline__ void agent_terms(int p, int q, int SV, const int* order,
+											const float* sec, const float* sat,
+											const float* upt, const float* nex,
+											const float* intern, const float* vol,
+											float voxel_volume, float dt, float* num,
+											float* den, float* fac,
+											float* sintern, int* rank, lanes<V>& nu,
 											lanes<V>& de, lanes<V>& fa)
 {
-	const int i = __ldg(&order[p]);
+	const int i = order[p];
 	const size_t k = ((size_t)i * SV + q) * V, o = ((size_t)p * SV + q) * V;
 	lanes<V> se, sa, up, ne, in;
 	se.load(sec + k);
@@ -265,7 +266,7 @@ __device__ __forceinline__ void agent_terms(int p, int q, int SV, const int* __r
 	ne.load(nex + k);
 	if (sintern)
 		in.load(intern + k);
-	const float v = __ldg(&vol[i]);
+	const float v = vol[i];
 #pragma unroll
 	for (int c = 0; c < V; c++)
 	{
@@ -290,16 +291,18 @@ __device__ __forceinline__ void agent_terms(int p, int q, int SV, const int* __r
 // the terms where they are needed, instead of in agent order and then sorting them, saves three arrays
 // written and read.
 template <int V>
-__global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int SV, const int* __restrict__ order,
-															const float* __restrict__ sec, const float* __restrict__ sat,
-															const float* __restrict__ upt, const float* __restrict__ nex,
-															const float* __restrict__ intern,
-															const float* __restrict__ vol, float voxel_volume, float dt,
-															float* __restrict__ num, float* __restrict__ den,
-															float* __restrict__ fac, float* __restrict__ sintern,
-															int* __restrict__ rank)
+__global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int SV, const int* order,
+															const float* sec, const float* sat,
+															const float* upt, const float* nex,
+															const float* intern,
+															const float* vol, float voxel_volume, float dt,
+															float* num, float* den,
+															float* fac, float* sintern,
+															int* rank)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	let_next_launch();
+	wait_previous();
 	if (t >= total)
 		return;
 	int q;
@@ -313,26 +316,31 @@ __global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int 
 // (bins.cu) leaves no segments.
 template <int V>
 __global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int SV, int* counts,
-															 const int* __restrict__ seg_start,
-															 const float* __restrict__ num, const float* __restrict__ den,
-															 const float* __restrict__ fac, float* __restrict__ red_num,
-															 float* __restrict__ red_den, float* __restrict__ red_fac,
-															 const int* gave_up)
+															 const int* seg_start,
+															 const float* num, const float* den,
+															 const float* fac, float* red_num,
+															 float* red_den, float* red_fac,
+															 const int* gave_up, uint4* clear, long long units)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	let_next_launch();
+	wait_previous();
 	if (gave_up && *gave_up)
 	{
 		if (t == 0)
 			counts[0] = 0;
 		return;
 	}
+	// the binning's scratch, for the next one
+	for (long long k = t; k < units; k += (long long)gridDim.x * blockDim.x)
+		clear[k] = make_uint4(0, 0, 0, 0);
 	if (t >= total)
 		return;
 	int q;
 	const int seg = split_index(t, SV, q);
 	if (seg >= counts[0])
 		return;
-	const int b = __ldg(&seg_start[seg]), e = __ldg(&seg_start[seg + 1]);
+	const int b = seg_start[seg], e = seg_start[seg + 1];
 	const size_t w = ((size_t)b * SV + q) * V;
 	lanes<V> rn, rd, rf;
 	rn.load(num + w);
@@ -369,14 +377,16 @@ __global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int
 // segment, or an agent outside the mesh, and walks its agents.
 template <int V>
 __global__ void __launch_bounds__(256) segment_terms_kernel(
-	long long total, int SV, int A, const int* __restrict__ counts, const int* __restrict__ seg_start,
-	const int* __restrict__ order, const float* __restrict__ sec, const float* __restrict__ sat,
-	const float* __restrict__ upt, const float* __restrict__ nex, const float* __restrict__ intern,
-	const float* __restrict__ vol, float voxel_volume, float dt, float* __restrict__ num, float* __restrict__ den,
-	float* __restrict__ fac, float* __restrict__ sintern, int* __restrict__ rank, float* __restrict__ red_num,
-	float* __restrict__ red_den, float* __restrict__ red_fac)
+	long long total, int SV, int A, const int* counts, const int* seg_start,
+	const int* order, const float* sec, const float* sat,
+	const float* upt, const float* nex, const float* intern,
+	const float* vol, float voxel_volume, float dt, float* num, float* den,
+	float* fac, float* sintern, int* rank, float* red_num,
+	float* red_den, float* red_fac)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	let_next_launch();
+	wait_previous();
 	if (t >= total)
 		return;
 	int q;
@@ -411,16 +421,18 @@ __global__ void __launch_bounds__(256) segment_terms_kernel(
 // One array between the two orders: to_sorted, row p of `sorted` takes row order[p] of `agent`;
 // otherwise row order[p] of `agent` takes row p of `sorted`.
 template <int V>
-__global__ void __launch_bounds__(256) permute_rows_kernel(long long total, int SV, const int* __restrict__ order,
-															float* __restrict__ agent, float* __restrict__ sorted,
+__global__ void __launch_bounds__(256) permute_rows_kernel(long long total, int SV, const int* order,
+															float* agent, float* sorted,
 															int to_sorted)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	let_next_launch();
+	wait_previous();
 	if (t >= total)
 		return;
 	int q;
 	const int p = split_index(t, SV, q);
-	const size_t k = ((size_t)__ldg(&order[p]) * SV + q) * V, o = (size_t)t * V;
+	const size_t k = ((size_t)order[p] * SV + q) * V, o = (size_t)t * V;
 	lanes<V> x;
 	x.load((to_sorted ? agent + k : sorted + o));
 	x.store((to_sorted ? sorted + o : agent + k));
@@ -587,52 +599,51 @@ int cell_alloc(bfvm_solver* s, int count)
 }
 
 // A kernel over the agents' [A][S] rows, four substrates per thread where S allows.
-#define LAUNCH_ROWS(s, kernel, ...)                                                                                     \
+#define LAUNCH_ROWS(s, follows, kernel, ...)                                                                                \
 	do                                                                                                                 \
 	{                                                                                                                  \
 		const int v_ = (s)->S % 4 == 0 ? 4 : 1, sv_ = (s)->S / v_;                                                     \
 		const long long rows_ = (long long)(s)->ag.count * sv_;                                                        \
 		const unsigned blocks_ = (unsigned)((rows_ + 255) / 256);                                                      \
 		if (v_ == 4)                                                                                                   \
-			kernel<4><<<blocks_, 256, 0, (s)->stream>>>(rows_, sv_, __VA_ARGS__);                                      \
+			st = launch_overlapped(s, #kernel, kernel<4>, dim3(blocks_), dim3(256), 0, follows, rows_, sv_, __VA_ARGS__); \
 		else                                                                                                           \
-			kernel<1><<<blocks_, 256, 0, (s)->stream>>>(rows_, sv_, __VA_ARGS__);                                      \
+			st = launch_overlapped(s, #kernel, kernel<1>, dim3(blocks_), dim3(256), 0, follows, rows_, sv_, __VA_ARGS__); \
 	} while (0)
 
 // The binning, the agent terms in its order and the per-voxel sums; with internalized substrates also
 // the amounts in that order.
-static int rebuild_bins(bfvm_solver* s)
+static int rebuild_bins(bfvm_solver* s, bool follows)
 {
 	agent_state& a = s->ag;
 	int st;
-	if ((st = launch_bins(s)))
+	if ((st = launch_bins(s, follows)))
 		return st;
 	if (a.count <= BIN_BLOCK_AGENTS)
 	{
-		LAUNCH_ROWS(s, segment_terms_kernel, a.count, a.seg_count_dev, a.seg_start, a.vals, a.sec, a.sat, a.upt, a.nex,
+		LAUNCH_ROWS(s, true, segment_terms_kernel, a.count, a.seg_count_dev, a.seg_start, a.vals, a.sec, a.sat, a.upt, a.nex,
 					a.intern, a.vol, (float)(s->voxel[0] * s->voxel[1] * s->voxel[2]), s->dt, a.num, a.den, a.fac,
 					s->internalized ? a.sintern : nullptr, a.rank, a.red_num, a.red_den, a.red_fac);
-		a.binned = true;
-		return check_launch(s, "segment_terms_kernel");
+		a.binned = !st;
+		return st;
 	}
-	LAUNCH_ROWS(s, sorted_terms_kernel, a.vals, a.sec, a.sat, a.upt, a.nex, a.intern, a.vol,
+	LAUNCH_ROWS(s, false, sorted_terms_kernel, a.vals, a.sec, a.sat, a.upt, a.nex, a.intern, a.vol,
 				(float)(s->voxel[0] * s->voxel[1] * s->voxel[2]), s->dt, a.num, a.den, a.fac,
 				s->internalized ? a.sintern : nullptr, a.rank);
-	if ((st = check_launch(s, "sorted_terms_kernel")))
+	if (st)
 		return st;
-	LAUNCH_ROWS(s, reduce_sorted_kernel, a.seg_count_dev, a.seg_start, a.num, a.den, a.fac, a.red_num, a.red_den,
-				a.red_fac, reinterpret_cast<const int*>(a.bin_state));
-	if ((st = check_launch(s, "reduce_sorted_kernel")))
-		return st;
-	a.binned = true;
-	return BFVM_OK;
+	LAUNCH_ROWS(s, false, reduce_sorted_kernel, a.seg_count_dev, a.seg_start, a.num, a.den, a.fac, a.red_num, a.red_den,
+				a.red_fac, reinterpret_cast<const int*>(a.bin_state), reinterpret_cast<uint4*>(a.bin_state), bins_dirty(s));
+	a.binned = !st;
+	return st;
 }
 
 // One per-agent array between agent order and the binning's sorted order.
 static int permute_rows(bfvm_solver* s, float* agent, float* sorted, bool to_sorted)
 {
-	LAUNCH_ROWS(s, permute_rows_kernel, s->ag.vals, agent, sorted, to_sorted ? 1 : 0);
-	return check_launch(s, "permute_rows_kernel");
+	int st;
+	LAUNCH_ROWS(s, false, permute_rows_kernel, s->ag.vals, agent, sorted, to_sorted ? 1 : 0);
+	return st;
 }
 
 // While the agent terms are sorted, the internalized amounts live in sintern: write them back to
@@ -673,7 +684,8 @@ int prepare_agent_terms(bfvm_solver* s, bool recompute)
 	if (!agents_rebin(s, recompute))
 		return BFVM_OK;
 	int st;
-	if ((st = agents_unsort(s, false)) || (st = rebuild_bins(s)))
+	const bool follows = a.sorted; // the binning then follows the kernel that writes the amounts back
+	if ((st = agents_unsort(s, false)) || (st = rebuild_bins(s, follows)))
 		return st;
 	a.sorted = s->internalized;
 	return BFVM_OK;
