@@ -127,6 +127,35 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, i
 				 : "memory");
 }
 
+// Two floats in one instruction (each half rounded as the scalar operation rounds it).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+	uint64_t r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+	return r;
+}
+
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+	float2 r;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+	return r;
+}
+
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+	uint64_t r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+	uint64_t r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+
 } // namespace bfvm
 
 // cuTensorMapEncodeTiled from the driver (sweep_tma.cu); null when the driver does not offer it

@@ -162,14 +162,71 @@ struct tile_line
 	}
 };
 
-// Shared-memory tables of the padded partition: the per-element tables transposed to [S][NP],
-// NP = 32P + 1, so that a thread reaches its substrate's column with immediate offsets and the
-// substrates of a warp fall into distinct banks, and c.  The per-block tables (gq, tgp, Gp; a few
-// hundred floats read only by the carry folds) stay in global memory and are served by L1.
+// Shared-memory tables of the padded partition: the per-element tables transposed to a column per
+// substrate, b' four elements and (tg, tg, G, G) two elements to a 16-byte load, and c.  The columns
+// are 16 bytes longer than their elements, so that the substrates of a warp fall into distinct banks.
+// The per-block tables (gq, tgp, Gp; a few hundred floats read only by the carry folds) stay in
+// global memory and are served by L1.
 __host__ __device__ __forceinline__ int staged_table_floats(int P, int S)
 {
-	const int NP = 32 * P + 1;
-	return 3 * S * NP + S;
+	const int N = 32 * P;
+	return S * (N + 4) + S * (2 * N + 4) + S;
+}
+
+// The block's two recurrences from zero carries, in registers: forward f_v = d_v - e_{v-1} f_{v-1}
+// with e = c b' the float product the reference stores, `carry` = f_q, then backward t_q = f_q b'_q,
+// t_v = (f_v - c t_{v+1}) b'_v.  b' comes four elements to a load and e two to a multiplication: the
+// sweeps wait for issue slots as much as for memory (three sweeps of 220^3 x 8: 478 -> 454 us, 250^3 x 4:
+// 345 -> 334, 320^3 x 16, bound by memory: 2.54 -> 2.50 ms).
+template <int M>
+__device__ __forceinline__ void block_forward(float (&d)[M], float cs, const float4* bq)
+{
+	const uint64_t cc = pack2(cs, cs);
+#pragma unroll
+	for (int i = 0; i < M / 4; i++)
+	{
+		const float4 b = bq[i];
+		const float2 e0 = unpack2(mul2(cc, pack2(b.x, b.y)));
+		const float2 e1 = unpack2(mul2(cc, pack2(b.z, b.w)));
+		d[4 * i + 1] = __fsub_rn(d[4 * i + 1], __fmul_rn(e0.x, d[4 * i]));
+		d[4 * i + 2] = __fsub_rn(d[4 * i + 2], __fmul_rn(e0.y, d[4 * i + 1]));
+		d[4 * i + 3] = __fsub_rn(d[4 * i + 3], __fmul_rn(e1.x, d[4 * i + 2]));
+		if (4 * i + 4 < M)
+			d[4 * i + 4] = __fsub_rn(d[4 * i + 4], __fmul_rn(e1.y, d[4 * i + 3]));
+	}
+}
+
+template <int M>
+__device__ __forceinline__ void block_backward(float (&d)[M], float cs, const float4* bq)
+{
+#pragma unroll
+	for (int i = M / 4 - 1; i >= 0; i--)
+	{
+		const float4 b = bq[i];
+		const float bv[4] = { b.x, b.y, b.z, b.w };
+#pragma unroll
+		for (int k = 3; k >= 0; k--)
+		{
+			const int v = 4 * i + k;
+			d[v] = __fmul_rn(v == M - 1 ? d[v] : __fsub_rn(d[v], __fmul_rn(cs, d[v == M - 1 ? v : v + 1])), bv[k]);
+		}
+	}
+}
+
+// x = t + C tg + X G for the block, two elements to an instruction.
+template <int M>
+__device__ __forceinline__ void block_fixup(float (&d)[M], float C, float X, const float4* tq)
+{
+	const uint64_t cc = pack2(C, C), xx = pack2(X, X);
+#pragma unroll
+	for (int i = 0; i < M / 2; i++)
+	{
+		const float4 r = tq[i];
+		const float2 x =
+			unpack2(fma2(xx, pack2(r.z, r.w), fma2(cc, pack2(r.x, r.y), pack2(d[2 * i], d[2 * i + 1]))));
+		d[2 * i] = x.x;
+		d[2 * i + 1] = x.y;
+	}
 }
 
 // Copy tile wn (if it exists) into a stage whose previous contents every thread has read.
@@ -710,7 +767,6 @@ __global__ void __launch_bounds__(640, 1)
 	const int S = a.S;
 	const int P = a.vP;
 	const int N = 32 * P;
-	const int NP = N + 1;
 	// SLAB 2: this CTA's chunk, its place among the chunk's CTAs, offsets, tables and carries
 	const int kc = SLAB == 2 ? (int)(blockIdx.x % tt.chunks) : 0;
 	const long long cta = SLAB == 2 ? blockIdx.x / tt.chunks : blockIdx.x;
@@ -720,9 +776,10 @@ __global__ void __launch_bounds__(640, 1)
 	const float* const vtab = SLAB == 2 ? tt.chunk_vtab[kc] : a.vtab;
 	const float* const carry_in = SLAB == 2 ? a.slab_carry + (size_t)kc * 2 * a.slab_lines : a.slab_carry;
 	float* tab = stages0 + (size_t)U * NST * tt.stage_floats;
-	float2* tgtab = reinterpret_cast<float2*>(tab); // [S][NP] (tg, G)
-	float* btab = tab + 2 * S * NP;					// [S][NP] b'
-	float* ctab = btab + S * NP;					// [S]
+	const int tg_pitch = 2 * N + 4, b_pitch = N + 4;
+	float* tgtab = tab;					// [S][N / 2] (tg, tg, G, G)
+	float* btab = tab + S * tg_pitch;	// [S][N] b'
+	float* ctab = btab + S * b_pitch;	// [S]
 	const float* gqtab = vtab + (size_t)3 * N * S + S; // [P][S], global
 	const float* tgptab = gqtab + P * S;				 // [P][S], global
 	const float* Gptab = tgptab + P * S;				 // [P][S], global
@@ -757,14 +814,17 @@ __global__ void __launch_bounds__(640, 1)
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	{
-		// tables: global [v][S] -> shared [S][NP]
+		// tables: global [v][S] -> a column per substrate
 		const float* gb = vtab;
 		const float2* gt = reinterpret_cast<const float2*>(vtab + (size_t)N * S);
 		for (int t = tid; t < N * S; t += nthr)
 		{
 			const int v = t / S, s = t - v * S;
-			btab[s * NP + v] = gb[t];
-			tgtab[s * NP + v] = gt[t];
+			btab[s * b_pitch + v] = gb[t];
+			const float2 r = gt[t];
+			float* q = tgtab + s * tg_pitch + (v >> 1) * 4 + (v & 1);
+			q[0] = r.x;
+			q[2] = r.y;
 		}
 		const float* gr = vtab + (size_t)3 * N * S;
 		for (int t = tid; t < S; t += nthr)
@@ -871,7 +931,7 @@ __global__ void __launch_bounds__(640, 1)
 		const bool ok = mbar_wait(&bars[st], parity, a.wait_limit);
 
 		const float cs = ctab[s];
-		const float* bcol = btab + s * NP + p; // b' of this block: bcol[k]
+		const float4* bq = reinterpret_cast<const float4*>(btab + s * b_pitch + p); // b' of this block
 		float d[M];
 		{
 			const float* src = cur + sbase + p * sstride;
@@ -879,17 +939,9 @@ __global__ void __launch_bounds__(640, 1)
 			for (int k = 0; k < M; k++)
 				d[k] = src[k * sstride];
 		}
-		// forward elimination from a zero carry: f_v = d_v - e_{v-1} f_{v-1}, with e = c b' the
-		// float product the reference stores
-#pragma unroll
-		for (int k = 1; k < M; k++)
-			d[k] = __fsub_rn(d[k], __fmul_rn(__fmul_rn(cs, bcol[k - 1]), d[k - 1]));
+		block_forward(d, cs, bq);
 		carry_f[j * 32 + lane] = d[M - 1];
-		// backward substitution from a zero carry: t_q = f_q b'_q, t_v = (f_v - c t_{v+1}) b'_v
-		d[M - 1] = __fmul_rn(d[M - 1], bcol[M - 1]);
-#pragma unroll
-		for (int k = M - 2; k >= 0; k--)
-			d[k] = __fmul_rn(__fsub_rn(d[k], __fmul_rn(cs, d[k + 1])), bcol[k]);
+		block_backward(d, cs, bq);
 
 		if (!group_sync_and(bar_id, gthr, ok))
 		{
@@ -931,13 +983,7 @@ __global__ void __launch_bounds__(640, 1)
 			// X_k = x^{k+1}_p + Gp_{k+1} X_{k+1} from X_{P-1} = the slab's right carry
 			for (int k = P - 1; k > j; k--)
 				Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
-			const float2* tcol = tgtab + s * NP + p;
-#pragma unroll
-			for (int k = 0; k < M; k++)
-			{
-				const float2 r = tcol[k];
-				d[k] = fmaf(Xc, r.y, fmaf(C, r.x, d[k]));
-			}
+			block_fixup(d, C, Xc, reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p));
 		}
 		else if (P > 1)
 		{
@@ -964,13 +1010,7 @@ __global__ void __launch_bounds__(640, 1)
 				for (int k = P - 2; k > j; k--)
 					Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
 			}
-			const float2* tcol = tgtab + s * NP + p;
-#pragma unroll
-			for (int k = 0; k < M; k++)
-			{
-				const float2 r = tcol[k];
-				d[k] = fmaf(Xc, r.y, fmaf(C, r.x, d[k]));
-			}
+			block_fixup(d, C, Xc, reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p));
 		}
 
 		if (FACES && a.face_apply) // the overwrite after this sweep
