@@ -752,8 +752,8 @@ __global__ void __launch_bounds__(512) grad_deferred_kernel(const __grid_constan
 // registers for either.
 // SC (x sweep): the substrate count when the launch fixes it at compile time (0: read at run time),
 // so that the element strides in shared and global memory become immediate offsets.
-template <bool ROWS, bool NOALLOC, int SLAB, int GRAD, int MODE, bool PAIR, int SC = 0>
-__global__ void __launch_bounds__(640, 1)
+template <bool ROWS, bool NOALLOC, int SLAB, int GRAD, int MODE, bool PAIR, int SC, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
 	sweep_tma_kernel(const __grid_constant__ sweep_args a, const __grid_constant__ CUtensorMap map,
 					 const __grid_constant__ tma_tile tt, const __grid_constant__ grad_fuse gf)
 {
@@ -1161,11 +1161,14 @@ template <bool ROWS, bool NOALLOC, int SLAB = 0, int GRAD = 0, int MODE = 0, boo
 static int launch_tma_variant(bfvm_solver* st, const sweep_args& a, const CUtensorMap& map, const tma_tile& tt,
 							  size_t smem, const grad_fuse* gfp = nullptr)
 {
-	auto kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC>;
+	const int threads = 32 * a.vP * tt.groups;
+	auto kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 640>;
+	if constexpr (GRAD == 0 && MODE != 1)
+		if (threads > 640)
+			kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 768>;
 	int rc = set_smem(kernel, smem);
 	if (rc)
 		return rc;
-	const int threads = 32 * a.vP * tt.groups;
 	// one CTA per G tiles (per G / 2 slots of two tiles when paired); chunks in one launch (SLAB 2)
 	// split the resident CTAs evenly among them
 	int grid =
@@ -1302,15 +1305,21 @@ int launch_sweep_tma(bfvm_solver* st, int axis, const sweep_args& a_in, bool& ha
 	int dev = 0, optin = 0;
 	cudaGetDevice(&dev);
 	cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-	// warp groups per CTA: up to 640 threads (20 warps per SM) in at most 8 groups (named barriers
-	// 1..8), fewer when their stages (at least two each) do not fit; each group then takes as many
+	// warp groups per CTA: up to 768 threads (24 warps per SM; two stages of 32 lines for each take all
+	// the shared memory) in at most 8 groups (named barriers 1..8).  More than 640 threads leave 80 registers
+	// each, which pays where they are a whole group more (lines of 7 or 8 blocks, 3 groups for 2: three
+	// sweeps of 250^3 x 4 334 -> 328 us, 220^3 x 8 454 -> 437, 400 x 200^2 x 4 403 -> 385) and costs
+	// where they are not (320^3 x 16 held to 80 registers: 2.47 -> 2.51 ms); up to 640 the instances of
+	// 96 registers run.  The per-tile Dirichlet lists and the gradient inside the sweep hold more registers:
+	// 640.  Fewer when their stages (at least two each) do not fit; each group then takes as many
 	// stages as fit, up to 4
 	const size_t stage_bytes = (size_t)tt.stage_floats * sizeof(float);
+	const int mode = a.dir.items > 0 ? 1 : (a.face_apply ? 2 : 0);
 	auto fixed_bytes = [&](int G) {
 		return 128 + (staged_table_floats(a.vP, (int)S) + (size_t)G * 2 * a.vP * 32) * sizeof(float) + 8
 			   + (size_t)G * 4 * (sizeof(uint64_t) + sizeof(unsigned));
 	};
-	const int Gmax = std::max(1, std::min(8, 20 / a.vP));
+	const int Gmax = std::max(1, std::min(8, (gf || (mode == 1 && !chunk) ? 20 : 24) / a.vP));
 	auto max_stages = [&](int G) { return (int)std::min<size_t>(4, ((size_t)optin - std::min((size_t)optin, fixed_bytes(G))) / ((size_t)G * stage_bytes)); };
 	if (shapes)
 	{
@@ -1343,7 +1352,6 @@ int launch_sweep_tma(bfvm_solver* st, int axis, const sweep_args& a_in, bool& ha
 	// pairs of groups sharing 64-column stages (the same shared memory: half the stages, twice the
 	// width): the plain y and z sweeps over the whole field, an even number of groups, and for y an
 	// even number of tiles per plane so that no pair spans two planes
-	const int mode = a.dir.items > 0 ? 1 : (a.face_apply ? 2 : 0);
 	const bool pair = (axis == 2 ? st->tma_pairs >= 1 : axis == 1 && st->tma_pairs == 2) && !slab_solve && !gf && !chunk
 					  && mode != 1 && w_begin == 0 && w_end < 0 && G % 2 == 0 && (axis == 2 || tt.col_tiles % 2 == 0);
 	if (pair)
