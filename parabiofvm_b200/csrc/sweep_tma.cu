@@ -320,24 +320,26 @@ __device__ __forceinline__ void store_block(float* p, const float (&d)[M])
 }
 
 // The x sweep of SC substrates (R = 32 / SC rows per tile): the stores of a block transposed
-// across the warp, so that each store instruction writes 128 contiguous bytes of one row (R
-// consecutive elements of its SC substrates) instead of SC * 4 bytes in each of R rows.  Lane
-// L = g * SC + s holds row g, substrate s.  For each run of R elements K .. K + R - 1, a butterfly
-// of log2 R shuffle stages turns lane (g, s)'s values v[m] = element K + m of row g into v[r] =
-// element K + g of row r (substrate s), which row r's store then writes at lane L.  r0 points at
-// element 0 of the block in row 0 plus the lane; rows are XS floats apart; `rows` of them exist.
-template <bool NOALLOC, int SC, int M, int K = 0>
-__device__ __forceinline__ void store_block_rows(float* r0, long long XS, float (&d)[M], int g, int rows)
+// across the warp among Q rows, so that each store instruction writes Q consecutive elements (Q * SC * 4
+// contiguous bytes) in each of R / Q rows instead of SC * 4 bytes in each of R rows.  Lane
+// L = g * SC + s holds row g, substrate s; gl = g % Q.  For each run of Q elements K .. K + Q - 1, a
+// butterfly of log2 Q shuffle stages turns lane (g, s)'s values v[m] = element K + m of row g into
+// v[r] = element K + gl of row g - gl + r (substrate s), which the store of step r then writes.  r0 points
+// at the lane's place in element 0 of row g - gl; rows are XS floats apart; `rows` of them exist from there.
+// Q = R up to 4: the third stage that 4 substrates would take to write 128 bytes of one row costs
+// more than the two 64-byte pieces do (three sweeps of 250^3 x 4: Q = 8 328 us, 4 316, 2 315; the long
+// lines of 640 x 160 x 128 x 4: 305, 302, 306).
+template <bool NOALLOC, int SC, int Q, int M, int K = 0>
+__device__ __forceinline__ void store_block_rows(float* r0, long long XS, float (&d)[M], int gl, int rows)
 {
-	constexpr int R = 32 / SC;
 	if constexpr (K < M)
 	{
 #pragma unroll
-		for (int b = 1; b < R; b <<= 1)
+		for (int b = 1; b < Q; b <<= 1)
 		{
-			const bool hi = (g & b) != 0;
+			const bool hi = (gl & b) != 0;
 #pragma unroll
-			for (int m = 0; m < R; m++)
+			for (int m = 0; m < Q; m++)
 				if (!(m & b))
 				{
 					const float send = hi ? d[K + m] : d[K + m + b];
@@ -349,10 +351,10 @@ __device__ __forceinline__ void store_block_rows(float* r0, long long XS, float 
 				}
 		}
 #pragma unroll
-		for (int r = 0; r < R; r++)
+		for (int r = 0; r < Q; r++)
 			if (r < rows)
 				store_element_at<NOALLOC, K * SC>(r0 + r * XS, d[K + r]);
-		store_block_rows<NOALLOC, SC, M, K + R>(r0, XS, d, g, rows);
+		store_block_rows<NOALLOC, SC, Q, M, K + Q>(r0, XS, d, gl, rows);
 	}
 }
 
@@ -1025,11 +1027,13 @@ __global__ void __launch_bounds__(THREADS, 1)
 			if (ROWS && SC >= 4 && (j > 0 || a.pad == 0))
 			{
 				// every lane takes part in the shuffles; the rows' existence predicates the stores
-				constexpr int R = SC ? 32 / SC : 1;
-				const long long row0 = w2 * R;
-				float* r0 = a.data + coff + row0 * tt.XS + (long long)(p - a.pad) * SC + lane;
+				constexpr int R = SC ? 32 / SC : 1, C = SC ? SC : 32;
+				constexpr int Q = R < 4 ? R : 4;
+				const int gl = lane / C % Q, gh = lane / (C * Q) * Q;
+				const long long row0 = w2 * R + gh;
+				float* r0 = a.data + coff + row0 * tt.XS + (long long)(p - a.pad) * SC + lane % (C * Q);
 				const int rows = (int)min((long long)R, tt.nrows - row0);
-				store_block_rows<NOALLOC, (SC ? SC : 32)>(r0, tt.XS, d, lane / (SC ? SC : 32), rows);
+				store_block_rows<NOALLOC, C, Q>(r0, tt.XS, d, gl, rows);
 			}
 			else if (tl2.active)
 			{
