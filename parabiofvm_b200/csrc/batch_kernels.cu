@@ -14,6 +14,7 @@
 
 #include <algorithm>
 
+#include "block_solve.cuh"
 #include "agent_kernels.cuh"
 #include "ensemble.h"
 #include "sweep_common.cuh"
@@ -446,16 +447,15 @@ __global__ void __launch_bounds__(256) ens_secretion_kernel(const ens_inst* __re
 // ------------------------------------------------------------------------------------------------
 // sweeps: one unit = one tile of 32 lines (the tiles of sweep_tma.cu), blockDim = (32, maxP)
 
-// staged tables of one mesh and axis: (tg, G) pairs and b' as [S][NP], NP = 32P + 1, then c [S],
-// the face bits [S] (0 where the sweeps write no faces) and the face values [6][S]
+// staged tables of one mesh and axis: (tg, tg, G, G) [S][N / 2] and b' [S][N] (N = 32 P), columns 16 bytes
+// longer than their elements, then c [S], the face bits [S] (0 where the sweeps write no faces) and the face values [6][S]
 __device__ __forceinline__ void ens_stage_tables(const ens_inst& m, int AXIS, float* tab)
 {
 	const float* __restrict__ vtab = m.vtab[AXIS];
 	const int P = m.vP[AXIS], S = m.S;
-	const int N = 32 * P, NP = N + 1;
-	float2* tgtab = reinterpret_cast<float2*>(tab);
-	float* btab = tab + 2 * S * NP;
-	float* ctab = btab + S * NP;
+	const int N = 32 * P;
+	float* btab = tab + S * (2 * N + 4);
+	float* ctab = btab + S * (N + 4);
 	int* fbits = reinterpret_cast<int*>(ctab + S);
 	float* fvals = ctab + 2 * S;
 	const float2* gt = reinterpret_cast<const float2*>(vtab + (size_t)N * S);
@@ -464,8 +464,11 @@ __device__ __forceinline__ void ens_stage_tables(const ens_inst& m, int AXIS, fl
 	for (int t = tid; t < N * S; t += nthr)
 	{
 		const int v = t / S, s = t - v * S;
-		btab[s * NP + v] = __ldg(&vtab[t]);
-		tgtab[s * NP + v] = __ldg(&gt[t]);
+		btab[s * (N + 4) + v] = __ldg(&vtab[t]);
+		const float2 r = __ldg(&gt[t]);
+		float* q = tab + s * (2 * N + 4) + (v >> 1) * 4 + (v & 1);
+		q[0] = r.x;
+		q[2] = r.y;
 	}
 	for (int t = tid; t < S; t += nthr)
 	{
@@ -580,10 +583,9 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 		const ens_inst& m = inst[cur];
 		const int S = m.S, P = m.vP[AXIS], pad = m.pad[AXIS];
 		const float* vtab = m.vtab[AXIS];
-		const int N = 32 * P, NP = N + 1;
-		const float2* tgtab = reinterpret_cast<const float2*>(tab);
-		const float* btab = tab + 2 * S * NP;
-		const float* ctab = btab + S * NP;
+		const int N = 32 * P;
+		const float* btab = tab + S * (2 * N + 4);
+		const float* ctab = btab + S * (N + 4);
 		const float* gqtab = vtab + (size_t)3 * N * S + S;
 		const float* tgptab = gqtab + P * S;
 		const float* Gptab = tgptab + P * S;
@@ -623,22 +625,18 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 		if (mine)
 		{
 			const float cs = ctab[s];
-			const float* bcol = btab + s * NP + p;
+			const float4* bcol = reinterpret_cast<const float4*>(btab + s * (N + 4) + p);
+			auto bq = [&](int i) { return bcol[i]; };
 #pragma unroll
 			for (int k = 0; k < M; k++)
 			{
 				const int r = p + k - pad; // real element of virtual element p + k
 				d[k] = (active && r >= 0) ? line[r * stride] : 0.f;
 			}
-			// forward and backward recurrences from zero carries (sweep_tma.cu)
-#pragma unroll
-			for (int k = 1; k < M; k++)
-				d[k] = __fsub_rn(d[k], __fmul_rn(__fmul_rn(cs, bcol[k - 1]), d[k - 1]));
+			// forward and backward recurrences from zero carries
+			block_forward(d, cs, bq);
 			carry_f[j * 32 + lane] = d[M - 1];
-			d[M - 1] = __fmul_rn(d[M - 1], bcol[M - 1]);
-#pragma unroll
-			for (int k = M - 2; k >= 0; k--)
-				d[k] = __fmul_rn(__fsub_rn(d[k], __fmul_rn(cs, d[k + 1])), bcol[k]);
+			block_backward(d, cs, bq);
 		}
 		__syncthreads();
 		if (mine && P > 1)
@@ -663,13 +661,8 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 					for (int k = P - 2; k > j; k--)
 						Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
 				}
-				const float2* tcol = tgtab + s * NP + p;
-#pragma unroll
-				for (int k = 0; k < M; k++)
-				{
-					const float2 r = tcol[k];
-					d[k] = fmaf(Xc, r.y, fmaf(C, r.x, d[k]));
-				}
+				const float4* tcol = reinterpret_cast<const float4*>(tab + s * (2 * N + 4) + 2 * p);
+				block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
 			}
 			if (active)
 			{
@@ -748,8 +741,9 @@ bool ensemble_eligible(const bfvm_solver* s)
 	return s->S <= 32 && s->V * s->S < (1LL << 31);
 }
 
-// the staged tables of ens_stage_tables: (tg, G) and b' as [S][NP], c [S], face bits [S], face values [6][S]
-static size_t staged_floats(int P, int S) { return 3 * (size_t)S * (32 * P + 1) + 8 * (size_t)S; }
+// the staged tables of ens_stage_tables: (tg, G) and b' with their columns' padding, c [S], face bits [S], face
+// values [6][S]
+static size_t staged_floats(int P, int S) { return (size_t)S * (3 * 32 * P + 8) + 8 * (size_t)S; }
 
 void ensemble_free(ensemble_plan& plan)
 {

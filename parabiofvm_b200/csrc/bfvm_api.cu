@@ -72,15 +72,16 @@ static int upload_plan(bfvm_solver* s, int axis)
 		BFVM_CUDA(cudaMemcpy(p.vtab, vt.data(), vt.size() * sizeof(float), cudaMemcpyHostToDevice));
 		if (s->V * s->S <= small_elements(s->S))
 		{
-			// the per-element tables with a substrate's values side by side
+			// the per-element tables with a substrate's values side by side, the responses as (tg, tg, G, G)
 			const size_t N = (size_t)32 * p.vP, S = (size_t)s->S;
 			std::vector<float> lt(3 * N * S);
 			for (size_t v = 0; v < N; v++)
 				for (size_t k = 0; k < S; k++)
 				{
 					lt[k * N + v] = vt[v * S + k];
-					lt[N * S + 2 * (k * N + v)] = vt[N * S + 2 * (v * S + k)];
-					lt[N * S + 2 * (k * N + v) + 1] = vt[N * S + 2 * (v * S + k) + 1];
+					float* r = &lt[N * S + 2 * k * N + (v >> 1) * 4 + (v & 1)];
+					r[0] = vt[N * S + 2 * (v * S + k)];
+					r[2] = vt[N * S + 2 * (v * S + k) + 1];
 				}
 			if ((st = device_alloc(&p.ltab, lt.size())))
 				return st;

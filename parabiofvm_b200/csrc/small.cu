@@ -17,6 +17,7 @@
 // 97 x 61 x 83 x 5 53 -> 45, 100^3 x 4 90 -> 62, 128^3 x 4 103 -> 80; lines beyond 512: 800 x 600 x 4 61 -> 33,
 // 40 x 900 x 3 33 -> 18, 60 x 60 x 900 x 2 129 -> 74.
 
+#include "block_solve.cuh"
 #include "small.h"
 #include "sweep_common.cuh"
 
@@ -25,7 +26,7 @@ namespace bfvm {
 struct small_sweep_args
 {
 	float* data;
-	const float* ltab;		   // b' [S][N], then (tg, G) pairs [S][N], of the padded tables (N = 32 P)
+	const float* ltab;		   // b' [S][N], then (tg, tg, G, G) [S][N / 2], of the padded tables (N = 32 P)
 	const float* vtab;		   // the padded tables: c and the per-block products
 	const unsigned int* masks; // per tile, block and lane: the elements with a condition; null: none
 	const float* conditions;   // [V * S]: their values
@@ -102,7 +103,7 @@ struct small_coefficients
 {
 	float b[STAGED ? 1 : 32];
 	const float* bs;
-	const float2* ts;
+	const float4* ts;
 
 	__device__ __forceinline__ small_coefficients(const small_sweep_args& a, int S, int s, int p, const float* tab)
 	{
@@ -110,7 +111,7 @@ struct small_coefficients
 		if constexpr (STAGED)
 		{
 			bs = tab + s * (N + 4) + p;
-			ts = reinterpret_cast<const float2*>(tab + S * (N + 4) + s * (2 * N + 8)) + p;
+			ts = reinterpret_cast<const float4*>(tab + S * (N + 4) + s * (2 * N + 8) + 2 * p);
 		}
 		else
 		{
@@ -124,12 +125,18 @@ struct small_coefficients
 				b[k + 2] = t.z;
 				b[k + 3] = t.w;
 			}
-			ts = reinterpret_cast<const float2*>(a.ltab + (size_t)S * N + 2 * ((size_t)s * N + p));
+			ts = reinterpret_cast<const float4*>(a.ltab + (size_t)S * N + 2 * ((size_t)s * N + p));
 		}
 	}
 
-	__device__ __forceinline__ float operator[](int k) const { return STAGED ? bs[k] : b[STAGED ? 0 : k]; }
-	__device__ __forceinline__ float2 response(int k) const { return STAGED ? ts[k] : __ldg(ts + k); }
+	__device__ __forceinline__ float4 quad(int i) const
+	{
+		if constexpr (STAGED)
+			return reinterpret_cast<const float4*>(bs)[i];
+		else
+			return make_float4(b[4 * i], b[4 * i + 1], b[4 * i + 2], b[4 * i + 3]);
+	}
+	__device__ __forceinline__ float4 response(int i) const { return STAGED ? ts[i] : __ldg(ts + i); }
 };
 
 // The recurrences and carry folds of one block, element by element those of sweep_tma.cu.  Every thread of
@@ -140,15 +147,11 @@ __device__ __forceinline__ void small_solve(float (&d)[32], const small_coeffici
 {
 	constexpr int M = 32;
 	const int P = a.P, N = 32 * P;
-#pragma unroll
-	for (int k = 1; k < M; k++)
-		d[k] = __fsub_rn(d[k], __fmul_rn(__fmul_rn(cs, b[k - 1]), d[k - 1]));
+	auto bq = [&](int i) { return b.quad(i); };
+	block_forward(d, cs, bq);
 	carry_f[j * 32 + lane] = d[M - 1];
 	asm volatile("" ::: "memory"); // staged b' is read again, not kept in 32 registers
-	d[M - 1] = __fmul_rn(d[M - 1], b[M - 1]);
-#pragma unroll
-	for (int k = M - 2; k >= 0; k--)
-		d[k] = __fmul_rn(__fsub_rn(d[k], __fmul_rn(cs, d[k + 1])), b[k]);
+	block_backward(d, cs, bq);
 	if (P == 1)
 		return;
 	const float* gqtab = a.vtab + (size_t)3 * N * S + S;
@@ -170,12 +173,7 @@ __device__ __forceinline__ void small_solve(float (&d)[32], const small_coeffici
 		for (int k = P - 2; k > j; k--)
 			Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
 	}
-#pragma unroll
-	for (int k = 0; k < M; k++)
-	{
-		const float2 t = b.response(k);
-		d[k] = fmaf(Xc, t.y, fmaf(C, t.x, d[k]));
-	}
+	block_fixup(d, C, Xc, [&](int i) { return b.response(i); });
 }
 
 // v = *p where `on` is not zero: straight into the register (a load into a temporary would need 32 more)

@@ -33,6 +33,7 @@
 
 #include <cstring>
 
+#include "block_solve.cuh"
 #include "sm100_common.cuh"
 #include "sweep_common.cuh"
 
@@ -171,62 +172,6 @@ __host__ __device__ __forceinline__ int staged_table_floats(int P, int S)
 {
 	const int N = 32 * P;
 	return S * (N + 4) + S * (2 * N + 4) + S;
-}
-
-// The block's two recurrences from zero carries, in registers: forward f_v = d_v - e_{v-1} f_{v-1}
-// with e = c b' the float product the reference stores, `carry` = f_q, then backward t_q = f_q b'_q,
-// t_v = (f_v - c t_{v+1}) b'_v.  b' comes four elements to a load and e two to a multiplication: the
-// sweeps wait for issue slots as much as for memory (three sweeps of 220^3 x 8: 478 -> 454 us, 250^3 x 4:
-// 345 -> 334, 320^3 x 16, bound by memory: 2.54 -> 2.50 ms).
-template <int M>
-__device__ __forceinline__ void block_forward(float (&d)[M], float cs, const float4* bq)
-{
-	const uint64_t cc = pack2(cs, cs);
-#pragma unroll
-	for (int i = 0; i < M / 4; i++)
-	{
-		const float4 b = bq[i];
-		const float2 e0 = unpack2(mul2(cc, pack2(b.x, b.y)));
-		const float2 e1 = unpack2(mul2(cc, pack2(b.z, b.w)));
-		d[4 * i + 1] = __fsub_rn(d[4 * i + 1], __fmul_rn(e0.x, d[4 * i]));
-		d[4 * i + 2] = __fsub_rn(d[4 * i + 2], __fmul_rn(e0.y, d[4 * i + 1]));
-		d[4 * i + 3] = __fsub_rn(d[4 * i + 3], __fmul_rn(e1.x, d[4 * i + 2]));
-		if (4 * i + 4 < M)
-			d[4 * i + 4] = __fsub_rn(d[4 * i + 4], __fmul_rn(e1.y, d[4 * i + 3]));
-	}
-}
-
-template <int M>
-__device__ __forceinline__ void block_backward(float (&d)[M], float cs, const float4* bq)
-{
-#pragma unroll
-	for (int i = M / 4 - 1; i >= 0; i--)
-	{
-		const float4 b = bq[i];
-		const float bv[4] = { b.x, b.y, b.z, b.w };
-#pragma unroll
-		for (int k = 3; k >= 0; k--)
-		{
-			const int v = 4 * i + k;
-			d[v] = __fmul_rn(v == M - 1 ? d[v] : __fsub_rn(d[v], __fmul_rn(cs, d[v == M - 1 ? v : v + 1])), bv[k]);
-		}
-	}
-}
-
-// x = t + C tg + X G for the block, two elements to an instruction.
-template <int M>
-__device__ __forceinline__ void block_fixup(float (&d)[M], float C, float X, const float4* tq)
-{
-	const uint64_t cc = pack2(C, C), xx = pack2(X, X);
-#pragma unroll
-	for (int i = 0; i < M / 2; i++)
-	{
-		const float4 r = tq[i];
-		const float2 x =
-			unpack2(fma2(xx, pack2(r.z, r.w), fma2(cc, pack2(r.x, r.y), pack2(d[2 * i], d[2 * i + 1]))));
-		d[2 * i] = x.x;
-		d[2 * i + 1] = x.y;
-	}
 }
 
 // Copy tile wn (if it exists) into a stage whose previous contents every thread has read.
@@ -933,7 +878,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 		const bool ok = mbar_wait(&bars[st], parity, a.wait_limit);
 
 		const float cs = ctab[s];
-		const float4* bq = reinterpret_cast<const float4*>(btab + s * b_pitch + p); // b' of this block
+		const float4* bcol = reinterpret_cast<const float4*>(btab + s * b_pitch + p); // b' of this block
+		auto bq = [&](int i) { return bcol[i]; };
 		float d[M];
 		{
 			const float* src = cur + sbase + p * sstride;
@@ -985,7 +931,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 			// X_k = x^{k+1}_p + Gp_{k+1} X_{k+1} from X_{P-1} = the slab's right carry
 			for (int k = P - 1; k > j; k--)
 				Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
-			block_fixup(d, C, Xc, reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p));
+			const float4* tcol = reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p);
+			block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
 		}
 		else if (P > 1)
 		{
@@ -1012,7 +959,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 				for (int k = P - 2; k > j; k--)
 					Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
 			}
-			block_fixup(d, C, Xc, reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p));
+			const float4* tcol = reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p);
+			block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
 		}
 
 		if (FACES && a.face_apply) // the overwrite after this sweep
