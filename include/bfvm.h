@@ -198,11 +198,13 @@ int bfvm_synchronize(bfvm_solver* s);
  *   copies (default 0).  Results are identical either way.
  * - "chunk_elements" N in [64, 512], or 0 (the default, automatic): lines longer than N are swept as
  *   chunks of at most N elements by the staged sweep, joined by per-line carries; automatic cuts
- *   lines longer than 512 into chunks of at most 320 along x and 512 along y and z.  Results agree
- *   to rounding with the sweep of whole lines.
+ *   lines longer than 512 into chunks of at most 320 along x and 512 along y and z, except in small
+ *   meshes (2^21 to 2^24 elements by substrates), which sweep lines of up to 1024 voxels whole.
+ *   Results agree to rounding with the sweep of whole lines.
  * - "tma_pairs" 0/1/2: staged sweeps whose two warp groups share each shared-memory stage, which then
- *   holds two adjacent tiles copied as one 64-column box: 1 (the default) the z sweep, 2 the y and z
- *   sweeps, 0 neither.  Results are identical either way.
+ *   holds two adjacent tiles copied as one 64-column box: 1 the z sweep, 2 the y and z sweeps, 0
+ *   neither.  Until it is set, whichever of y and z measured faster paired at the launch's number of
+ *   groups.  Results are identical either way.
  * - "fused_dirichlet" 0/1: in the LOD step (bfvm_diffusion_solve, bfvm_run_steps) a staged sweep
  *   writes the Dirichlet overwrite that follows it, tile by tile (default 0: the scatter kernel
  *   after the sweep, measured faster).  Results are identical either way.
