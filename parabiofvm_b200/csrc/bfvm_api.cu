@@ -248,7 +248,7 @@ static int end_async_copy(bfvm_solver* s)
 // for them (the copy stream's last event; inside a capture, an external event node that waits for the
 // copies issued before each launch of the graph).  It reads agent data only, so inside a capture it runs
 // beside the diffusion and the gradient, on a branch of the graph: at 50^3 x 4 with 5,000 agents a
-// step with rebinning takes 55 us, where the binning after the gradient made it 23 + 45.
+// step with rebinning takes 45 us, where the binning after the gradient made it 23 + 40.
 int one_step(bfvm_solver* s, bool recompute)
 {
 	int st;

@@ -9,8 +9,9 @@
 //    digit ranks and scatters (single-pass radix sort with decoupled look-back, after Adinets and
 //    Merrill, "Onesweep", 2022), and one finds the segments with the same look-back.
 // The sort was three or more launches per digit (histogram, scan, scatter) and five for the segments, 22 to
-// 28 in all.  One step with rebinning at 100^3 x 4 with 50,000 agents: 200 -> 145 us; ten steps (one
-// rebinning) at 50^3 x 4 with 5,000: 616 -> 571 us, at 128^3 x 4 with 200,000: 1179 -> 1109 us.
+// 28 in all.  One step with rebinning at 100^3 x 4 with 50,000 agents: 200 -> 145 us; now
+// that it runs beside the diffusion (one_step) 80, against 59 without, 45 against 23 at 50^3 x 4 with 5,000 agents,
+// 133 against 76 at 128^3 x 4 with 200,000.
 // The one-CTA form and what follows it launch ahead of their predecessors' ends (small.h), so what one writes
 // the next reads with ordinary loads.  The multi-CTA form does not: beside a captured step's diffusion, CTAs
 // that wait hold the registers that the sweeps need (250^3 x 4, a step with rebinning: 1198 us against 1006).

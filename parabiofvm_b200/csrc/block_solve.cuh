@@ -9,9 +9,10 @@ namespace bfvm {
 
 // The block's two recurrences from zero carries, in registers: forward f_v = d_v - e_{v-1} f_{v-1}
 // with e = c b' the float product the reference stores, then backward t_q = f_q b'_q,
-// t_v = (f_v - c t_{v+1}) b'_v.  bq(i) is b' of elements 4 i .. 4 i + 3.  b' comes four elements to a load and e two to a multiplication: the
-// sweeps wait for issue slots as much as for memory (three sweeps of 220^3 x 8: 478 -> 454 us, 250^3 x 4:
-// 345 -> 334, 320^3 x 16, bound by memory: 2.54 -> 2.50 ms; a step of 128^3 x 4 80 -> 76 us).
+// t_v = (f_v - c t_{v+1}) b'_v.  bq(i) is b' of elements 4 i .. 4 i + 3.  b' comes four elements to a load and e
+// two to a multiplication: the sweeps wait for issue slots as much as for memory (three sweeps of 220^3 x 8:
+// 478 -> 454 us, 250^3 x 4 345 -> 334, 320^3 x 16, bound by memory, 2.54 -> 2.50 ms; a step of
+// 128^3 x 4 80 -> 76 us).
 template <int M, class B>
 __device__ __forceinline__ void block_forward(float (&d)[M], float cs, B&& bq)
 {

@@ -14,7 +14,7 @@
 // The arithmetic is that of the staged sweeps on the same tables (front-padded blocks of 32, precompute.cpp),
 // element by element, so results are the same bits.
 // One step without rebinning, before and now, us: 20^3 x 1 41 -> 12, 50^3 x 4 53 -> 23, 400 x 300 x 3 35 -> 18,
-// 97 x 61 x 83 x 5 53 -> 45, 100^3 x 4 90 -> 62, 128^3 x 4 103 -> 80; lines beyond 512: 800 x 600 x 4 61 -> 33,
+// 97 x 61 x 83 x 5 53 -> 45, 100^3 x 4 90 -> 59, 128^3 x 4 103 -> 76; lines beyond 512: 800 x 600 x 4 61 -> 33,
 // 40 x 900 x 3 33 -> 18, 60 x 60 x 900 x 2 129 -> 74.
 
 #include "block_solve.cuh"

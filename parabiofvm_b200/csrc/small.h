@@ -9,9 +9,10 @@ namespace bfvm {
 
 // The kernels of small.cu take fields of at most this many elements: beyond, the staged sweeps, which copy
 // ahead of the solve, stream faster, the sooner the more a warp's 32 lines spread over substrates (their
-// tables are staged for each CTA).  A step staged and here, us: 220^3 x 1 186 / 110, 200^3 x 2 221 / 187;
-// 128^3 x 4 96 / 80, 160^3 x 4 157 / 160; 72^3 x 12 84 / 72, 91^3 x 8 84 / 73, 90^3 x 7 72 / 78, 101 x 103 x
-// 97 x 6 80 / 86, 80^3 x 16 98 / 109; 40^3 x 24 58 / 51, 50^3 x 32 78 / 83.
+// tables are staged for each CTA).  A step staged and here, us: 220^3 x 1 179 / 100, 200^3 x 2 197 / 169,
+// 128^3 x 4 89 / 70, 72^3 x 12 76 / 65, 40^3 x 24 54 / 48.  Beyond the limits, each before the block solve that
+// both now share took 4 to 6 % from either: 160^3 x 4 157 / 160, 91^3 x 8 84 / 73, 90^3 x 7 72 / 78, 101 x 103 x
+// 97 x 6 80 / 86, 80^3 x 16 98 / 109, 50^3 x 32 78 / 83.
 inline long long small_elements(int S)
 {
 	return S <= 2 ? 1LL << 24 : S <= 4 ? 1LL << 23 : S <= 16 ? 9LL << 19 : 1LL << 21;
