@@ -1049,8 +1049,8 @@ int bfvm_run_steps(bfvm_solver* s, int32_t steps, int32_t first_step)
 	if (steps < 0)
 		return fail(BFVM_ERR_INVALID_ARGUMENT, "steps must not be negative");
 	REFUSE_SLABS(s, "bfvm_run_steps");
-	// agent copies issued on the copy stream are waited for inside each step that rebins (one_step); the
-	// events exist before any graph is captured, so every such graph holds that wait
+	// agent copies issued on the copy stream are waited for inside each step that rebins (one_step) and at the
+	// end; the events exist before any graph is captured, so every such graph holds that wait
 	int oc;
 	if (s->ag.count > 0 && ((oc = ensure_copy_stream(s)) || (oc = ensure_bin_stream(s))))
 		return oc;
@@ -1108,7 +1108,8 @@ int bfvm_run_steps(bfvm_solver* s, int32_t steps, int32_t first_step)
 			s->ag.sorted = s->graph_sorted_after[gi];
 		}
 	}
-	return BFVM_OK;
+	// steps that do not rebin have not waited for the copies: what follows on the stream does
+	return order_after_copies(s);
 }
 
 int bfvm_synchronize(bfvm_solver* s)
