@@ -169,7 +169,9 @@ __device__ __forceinline__ void decode_tile(long long tile, const conv_params& p
 	x0 = xt * SUR_TILE;
 }
 
-// 32 bf16 values of a voxel, as loaded (the epilogue issues these loads before it waits)
+// 32 bf16 values of a voxel, as loaded (the epilogue issues these loads before it waits).  Ordinary loads: a
+// kernel that is launched ahead of its predecessors' ends may still run when this one starts, and then writes
+// what this one reads (small.h).
 struct bf16x32
 {
 	uint4 u[4];
@@ -179,7 +181,7 @@ struct bf16x32
 		const uint4* s = reinterpret_cast<const uint4*>(src);
 #pragma unroll
 		for (int i = 0; i < 4; i++)
-			u[i] = __ldg(s + i);
+			u[i] = s[i];
 	}
 
 	// f(c, value) for each channel
