@@ -220,12 +220,16 @@ int bfvm_synchronize(bfvm_solver* s);
  * - "xy_band_planes" N, "zg_band_rows" N (default 0: off): the LOD step in bands that stay in L2
  *   between two kernels: the x and y sweeps band by band of N z planes, the z sweep and the gradient
  *   band by band of N y rows.  Results are identical either way; measured slower at 320^3 x 16.
- * - "wait_limit_cycles" bounds every wait of the staged sweeps on a tile copy, in GPU clock cycles
- *   (default 4e9, about two seconds; accepted range [1e4, 4e10]).  A wait that runs out makes the
- *   kernel give up its tile, let its copies in flight land and return; the next synchronising call
- *   returns BFVM_ERR_TIMEOUT, and the field is then not valid until it is stored again.
+ * - "wait_limit_cycles" bounds every wait of the staged sweeps on a tile copy and of the agent binning
+ *   (more than 16,384 agents) on another tile, in GPU clock cycles (default 4e9, about two seconds;
+ *   accepted range [1e4, 4e10]).  A wait that runs out makes the kernel give up its tile, let its copies
+ *   in flight land and return; the next synchronising call returns BFVM_ERR_TIMEOUT.  After a sweep's
+ *   the field is not valid until it is stored again.  After the binning's, field and internalized amounts
+ *   are valid, without the secretion and uptake since then, and the next secretion bins again.
  * - "test_drop_tile_copy" (tests of that bound only) names a staged-sweep tile whose stage barrier
  *   is armed but whose copies are never issued, so its wait runs out; -1 (the default) turns it off.
+ *   "test_drop_bin_tile" and "test_drop_segment_tile" do the same to the binning's first radix pass and
+ *   its segments: the tile they name publishes no count.
  */
 int bfvm_set_option(bfvm_solver* s, const char* name, int64_t value);
 

@@ -181,10 +181,13 @@ int check_device_errors(bfvm_solver* s)
 	{
 		BFVM_CUDA(cudaMemsetAsync(s->dev_error, 0, sizeof(int), s->stream));
 		int st;
-		if ((e & DEVERR_TIMEOUT) && (st = bins_reset(s)))
+		if ((e & DEVERR_BINNING) && (st = bins_recover(s)))
 			return st;
 		if (e & DEVERR_TIMEOUT)
 			return fail(BFVM_ERR_TIMEOUT, "a sweep kernel timed out waiting for a tile copy; the field is not valid");
+		if (e & DEVERR_BINNING)
+			return fail(BFVM_ERR_TIMEOUT, "the agent binning timed out waiting for another tile; secretion and uptake were "
+										  "left out since, and the next one bins the agents again");
 		if (e & DEVERR_AGENT_OUTSIDE)
 			return fail(BFVM_ERR_AGENT_OUTSIDE, "an agent position lies outside the mesh; it was left out of "
 												"secretion/uptake");
@@ -1171,6 +1174,12 @@ int bfvm_set_option(bfvm_solver* s, const char* name, int64_t value)
 		if (value < -1)
 			return fail(BFVM_ERR_INVALID_ARGUMENT, "test_drop_tile_copy takes a tile index or -1");
 		s->drop_tile_copy = value;
+	}
+	else if (n == "test_drop_bin_tile" || n == "test_drop_segment_tile")
+	{
+		if (value < -1 || value > INT32_MAX)
+			return fail(BFVM_ERR_INVALID_ARGUMENT, n + " takes a tile index or -1");
+		s->drop_bin_tile[n == "test_drop_bin_tile" ? 0 : 1] = (int)value;
 	}
 	else
 		return fail(BFVM_ERR_INVALID_ARGUMENT, "unknown option " + n);

@@ -40,7 +40,8 @@ int cuda_fail(cudaError_t e, const char* what);
 enum device_error_bits : int
 {
 	DEVERR_AGENT_OUTSIDE = 1,
-	DEVERR_TIMEOUT = 2, // a bounded wait on an asynchronous copy gave up
+	DEVERR_TIMEOUT = 2,	// a bounded wait on an asynchronous copy gave up
+	DEVERR_BINNING = 4,	// ... of the agent binning on another tile
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -223,9 +224,10 @@ struct bfvm_solver
 	int* grad_tile_done = nullptr; // [z tiles] and [1 + z tiles] of the gradient inside the z sweep
 	int* grad_deferred = nullptr;
 	long long grad_tiles = 0;
-	long long wait_limit_cycles = 4000000000LL; // bound of the staged sweeps' waits on tile copies (clock64 cycles;
+	long long wait_limit_cycles = 4000000000LL; // bound of the staged sweeps' and the binning's waits (clock64 cycles;
 												// the default is the kernels' WAIT_LIMIT_CYCLES)
 	long long drop_tile_copy = -1;				// tests only: a staged-sweep tile whose copies are never issued
+	int drop_bin_tile[2] = { -1, -1 };			// ... a tile whose count the first radix pass, the segments' kernel never publishes
 	bfvm::sweep_tuning tune[3];	 // staged sweep launch shape per axis
 
 	// graphs for run_steps: [2 * recompute + agent terms sorted before the step]
@@ -339,7 +341,7 @@ bool agents_rebin(const bfvm_solver* s, bool recompute);
 // the binning and the agent terms' order a secretion update needs (a rebinning when `recompute`)
 int prepare_agent_terms(bfvm_solver* s, bool recompute);
 int agents_unsort(bfvm_solver* s, bool keep_sorted); // internalized amounts back to agent order (cell.cu)
-int bins_reset(bfvm_solver* s); // the binning's scratch after a wait that ran out (bins.cu)
+int bins_recover(bfvm_solver* s); // after a wait of the binning that ran out (bins.cu)
 int solver_drop_graphs(bfvm_solver* s);			  // after queued work, drop the step graphs (bfvm_api.cu)
 int agents_resort_internalized(bfvm_solver* s);	  // stored internalized amounts into sorted order
 int launch_release(bfvm_solver* s, int index);

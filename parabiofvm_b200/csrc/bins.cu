@@ -16,10 +16,10 @@
 // the next reads with ordinary loads.  The multi-CTA form does not: beside a captured step's diffusion, CTAs
 // that wait hold the registers that the sweeps need (250^3 x 4, a step with rebinning: 1198 us against 1006).
 // CTAs of the look-back kernels take their tiles from a counter, so a tile only ever waits for tiles
-// whose CTAs already run; the waits are bounded, and one that runs out raises DEVERR_TIMEOUT and the
+// whose CTAs already run; the waits are bounded, and one that runs out raises DEVERR_BINNING and the
 // scratch's abort word, after which the remaining kernels leave at once with no segments.  What is left
-// in keys and vals then are valid indices of some order (vals starts zeroed), so nothing indexes out of
-// the agents' arrays.
+// in vals then are valid indices (it starts zeroed), so nothing indexes out of the agents' arrays, and the
+// kernel that ends the binning replaces them by the agents' own order (reduce_sorted_kernel).
 
 #include <algorithm>
 
@@ -299,7 +299,7 @@ __device__ __forceinline__ void tile_publish(unsigned long long* p, unsigned lon
 // The counts of the tiles before `tile`: state of tile t at state[t * stride], read LOOK tiles at a time
 // so that their latencies overlap.  False when a wait ran out or the binning was aborted.
 __device__ __forceinline__ bool look_back(const unsigned long long* state, long long stride, int tile,
-										  const volatile int* abort_word, int& sum)
+										  const volatile int* abort_word, long long limit, int& sum)
 {
 	constexpr int LOOK = 8;
 	sum = 0;
@@ -321,7 +321,7 @@ __device__ __forceinline__ bool look_back(const unsigned long long* state, long 
 			if (v[k] & TILE_TOTAL)
 				return true;
 		}
-		if (clock64() - t0 > WAIT_LIMIT_CYCLES || *abort_word)
+		if (clock64() - t0 > limit || *abort_word)
 			return false;
 	}
 	return true;
@@ -329,7 +329,7 @@ __device__ __forceinline__ bool look_back(const unsigned long long* state, long 
 
 // The same for one count per tile, by a warp: 32 tiles at a time.
 __device__ __forceinline__ bool warp_look_back(const unsigned long long* state, int tile, int lane, const volatile int* abort_word,
-											   int& sum)
+											   long long limit, int& sum)
 {
 	sum = 0;
 	const long long t0 = clock64();
@@ -354,7 +354,7 @@ __device__ __forceinline__ bool warp_look_back(const unsigned long long* state, 
 			t -= 32;
 			continue;
 		}
-		const bool give_up = clock64() - t0 > WAIT_LIMIT_CYCLES || *abort_word;
+		const bool give_up = clock64() - t0 > limit || *abort_word;
 		if (__any_sync(0xffffffffu, give_up))
 			return false;
 	}
@@ -400,11 +400,11 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_keys_kernel(const float* pos
 
 // One digit: a tile of PASS_THREADS * ITEMS keys is ranked within the CTA, its digit counts are joined
 // with those of the tiles before it, and its keys go to their places.  vin null: agent indices (the
-// first pass).
+// first pass).  drop: a tile that publishes nothing, for the tests of the waits (-1: none).
 template <int ITEMS>
 __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned int* kin, const int* vin, unsigned int* kout,
 																 int* vout, int n, int pass, int bits, bin_state* st,
-																 unsigned long long* state, int* err)
+																 unsigned long long* state, int* err, long long wait_limit, int drop)
 {
 	__shared__ unsigned short cnt[PASS_WARPS][DIGITS];
 	__shared__ int place[DIGITS]; // where the tile's first key of a digit goes
@@ -464,7 +464,8 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 				cnt[w][d0 + k] = (unsigned short)total[k];
 				total[k] += c;
 			}
-			tile_publish(state + (((long long)tile << bits) + d0 + k), (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total[k]);
+			if (tile != drop)
+				tile_publish(state + (((long long)tile << bits) + d0 + k), (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total[k]);
 			own[k] = st->hist[pass][d0 + k];
 		}
 	// keys of smaller digits: exclusive scan of the pass's histogram
@@ -489,13 +490,13 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 			int before = 0;
 			if (tile > 0)
 			{
-				if (!look_back(state + d0 + k, 1LL << bits, tile, &st->abort, before))
+				if (!look_back(state + d0 + k, 1LL << bits, tile, &st->abort, wait_limit, before))
 				{
-					atomicOr(err, DEVERR_TIMEOUT);
+					atomicOr(err, DEVERR_BINNING);
 					atomicExch(&st->abort, 1);
 					stop = 1;
 				}
-				else
+				else if (tile != drop)
 					tile_publish(state + (((long long)tile << bits) + d0 + k), TILE_TOTAL | (unsigned int)(before + total[k]));
 			}
 			place[d0 + k] = smaller + before;
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 template <int ITEMS>
 __global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsigned int* keys, int n, unsigned int invalid,
 																	 int* seg_start, int* counts, bin_state* st,
-																	 unsigned long long* state, int* err)
+																	 unsigned long long* state, int* err, long long wait_limit, int drop)
 {
 	__shared__ int wsum[PASS_WARPS];
 	__shared__ int tile_s, stop, before_s;
@@ -571,19 +572,19 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsign
 	}
 	if (warp == 0)
 	{
-		if (lane == 0)
+		if (lane == 0 && tile != drop)
 			tile_publish(state + tile, (tile == 0 ? TILE_TOTAL : TILE_SUM) | (unsigned int)total);
 		int before = 0;
-		const bool found = tile == 0 || warp_look_back(state, tile, lane, &st->abort, before);
+		const bool found = tile == 0 || warp_look_back(state, tile, lane, &st->abort, wait_limit, before);
 		if (lane == 0)
 		{
 			if (!found)
 			{
-				atomicOr(err, DEVERR_TIMEOUT);
+				atomicOr(err, DEVERR_BINNING);
 				atomicExch(&st->abort, 1);
 				stop = 1;
 			}
-			else if (tile > 0)
+			else if (tile > 0 && tile != drop)
 				tile_publish(state + tile, TILE_TOTAL | (unsigned int)(before + total));
 			before_s = before;
 		}
@@ -657,11 +658,22 @@ long long bins_dirty(const bfvm_solver* s)
 	return ((long long)(sizeof(bin_state) + 255) / 256 * 256 + states * (long long)sizeof(unsigned long long) + 15) / 16;
 }
 
-// After a wait that ran out: the scratch as it was when allocated.
-int bins_reset(bfvm_solver* s)
+// After a wait that ran out: the scratch as it was when allocated and, where the present agents' binning is the
+// one that gave up, no binning: the next secretion rebins.  (The scratch may have been allocated anew since, or
+// the agents binned by one CTA.)
+int bins_recover(bfvm_solver* s)
 {
-	if (s->ag.bin_state)
-		BFVM_CUDA(cudaMemsetAsync(s->ag.bin_state, 0, s->ag.bin_state_bytes, s->stream));
+	agent_state& a = s->ag;
+	if (!a.bin_state)
+		return BFVM_OK;
+	int gave_up = 0;
+	BFVM_CUDA(cudaMemcpyAsync(&gave_up, a.bin_state, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+	BFVM_CUDA(cudaStreamSynchronize(s->stream));
+	if (!gave_up)
+		return BFVM_OK;
+	BFVM_CUDA(cudaMemsetAsync(a.bin_state, 0, a.bin_state_bytes, s->stream));
+	if (a.count > BIN_BLOCK_AGENTS)
+		a.binned = false;
 	return BFVM_OK;
 }
 
@@ -680,13 +692,15 @@ static int launch_tiles(bfvm_solver* s, bin_state* st, unsigned long long* tiles
 	for (int p = 0; p < passes; p++)
 	{
 		if ((rc = launch_overlapped(s, "bin_pass_kernel", bin_pass_kernel<ITEMS>, dim3(grid), dim3(PASS_THREADS), 0, false, kin,
-									p ? vin : nullptr, kout, vout, A, p, bits, st, tiles + ((size_t)p << bits) * grid, s->dev_error)))
+									p ? vin : nullptr, kout, vout, A, p, bits, st, tiles + ((size_t)p << bits) * grid, s->dev_error,
+									s->wait_limit_cycles, p ? -1 : s->drop_bin_tile[0])))
 			return rc;
 		std::swap(kin, kout);
 		std::swap(vin, vout);
 	}
 	return launch_overlapped(s, "bin_segments_kernel", bin_segments_kernel<ITEMS>, dim3(grid), dim3(PASS_THREADS), 0, false, a.keys,
-							 A, invalid, a.seg_start, a.seg_count_dev, st, tiles + ((size_t)passes << bits) * grid, s->dev_error);
+							 A, invalid, a.seg_start, a.seg_count_dev, st, tiles + ((size_t)passes << bits) * grid, s->dev_error,
+							 s->wait_limit_cycles, s->drop_bin_tile[1]);
 }
 
 int launch_bins(bfvm_solver* s, bool follows)

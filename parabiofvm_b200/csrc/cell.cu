@@ -313,22 +313,38 @@ __global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int 
 }
 
 // The per-voxel sums over the sorted rows (reduce_kernel's, in the same order).  A binning that gave up
-// (bins.cu) leaves no segments.
+// (bins.cu) leaves no segments, and its order is made the agents' own, so that what holds the amounts and finds
+// an agent's row stays right until the host has seen the error.
 template <int V>
 __global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int SV, int* counts,
 															 const int* seg_start,
 															 const float* num, const float* den,
 															 const float* fac, float* red_num,
 															 float* red_den, float* red_fac,
-															 const int* gave_up, uint4* clear, long long units)
+															 const int* gave_up, uint4* clear, long long units, int* order, int* rank,
+															 const float* intern, float* sintern)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	let_next_launch();
 	wait_previous();
-	if (gave_up && *gave_up)
+	if (*gave_up)
 	{
 		if (t == 0)
 			counts[0] = 0;
+		if (t >= total)
+			return;
+		int q;
+		const int i = split_index(t, SV, q);
+		if (q == 0)
+			order[i] = i;
+		if (sintern)
+		{
+			lanes<V> in;
+			in.load(intern + (size_t)t * V);
+			in.store(sintern + (size_t)t * V);
+			if (q == 0)
+				rank[i] = i;
+		}
 		return;
 	}
 	// the binning's scratch, for the next one
@@ -633,7 +649,8 @@ static int rebuild_bins(bfvm_solver* s, bool follows)
 	if (st)
 		return st;
 	LAUNCH_ROWS(s, false, reduce_sorted_kernel, a.seg_count_dev, a.seg_start, a.num, a.den, a.fac, a.red_num, a.red_den,
-				a.red_fac, reinterpret_cast<const int*>(a.bin_state), reinterpret_cast<uint4*>(a.bin_state), bins_dirty(s));
+				a.red_fac, reinterpret_cast<const int*>(a.bin_state), reinterpret_cast<uint4*>(a.bin_state), bins_dirty(s), a.vals,
+				a.rank, a.intern, s->internalized ? a.sintern : nullptr);
 	a.binned = !st;
 	return st;
 }
