@@ -3,6 +3,7 @@
 #pragma once
 
 #include <algorithm>
+#include <mutex>
 #include <string>
 
 #include "bfvm_internal.h"
@@ -186,6 +187,8 @@ inline int persistent_grid(K kernel, int threads, size_t smem, long long items, 
 	return (int)std::max<long long>(1, std::min<long long>(g, items));
 }
 
+// Lets `kernel` be launched with `smem` bytes of dynamic shared memory.  The limit is the kernel's, shared by all
+// solvers of the process, so it is only ever raised: another thread's launch with more must not find it lowered.
 template <typename K>
 inline int set_smem(K kernel, size_t smem)
 {
@@ -197,7 +200,16 @@ inline int set_smem(K kernel, size_t smem)
 												   + std::to_string(smem) + " bytes of shared memory)");
 	if (smem > 48 * 1024)
 	{
-		cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		cudaFuncAttributes now;
+		cudaError_t e = cudaFuncGetAttributes(&now, kernel);
+		if (e == cudaSuccess && now.maxDynamicSharedSizeBytes < (int)smem)
+		{
+			static std::mutex raise;
+			std::lock_guard<std::mutex> guard(raise);
+			e = cudaFuncGetAttributes(&now, kernel);
+			if (e == cudaSuccess && now.maxDynamicSharedSizeBytes < (int)smem)
+				e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		}
 		if (e != cudaSuccess)
 			return cuda_fail(e, "cudaFuncSetAttribute(max dynamic shared memory)");
 	}
