@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(THREADS, 1) bin_block_kernel(const __grid_cons
 
 	// segments: a position starts one when its key differs from the previous position's
 	int heads = 0, valid = 0;
+	unsigned int crowd = 0; // not zero: of these 32 positions, BIN_CROWD in a row continue a segment
 #pragma unroll
 	for (int r = 0; r < BLOCK_ITEMS; r++)
 		if (r < rounds)
@@ -227,14 +228,19 @@ __global__ void __launch_bounds__(THREADS, 1) bin_block_kernel(const __grid_cons
 			// segments that start before this position in the warp, and whether one starts here
 			vr[r] = (vr[r] & 0xffff0000u) | ((unsigned int)(heads + __popc(hb & below)) << 1) | (head ? 1u : 0u);
 			heads += __popc(hb);
-			valid += __popc(__ballot_sync(0xffffffffu, in));
+			const unsigned int vb = __ballot_sync(0xffffffffu, in);
+			valid += __popc(vb);
+			unsigned int more = vb & ~hb;
+			for (int o = 1; o < BIN_CROWD; o <<= 1)
+				more &= more >> o;
+			crowd |= more;
 		}
 	if (lane == 0)
 	{
 		wsum[warp] = heads;
 		wvalid[warp] = valid;
 	}
-	__syncthreads();
+	const int crowded = __syncthreads_or(crowd);
 	int ahead = 0, segments = 0, agents = 0;
 	for (int w = 0; w < BLOCK_WARPS; w++)
 	{
@@ -261,6 +267,7 @@ __global__ void __launch_bounds__(THREADS, 1) bin_block_kernel(const __grid_cons
 		j.counts[0] = segments;
 		j.counts[1] = agents;
 		j.counts[2] = agents > segments ? 1 : 0;
+		j.counts[3] = crowded;
 		j.seg_start[segments] = agents;
 	}
 }
@@ -624,7 +631,11 @@ static long long state_tiles(int A)
 int bins_alloc(bfvm_solver* s, int count)
 {
 	agent_state& a = s->ag;
+	const size_t rows = (size_t)std::min(count, BIN_BLOCK_AGENTS);
 	int st;
+	if ((st = device_alloc(&a.crowd_done, rows)))
+		return st;
+	BFVM_CUDA(cudaMemsetAsync(a.crowd_done, 0, rows * sizeof(int), s->stream));
 	if (count <= BIN_BLOCK_AGENTS)
 		return BFVM_OK;
 	// the most tiles of any count up to this one
