@@ -9,7 +9,9 @@
 // u(z) and u(z+1) in registers, so each plane comes from memory once; the x and y neighbours hit L1 or L2.
 // Columns are counted over the whole plane, so that short rows leave no threads idle, and zc follows the
 // mesh (planes_per_thread).  At 250^3 x 4 185 -> 168 us (6.0 TB/s), 640 x 160 x 128 x 4
-// 160 -> 141 us, 320^3 x 16 1.41 -> 1.37 ms, against rows of CTAs that march 32 planes whatever the mesh.
+// 160 -> 141 us, 320^3 x 16 1.41 -> 1.37 ms, against rows of CTAs that march 32 planes whatever the mesh.  A
+// column's row and voxel come from multiplications: with two divisions a thread of 2-D, which has one element,
+// executes 40 % more instructions (2000 x 2000 x 4: rows of CTAs 78 us, columns with divisions 82, as it is 66).
 
 #include "bfvm_internal.h"
 #include "small.h"
@@ -17,11 +19,28 @@
 
 namespace bfvm {
 
+// w / d for w < 2^31 as (umulhi(magic, w) + w) >> shift (Granlund and Montgomery, "Division by invariant
+// integers using multiplication", 1994)
+struct fixed_divisor
+{
+	unsigned magic;
+	int shift;
+
+	explicit fixed_divisor(unsigned d = 1)
+	{
+		shift = d > 1 ? 32 - __builtin_clz(d - 1) : 0;
+		magic = (unsigned)(((1ULL << 32) * ((1ULL << shift) - d)) / d + 1);
+	}
+
+	__device__ __forceinline__ unsigned divide(unsigned w) const { return (__umulhi(magic, w) + w) >> shift; }
+};
+
 struct gradient_args
 {
 	const float* u;
 	float* g;
 	int X, Y, Z, SV, zc;
+	fixed_divisor row, voxel; // by X * SV and SV
 	long long c0, c1;	// columns of this launch, in units of V elements
 	float b[3], c[3];	// 1/h and 1/(2h) per axis
 };
@@ -62,18 +81,21 @@ struct grad_vec
 	}
 };
 
-// The field is read with ordinary loads: the launch may overlap the end of the kernel that writes it (small.h).
-template <int DIMS, int V>
+// OVERLAP: the launch may overlap the end of the kernel that writes the field, which is read with ordinary loads
+// (small.h).  The two instructions for it cost 0.15 us a wave of CTAs, so in 1-D and 2-D, where a thread has one
+// element (2000 x 2000 x 1, 13 waves: 16.5 us without them, 18.5 with), other launches leave them out.
+template <int DIMS, int V, bool OVERLAP>
 __global__ void __launch_bounds__(256) gradient_kernel(const __grid_constant__ gradient_args a)
 {
-	let_next_launch();
+	if (OVERLAP)
+		let_next_launch();
 	const long long XS = (long long)a.X * a.SV, plane = XS * a.Y; // in units of V elements
 	const long long c = a.c0 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
 	int y, x;
-	if ((plane >> 31) == 0)
+	if (plane < (1LL << 31) - 256)
 	{
-		y = (int)((unsigned)c / (unsigned)XS);
-		x = (int)(((unsigned)c - (unsigned)y * (unsigned)XS) / (unsigned)a.SV);
+		y = (int)a.row.divide((unsigned)c);
+		x = (int)a.voxel.divide((unsigned)c - (unsigned)y * (unsigned)XS);
 	}
 	else
 	{
@@ -85,10 +107,11 @@ __global__ void __launch_bounds__(256) gradient_kernel(const __grid_constant__ g
 	const long long yh = y == a.Y - 1 ? 0 : XS, yl = y == 0 ? 0 : XS;
 	const float fx = (xh && xl) ? a.c[0] : a.b[0], fy = (yh && yl) ? a.c[1] : a.b[1];
 	const long long total = plane * a.Z * V;
-	wait_previous();
+	if (OVERLAP)
+		wait_previous();
 	if (c >= a.c1)
 		return;
-	const int z0 = blockIdx.y * a.zc, z1 = min(a.Z, z0 + a.zc);
+	const int z0 = DIMS == 3 ? blockIdx.y * a.zc : 0, z1 = DIMS == 3 ? min(a.Z, z0 + a.zc) : 1;
 	const float* u = a.u + (z0 * plane + c) * V;
 	float* g = a.g + (z0 * plane + c) * V * (DIMS == 3 ? 1 : DIMS);
 	grad_vec<V> prev, cur;
@@ -132,11 +155,12 @@ __global__ void __launch_bounds__(256) gradient_kernel(const __grid_constant__ g
 // Planes per thread.  A march re-reads the planes at its ends and sets its addresses up once, so up to 8 as
 // long as every SM has four CTAs; longer marches only where they still leave 16 CTAs an SM, as six are
 // resident and a last wave of few costs more (250^3 x 4: 16 planes 168 us, 32 planes 181 us; 97 x 61 x 83 x 5:
-// 8 planes 10.6 us, 2 planes 14.4 us).
+// 8 planes 10.6 us, 2 planes 14.4 us).  The marches are counted rounded up, so that a mesh of few planes is one
+// march where its columns suffice (1000 x 1000 x 3 x 4: 37 us as two, 35 as one; 700 x 700 x 10 x 8 111 and 107).
 static int planes_per_thread(const bfvm_solver* s, long long ctas)
 {
 	int zc = 1;
-	while (zc < 32 && ctas * (s->grid[2] / (2 * zc)) >= (zc < 8 ? 4LL : 16LL) * sm_count_impl(s->device))
+	while (zc < 32 && ctas * ((s->grid[2] + 2 * zc - 1) / (2 * zc)) >= (zc < 8 ? 4LL : 16LL) * sm_count_impl(s->device))
 		zc *= 2;
 	while ((s->grid[2] + zc - 1) / zc > 65535)
 		zc *= 2; // blockIdx.y
@@ -162,13 +186,15 @@ static int launch_gradient_columns(bfvm_solver* s, int y0, int y1, bool overlap)
 		a.b[d] = d < s->dims ? 1.f / s->voxel[d] : 0.f;
 		a.c[d] = d < s->dims ? 1.f / (s->voxel[d] * 2) : 0.f;
 	}
+	a.row = fixed_divisor((unsigned)a.X * (unsigned)a.SV);
+	a.voxel = fixed_divisor((unsigned)a.SV);
 	const long long ctas = (a.c1 - a.c0 + 255) / 256;
 	a.zc = planes_per_thread(s, ctas);
 	const dim3 grid((unsigned)ctas, (unsigned)((a.Z + a.zc - 1) / a.zc));
-	void (*kernel)(const gradient_args) = vec			 ? gradient_kernel<3, 4>
-										  : s->dims == 3 ? gradient_kernel<3, 1>
-										  : s->dims == 2 ? gradient_kernel<2, 1>
-														 : gradient_kernel<1, 1>;
+	void (*kernel)(const gradient_args) = vec			 ? gradient_kernel<3, 4, true>
+										  : s->dims == 3 ? gradient_kernel<3, 1, true>
+										  : s->dims == 2 ? (overlap ? gradient_kernel<2, 1, true> : gradient_kernel<2, 1, false>)
+														 : (overlap ? gradient_kernel<1, 1, true> : gradient_kernel<1, 1, false>);
 	return launch_overlapped(s, "gradient_kernel", kernel, grid, dim3(256), 0, overlap, a);
 }
 
