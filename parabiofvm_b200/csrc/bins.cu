@@ -373,11 +373,9 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_keys_kernel(const float* pos
 																 int bits, bin_state* st, int* counts, int* err)
 {
 	__shared__ int h[MAX_PASSES][DIGITS];
-	let_next_launch();
 	for (int t = threadIdx.x; t < MAX_PASSES * DIGITS; t += PASS_THREADS)
 		h[t / DIGITS][t % DIGITS] = 0;
 	__syncthreads();
-	wait_previous();
 	if (blockIdx.x == 0 && threadIdx.x < 3)
 		counts[threadIdx.x] = 0; // no segments, should no agent be inside
 	const unsigned int mask = (1u << bits) - 1u;
@@ -417,11 +415,9 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_pass_kernel(const unsigned i
 	__shared__ int place[DIGITS]; // where the tile's first key of a digit goes
 	__shared__ int wtot[PASS_WARPS];
 	__shared__ int tile_s, stop;
-	let_next_launch();
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	for (int t = tid; t < PASS_WARPS * DIGITS / 2; t += PASS_THREADS)
 		reinterpret_cast<unsigned int*>(&cnt[0][0])[t] = 0;
-	wait_previous();
 	if (tid == 0)
 	{
 		tile_s = atomicAdd(&st->ticket[pass], 1);
@@ -533,8 +529,6 @@ __global__ void __launch_bounds__(PASS_THREADS) bin_segments_kernel(const unsign
 	__shared__ int wsum[PASS_WARPS];
 	__shared__ int tile_s, stop, before_s;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	let_next_launch();
-	wait_previous();
 	if (tid == 0)
 	{
 		tile_s = atomicAdd(&st->ticket[MAX_PASSES], 1);

@@ -200,8 +200,8 @@ __global__ void reduce_kernel(long long total, int S, const int* __restrict__ co
 	red_fac[t] = rf;
 }
 
-// V consecutive substrates of a row: four as one 16-byte access (S % 4 == 0), else one.  The kernels below
-// launch ahead of their predecessors' ends (small.h): ordinary loads.
+// V consecutive substrates of a row: four as one 16-byte access (S % 4 == 0), else one.  Ordinary loads: some of
+// the kernels below launch ahead of their predecessors' ends (small.h).
 template <int V>
 struct lanes
 {
@@ -383,8 +383,6 @@ __global__ void __launch_bounds__(256) sorted_terms_kernel(long long total, int 
 															int* rank)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	let_next_launch();
-	wait_previous();
 	if (t >= total)
 		return;
 	int q;
@@ -407,8 +405,6 @@ __global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int
 															 const float* intern, float* sintern)
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	let_next_launch();
-	wait_previous();
 	if (*gave_up)
 	{
 		if (t == 0)
@@ -557,7 +553,6 @@ __global__ void __launch_bounds__(256) segment_terms_kernel(
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	int q;
 	const int item = split_index(t, SV, q);
-	let_next_launch();
 	wait_previous();
 	const int segments = counts[0], inside = counts[1];
 	if (counts[3])
@@ -586,7 +581,6 @@ __global__ void __launch_bounds__(256) permute_rows_kernel(long long total, int 
 {
 	const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	let_next_launch();
-	wait_previous();
 	if (t >= total)
 		return;
 	int q;
