@@ -203,8 +203,8 @@ int bfvm_synchronize(bfvm_solver* s);
  *   Results agree to rounding with the sweep of whole lines.
  * - "tma_pairs" 0/1/2: staged sweeps whose two warp groups share each shared-memory stage, which then
  *   holds two adjacent tiles copied as one 64-column box: 1 the z sweep, 2 the y and z sweeps, 0
- *   neither.  Until it is set, whichever of y and z measured faster paired at the launch's number of
- *   groups.  Results are identical either way.
+ *   neither.  Until it is set, whichever of y and z measured faster paired for the launch's groups and
+ *   line length.  Results are identical either way.
  * - "fused_dirichlet" 0/1: in the LOD step (bfvm_diffusion_solve, bfvm_run_steps) a staged sweep
  *   writes the Dirichlet overwrite that follows it, tile by tile (default 0: the scatter kernel
  *   after the sweep, measured faster).  Results are identical either way.

@@ -1304,11 +1304,13 @@ int launch_sweep_tma(bfvm_solver* st, int axis, const sweep_args& a_in, bool& ha
 	// pairs of groups sharing 64-column stages (the same shared memory: half the stages, twice the
 	// width): the plain y and z sweeps over the whole field, an even number of groups, and for y an
 	// even number of tiles per plane so that no pair spans two planes
-	// By default, with two groups a CTA (lines of 9 to 12 blocks) the y sweep and not the z sweep: 320^3 x 16 y
-	// 836 us paired 776, z 820 paired and 780 not; 300^3 x 4 y 167 / 153, z 176 / 171.  With more groups the z
-	// sweep and not the y sweep: three sweeps of 640 x 160 x 128 x 4 304 us, the other way 308.
+	// By default, y with two groups a CTA (lines of 9 to 12 blocks, and shorter ones in fields of few tiles): 300^3 x 4
+	// 166 us single, 153 paired, 380^3 x 2 168 / 151, 80 x 128 x 64 x 8 18.6 / 16.6.  With more groups the same or
+	// slower (three sweeps of 640 x 160 x 128 x 4 304 us, with y paired 308).  z but for lines of 9 and 10 blocks:
+	// 300^3 x 4 170 us single, 174 paired, 320^3 x 4 195 / 203; 11 and 12 blocks 200 x 200 x 350 x 4 101 / 97,
+	// 380^3 x 2 178 / 170; shorter lines 70 x 70 x 128 x 8 18.6 / 16.6, 96 x 96 x 128 x 5 18.6 / 16.8.
 	const bool y_paired = st->tma_pairs < 0 ? G == 2 : st->tma_pairs == 2;
-	const bool z_paired = st->tma_pairs < 0 ? G != 2 : st->tma_pairs >= 1;
+	const bool z_paired = st->tma_pairs < 0 ? a.vP < 9 || a.vP > 10 : st->tma_pairs >= 1;
 	const bool pair = (axis == 2 ? z_paired : axis == 1 && y_paired) && !slab_solve && !gf && !chunk
 					  && mode != 1 && w_begin == 0 && w_end < 0 && G % 2 == 0 && (axis == 2 || tt.col_tiles % 2 == 0);
 	if (pair)
