@@ -201,9 +201,9 @@ int bfvm_synchronize(bfvm_solver* s);
  *   lines longer than 512 into chunks of at most 320 along x and 512 along y and z, except in small
  *   meshes (2^21 to 2^24 elements by substrates), which sweep lines of up to 1024 voxels whole.
  *   Results agree to rounding with the sweep of whole lines.
- * - "tma_pairs" 0/1/2: staged sweeps whose two warp groups share each shared-memory stage, which then
+ * - "tma_pairs" -1/0/1/2: staged sweeps whose two warp groups share each shared-memory stage, which then
  *   holds two adjacent tiles copied as one 64-column box: 1 the z sweep, 2 the y and z sweeps, 0
- *   neither.  Until it is set, whichever of y and z measured faster paired for the launch's groups and
+ *   neither, -1 (the default) whichever of y and z measured faster paired for the launch's groups and
  *   line length.  Results are identical either way.
  * - "fused_dirichlet" 0/1: in the LOD step (bfvm_diffusion_solve, bfvm_run_steps) a staged sweep
  *   writes the Dirichlet overwrite that follows it, tile by tile (default 0: the scatter kernel

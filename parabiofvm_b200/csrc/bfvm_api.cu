@@ -1145,8 +1145,8 @@ int bfvm_set_option(bfvm_solver* s, const char* name, int64_t value)
 	}
 	else if (n == "tma_pairs")
 	{
-		if (value < 0 || value > 2)
-			return fail(BFVM_ERR_INVALID_ARGUMENT, "tma_pairs takes 0, 1 or 2");
+		if (value < -1 || value > 2)
+			return fail(BFVM_ERR_INVALID_ARGUMENT, "tma_pairs takes -1 (the default), 0, 1 or 2");
 		s->tma_pairs = (int)value;
 	}
 	else if (n == "fused_dirichlet")

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from parabiofvm_b200 import Solver
+from parabiofvm_b200 import BfvmError, Solver
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,21 @@ def test_default_pairing_is_the_faster_one(grid, S, axis):
         options.append(best())
     assert default <= 1.08 * min(options), (default, options)  # 12 % where it was lost; runs differ by 2 %
     s.close()
+
+
+def test_default_can_be_put_back():
+    w = np.random.default_rng(2).random(40 * 70 * 128 * 8, dtype=np.float32)
+    fields = []
+    for values in ((), (2, -1), (0,)):
+        s = Solver(3, (0,) * 3, (800, 1400, 2560), (20,) * 3, [1e4] * 8, [0.1] * 8, 0.01)
+        for v in values:
+            s.set_option("tma_pairs", v)
+        for v in (-2, 3):
+            with pytest.raises(BfvmError):
+                s.set_option("tma_pairs", v)
+        s.store_densities(w)
+        s.sweep(2)
+        fields.append(s.load_densities())
+        s.close()
+    for f in fields[1:]:
+        np.testing.assert_array_equal(f, fields[0])
