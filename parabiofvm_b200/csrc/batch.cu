@@ -19,6 +19,7 @@
 
 #include "agent_kernels.cuh"
 #include "ensemble.h"
+#include "small.h"
 
 struct bfvm_batch
 {
@@ -348,6 +349,9 @@ int bfvm_batch_run_steps(bfvm_batch* b, int32_t steps, int32_t first_step)
 		return fail(BFVM_ERR_INVALID_ARGUMENT, "steps must not be negative");
 	BFVM_CUDA(cudaSetDevice(b->device));
 	int st;
+	for (bfvm_solver* s : b->inst)
+		if (steps > 0 && !ensemble_eligible(s) && (st = small_prepare(s))) // steps of its own inside the graph
+			return st;
 	if ((st = batch_wait_instances(b)))
 		return st;
 	for (int32_t i = 0; i < steps; i++)

@@ -255,6 +255,8 @@ static int end_async_copy(bfvm_solver* s)
 int one_step(bfvm_solver* s, bool recompute)
 {
 	int st;
+	if ((st = small_prepare(s)))
+		return st;
 	bool gradient_done = false;
 	const bool rebin = agents_rebin(s, recompute);
 	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1058,6 +1060,8 @@ int bfvm_run_steps(bfvm_solver* s, int32_t steps, int32_t first_step)
 	if (s->ag.count > 0 && ((oc = ensure_copy_stream(s)) || (oc = ensure_bin_stream(s))))
 		return oc;
 	if (s->grad_fused && (oc = grad_fuse_buffers(s)))
+		return oc;
+	if (steps > 0 && (oc = small_prepare(s)))
 		return oc;
 	for (int i = 0; i < steps; i++)
 	{

@@ -191,6 +191,7 @@ struct bfvm_solver
 	float* dir_dense = nullptr;			  // small meshes: the conditions as an array over the field (small.cu)
 	unsigned int* dir_masks[3] = {};	  // ... and its elements as mask bits per axis
 	bool dir_dense_ok = false;			  // these hold the current list
+	bool dir_dense_due = false;			  // they are to hold it from the next step on (small_prepare)
 
 	bfvm::agent_state ag;
 

@@ -390,11 +390,11 @@ bool small_mesh(const bfvm_solver* s)
 }
 
 // The options that name the staged sweeps, and the tests of their bounded waits, keep them.
-bool small_step(const bfvm_solver* s)
+bool small_step(const bfvm_solver* s, bool prepared)
 {
 	return small_mesh(s) && s->use_tma && !s->tma_prefetch && !s->dir_fused && !s->grad_fused && !s->face_dirichlet
 		   && s->xy_band_planes == 0 && s->zg_band_rows == 0 && s->chunk_elements == 0 && s->drop_tile_copy < 0
-		   && (s->dir_qcount + s->dir_count == 0 || s->dir_dense_ok);
+		   && (prepared || s->dir_qcount + s->dir_count == 0 || s->dir_dense_ok);
 }
 
 template <int AXIS>
@@ -483,25 +483,37 @@ static int launch_small_sweep(bfvm_solver* s, bool overlap)
 }
 
 template <int AXIS>
-static int build_masks(bfvm_solver* s)
+static long long mask_words(const bfvm_solver* s)
 {
 	const small_sweep_args a = sweep_args_of<AXIS>(s);
-	const size_t words = (size_t)a.tiles * a.P * 32;
+	return (long long)a.tiles * a.P * 32;
+}
+
+int alloc_small_masks(bfvm_solver* s)
+{
+	const long long words[3] = { mask_words<0>(s), s->dims > 1 ? mask_words<1>(s) : 0, s->dims > 2 ? mask_words<2>(s) : 0 };
 	int st;
-	if (!s->dir_masks[AXIS] && (st = device_alloc(&s->dir_masks[AXIS], words)))
-		return st;
-	small_masks_kernel<AXIS><<<(unsigned)((words + 255) / 256), 256>>>(a, s->dir_masks[AXIS]);
-	BFVM_CUDA(cudaGetLastError());
+	for (int d = 0; d < s->dims; d++)
+		if (!s->dir_masks[d] && (st = device_alloc(&s->dir_masks[d], (size_t)words[d])))
+			return st;
 	return BFVM_OK;
 }
 
-int build_small_masks(bfvm_solver* s)
+template <int AXIS>
+static int fill_masks(bfvm_solver* s)
 {
-	int st = build_masks<0>(s);
+	small_masks_kernel<AXIS><<<(unsigned)((mask_words<AXIS>(s) + 255) / 256), 256, 0, s->stream>>>(sweep_args_of<AXIS>(s),
+																									s->dir_masks[AXIS]);
+	return check_launch(s, "small_masks_kernel");
+}
+
+int fill_small_masks(bfvm_solver* s)
+{
+	int st = fill_masks<0>(s);
 	if (!st && s->dims > 1)
-		st = build_masks<1>(s);
+		st = fill_masks<1>(s);
 	if (!st && s->dims > 2)
-		st = build_masks<2>(s);
+		st = fill_masks<2>(s);
 	return st;
 }
 

@@ -19,12 +19,15 @@ inline long long small_elements(int S)
 }
 static constexpr unsigned int SMALL_FREE = 0xffffffffu; // no condition in bfvm_solver::dir_dense (a NaN)
 
-// the mesh's shape is one that small.cu takes; its step runs there (no option names the other kernels)
+// the mesh's shape is one that small.cu takes; its step runs there (no option names the other kernels), or will
+// once its conditions are prepared; and what a step needs of them, before its first launch or capture
 bool small_mesh(const bfvm_solver* s);
-bool small_step(const bfvm_solver* s);
+bool small_step(const bfvm_solver* s, bool prepared = false);
+int small_prepare(bfvm_solver* s);
 // the overwrites and sweeps of the LOD step
 int launch_small_diffusion(bfvm_solver* s);
-int build_small_masks(bfvm_solver* s); // the sweeps' mask words from bfvm_solver::dir_dense, on the legacy stream
+int alloc_small_masks(bfvm_solver* s); // the sweeps' mask words
+int fill_small_masks(bfvm_solver* s);  // ... from bfvm_solver::dir_dense
 
 // Let the next kernel of the stream launch, and wait for the one before to finish (no-ops in launches
 // without the programmatic attribute).  Field data is read only after the wait, with ordinary loads: a

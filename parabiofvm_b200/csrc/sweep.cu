@@ -411,6 +411,8 @@ int launch_diffusion(bfvm_solver* st, bool gradient, bool* gradient_done)
 {
 	if (gradient_done)
 		*gradient_done = false;
+	if (const int prepared = small_prepare(st))
+		return prepared;
 	if (small_step(st))
 		return launch_small_diffusion(st);
 	// the face conditions by position: each staged sweep writes them into the values it stores, and
