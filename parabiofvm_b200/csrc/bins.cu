@@ -622,6 +622,25 @@ static long long state_tiles(int A)
 	return (A + (long long)tile - 1) / tile;
 }
 
+// radix passes of the multi-CTA form and their bits
+static int pass_count(const bfvm_solver* s, int& bits)
+{
+	int total = 1; // keys take the values 0 .. V
+	while (total < 32 && ((1ull << total) <= (unsigned long long)s->V))
+		total++;
+	const int passes = (total + PASS_BITS - 1) / PASS_BITS;
+	bits = (total + passes - 1) / passes;
+	return passes;
+}
+
+// tile states of a binning: a count per digit and pass, and one of the segments
+static long long states_per_tile(const bfvm_solver* s)
+{
+	int bits;
+	const long long passes = pass_count(s, bits);
+	return (passes << bits) + 1;
+}
+
 int bins_alloc(bfvm_solver* s, int count)
 {
 	agent_state& a = s->ag;
@@ -634,7 +653,7 @@ int bins_alloc(bfvm_solver* s, int count)
 		return BFVM_OK;
 	// the most tiles of any count up to this one
 	const long long tiles = std::max(state_tiles(count), state_tiles(std::min(count, SMALL_TILE_AGENTS)));
-	a.bin_state_bytes = (sizeof(bin_state) + 255) / 256 * 256 + (size_t)tiles * (MAX_PASSES * DIGITS + 1) * sizeof(unsigned long long);
+	a.bin_state_bytes = (sizeof(bin_state) + 255) / 256 * 256 + ((size_t)tiles * states_per_tile(s) + 1) / 2 * 16;
 	if ((st = device_alloc(&a.bin_state, a.bin_state_bytes)) || (st = device_alloc(&a.keys_alt, (size_t)count))
 		|| (st = device_alloc(&a.vals_alt, (size_t)count)))
 		return st;
@@ -643,23 +662,11 @@ int bins_alloc(bfvm_solver* s, int count)
 	return BFVM_OK;
 }
 
-// radix passes of the multi-CTA form and their bits
-static int pass_count(const bfvm_solver* s, int& bits)
-{
-	int total = 1; // keys take the values 0 .. V
-	while (total < 32 && ((1ull << total) <= (unsigned long long)s->V))
-		total++;
-	const int passes = (total + PASS_BITS - 1) / PASS_BITS;
-	bits = (total + passes - 1) / passes;
-	return passes;
-}
-
 // What a binning of the present agents leaves in its scratch, in 16-byte units: cleared by the kernel that ends
 // it (whose abort word is zero then).
 long long bins_dirty(const bfvm_solver* s)
 {
-	int bits;
-	const long long passes = pass_count(s, bits), states = state_tiles(s->ag.count) * ((passes << bits) + 1);
+	const long long states = state_tiles(s->ag.count) * states_per_tile(s);
 	return ((long long)(sizeof(bin_state) + 255) / 256 * 256 + states * (long long)sizeof(unsigned long long) + 15) / 16;
 }
 
