@@ -1,8 +1,8 @@
 // bfvm_secretion_solve_noalloc: the secretion/uptake step with recompute for callers that cannot
-// allocate GPU memory.  It runs the same kernels as bfvm_secretion_solve (agent keys, stable radix
-// sort, voxel segments, intermediates, reductions, update) in the same order, so its results are
-// the same bit for bit; the binning scratch lives in one static device array instead of buffers a
-// solver allocates.
+// allocate GPU memory.  The binning of bins.cu needs scratch that grows with the agents; this one (agent keys,
+// a stable radix sort of three launches a digit, segments by a scan, intermediates, reductions, update) lives in one
+// static device array.  Same order of agents, same sums and same update, so its results are those of
+// bfvm_secretion_solve bit for bit.
 
 #include <mutex>
 

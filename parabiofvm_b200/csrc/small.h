@@ -7,12 +7,14 @@
 
 namespace bfvm {
 
-// The kernels of small.cu take fields of at most this many elements: beyond, the staged sweeps, which copy
-// ahead of the solve, stream faster, the sooner the more a warp's 32 lines spread over substrates (their
-// tables are staged for each CTA).  A step staged and here, us: 220^3 x 1 179 / 100, 200^3 x 2 197 / 169,
-// 128^3 x 4 89 / 70, 72^3 x 12 76 / 65, 40^3 x 24 54 / 48.  Beyond the limits, each before the block solve that
-// both now share took 4 to 6 % from either: 160^3 x 4 157 / 160, 91^3 x 8 84 / 73, 90^3 x 7 72 / 78, 101 x 103 x
-// 97 x 6 80 / 86, 80^3 x 16 98 / 109, 50^3 x 32 78 / 83.
+// The kernels of small.cu take fields of at most this many elements: beyond, the staged sweeps, which copy ahead
+// of the solve, stream faster, the sooner the more a warp's 32 lines spread over substrates (their tables are
+// staged for each CTA).  A step staged and here, us: within the limits 256^3 x 1 262 / 198, 200^3 x 2 198 / 171,
+// 127^3 x 4 102 / 79, 90^3 x 6 70 / 62, 84^3 x 8 62 / 61, 73^3 x 12 80 / 72, 64^3 x 16 56 / 47, 40^3 x 32 59 / 54;
+// beyond them 320^3 x 1 506 / 425, 220^3 x 2 260 / 237, 160^3 x 4 145 / 142, 99^3 x 6 74 / 78, 90^3 x 7 68 / 71,
+// 91^3 x 8 79 / 66, 85^3 x 9 80 / 82, 80^3 x 12 88 / 76, 80^3 x 16 90 / 97, 56^3 x 17 60 / 62, 50^3 x 32 72 / 76.  So the
+// limit is near the crossing for 3 to 4 substrates, for 17 and more and for odd counts (which lose up to 7 % just
+// below it: 97^3 x 5 66 / 70, 78^3 x 9 67 / 72, 73^3 x 11 72 / 75), and low for 1, 2, 8 and 12.
 inline long long small_elements(int S)
 {
 	return S <= 2 ? 1LL << 24 : S <= 4 ? 1LL << 23 : S <= 16 ? 9LL << 19 : 1LL << 21;
