@@ -447,15 +447,34 @@ __global__ void __launch_bounds__(256) ens_secretion_kernel(const ens_inst* __re
 // ------------------------------------------------------------------------------------------------
 // sweeps: one unit = one tile of 32 lines (the tiles of sweep_tma.cu), blockDim = (32, maxP)
 
-// staged tables of one mesh and axis: (tg, tg, G, G) [S][N / 2] and b' [S][N] (N = 32 P), columns 16 bytes
-// longer than their elements, then c [S], the face bits [S] (0 where the sweeps write no faces) and the face values [6][S]
-__device__ __forceinline__ void ens_stage_tables(const ens_inst& m, int AXIS, float* tab)
+// QUADS: the solve of block_solve.cuh, for batches and in the z sweep.  In the x and y sweeps, which hold more to
+// place their lines, that form spills five of 64 registers, and its tables take longer to stage: over the runs of
+// tiles of a batch it still gains (32 meshes 577 -> 575 us a step, 256 meshes 7.76 -> 7.71 ms), on one mesh it
+// loses (x and y of 101 x 103 x 97 x 9 26.4 -> 30.0 and 22.6 -> 26.4 us), so there they take one element to a load.
+//
+// Staged tables of one mesh and axis (N = 32 P), then c [S], the face bits [S] (0 where the sweeps write no faces)
+// and the face values [6][S].  QUADS: (tg, tg, G, G) [S][N / 2] and b' [S][N], columns 16 bytes longer than their
+// elements; else (tg, G) and b' as [S][N + 1].
+template <bool QUADS>
+__device__ __forceinline__ int ens_b_offset(int S, int N)
+{
+	return QUADS ? S * (2 * N + 4) : 2 * S * (N + 1);
+}
+
+template <bool QUADS>
+__device__ __forceinline__ int ens_b_pitch(int N)
+{
+	return QUADS ? N + 4 : N + 1;
+}
+
+template <int AXIS, bool QUADS>
+__device__ __forceinline__ void ens_stage_tables(const ens_inst& m, float* tab)
 {
 	const float* __restrict__ vtab = m.vtab[AXIS];
 	const int P = m.vP[AXIS], S = m.S;
-	const int N = 32 * P;
-	float* btab = tab + S * (2 * N + 4);
-	float* ctab = btab + S * (N + 4);
+	const int N = 32 * P, b_pitch = ens_b_pitch<QUADS>(N);
+	float* btab = tab + ens_b_offset<QUADS>(S, N);
+	float* ctab = btab + S * b_pitch;
 	int* fbits = reinterpret_cast<int*>(ctab + S);
 	float* fvals = ctab + 2 * S;
 	const float2* gt = reinterpret_cast<const float2*>(vtab + (size_t)N * S);
@@ -464,11 +483,16 @@ __device__ __forceinline__ void ens_stage_tables(const ens_inst& m, int AXIS, fl
 	for (int t = tid; t < N * S; t += nthr)
 	{
 		const int v = t / S, s = t - v * S;
-		btab[s * (N + 4) + v] = __ldg(&vtab[t]);
+		btab[s * b_pitch + v] = __ldg(&vtab[t]);
 		const float2 r = __ldg(&gt[t]);
-		float* q = tab + s * (2 * N + 4) + (v >> 1) * 4 + (v & 1);
-		q[0] = r.x;
-		q[2] = r.y;
+		if (QUADS)
+		{
+			float* q = tab + s * (2 * N + 4) + (v >> 1) * 4 + (v & 1);
+			q[0] = r.x;
+			q[2] = r.y;
+		}
+		else
+			reinterpret_cast<float2*>(tab)[s * (N + 1) + v] = r;
 	}
 	for (int t = tid; t < S; t += nthr)
 	{
@@ -548,7 +572,7 @@ __device__ __forceinline__ void x_tile_rows(const ens_inst& m, long long local, 
 // CTAs of 3 warps per SM, too few warps to hide the loads and barriers.
 // MINB 0: lines of 17 to 32 blocks (one mesh alone), CTAs of up to 1024 threads, one per SM; the
 // register cap (64) is that of MINB 2.
-template <int AXIS, int MINB>
+template <int AXIS, int MINB, bool QUADS>
 __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) ens_sweep_kernel(const ens_inst* __restrict__ inst,
 														 const long long* __restrict__ first, int count,
 														 long long units, long long chunk, int maxP)
@@ -576,7 +600,7 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 			first_i = __ldg(&first[i]);
 			first_next = __ldg(&first[i + 1]);
 			__syncthreads(); // the previous mesh's tables are no longer read
-			ens_stage_tables(inst[i], AXIS, tab);
+			ens_stage_tables<AXIS, QUADS>(inst[i], tab);
 			__syncthreads();
 			cur = i;
 		}
@@ -584,8 +608,8 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 		const int S = m.S, P = m.vP[AXIS], pad = m.pad[AXIS];
 		const float* vtab = m.vtab[AXIS];
 		const int N = 32 * P;
-		const float* btab = tab + S * (2 * N + 4);
-		const float* ctab = btab + S * (N + 4);
+		const float* btab = tab + ens_b_offset<QUADS>(S, N);
+		const float* ctab = btab + S * ens_b_pitch<QUADS>(N);
 		const float* gqtab = vtab + (size_t)3 * N * S + S;
 		const float* tgptab = gqtab + P * S;
 		const float* Gptab = tgptab + P * S;
@@ -625,8 +649,8 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 		if (mine)
 		{
 			const float cs = ctab[s];
-			const float4* bcol = reinterpret_cast<const float4*>(btab + s * (N + 4) + p);
-			auto bq = [&](int i) { return bcol[i]; };
+			const float* bcol = btab + s * ens_b_pitch<QUADS>(N) + p;
+			auto bq = [&](int i) { return reinterpret_cast<const float4*>(bcol)[i]; };
 #pragma unroll
 			for (int k = 0; k < M; k++)
 			{
@@ -634,9 +658,24 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 				d[k] = (active && r >= 0) ? line[r * stride] : 0.f;
 			}
 			// forward and backward recurrences from zero carries
-			block_forward(d, cs, bq);
+			if constexpr (QUADS)
+				block_forward(d, cs, bq);
+			else
+			{
+#pragma unroll
+				for (int k = 1; k < M; k++)
+					d[k] = __fsub_rn(d[k], __fmul_rn(__fmul_rn(cs, bcol[k - 1]), d[k - 1]));
+			}
 			carry_f[j * 32 + lane] = d[M - 1];
-			block_backward(d, cs, bq);
+			if constexpr (QUADS)
+				block_backward(d, cs, bq);
+			else
+			{
+				d[M - 1] = __fmul_rn(d[M - 1], bcol[M - 1]);
+#pragma unroll
+				for (int k = M - 2; k >= 0; k--)
+					d[k] = __fmul_rn(__fsub_rn(d[k], __fmul_rn(cs, d[k + 1])), bcol[k]);
+			}
 		}
 		__syncthreads();
 		if (mine && P > 1)
@@ -661,8 +700,21 @@ __global__ void __launch_bounds__(MINB == 0 ? 1024 : 512, MINB == 0 ? 1 : MINB) 
 					for (int k = P - 2; k > j; k--)
 						Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
 				}
-				const float4* tcol = reinterpret_cast<const float4*>(tab + s * (2 * N + 4) + 2 * p);
-				block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
+				if constexpr (QUADS)
+				{
+					const float4* tcol = reinterpret_cast<const float4*>(tab + s * (2 * N + 4) + 2 * p);
+					block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
+				}
+				else
+				{
+					const float2* tcol = reinterpret_cast<const float2*>(tab) + s * (N + 1) + p;
+#pragma unroll
+					for (int k = 0; k < M; k++)
+					{
+						const float2 r = tcol[k];
+						d[k] = fmaf(Xc, r.y, fmaf(C, r.x, d[k]));
+					}
+				}
 			}
 			if (active)
 			{
@@ -741,8 +793,8 @@ bool ensemble_eligible(const bfvm_solver* s)
 	return s->S <= 32 && s->V * s->S < (1LL << 31);
 }
 
-// the staged tables of ens_stage_tables: (tg, G) and b' with their columns' padding, c [S], face bits [S], face
-// values [6][S]
+// the staged tables of ens_stage_tables: (tg, G) and b' with their columns' padding (the larger form's), c [S], face
+// bits [S], face values [6][S]
 static size_t staged_floats(int P, int S) { return (size_t)S * (3 * 32 * P + 8) + 8 * (size_t)S; }
 
 void ensemble_free(ensemble_plan& plan)
@@ -1057,7 +1109,7 @@ static size_t ens_sweep_smem(const ensemble_plan& plan, int axis)
 template <int AXIS, int MINB>
 static int launch_ens_sweep(const ensemble_plan& plan, long long units, cudaStream_t stream)
 {
-	auto kernel = ens_sweep_kernel<AXIS, MINB>;
+	auto kernel = AXIS == 2 || plan.count > 1 ? ens_sweep_kernel<AXIS, MINB, true> : ens_sweep_kernel<AXIS, MINB, AXIS == 2>;
 	const int P = plan.maxP[AXIS];
 	const size_t smem = ens_sweep_smem(plan, AXIS);
 	int rc = set_smem(kernel, smem);
