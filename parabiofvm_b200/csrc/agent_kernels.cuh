@@ -207,7 +207,7 @@ __global__ void scan_add_kernel(int* out, long long n, const int* tile_offsets);
 static constexpr int BIN_BLOCK_AGENTS = 16384;
 // agents of a voxel that one thread still walks there (segment_terms_kernel; a power of two.  bin_block_kernel
 // sees every voxel of twice as many, and most of those between)
-static constexpr int BIN_CROWD = 8;
+static constexpr int BIN_CROWD = 16;
 
 // bins.cu: the agents' order by voxel (agent_state::keys, vals) and its segments, on the solver's
 // stream (follows: launched ahead of the end of a kernel of small.h's kind); the buffers this needs for

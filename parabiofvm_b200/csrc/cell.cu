@@ -474,8 +474,9 @@ __global__ void __launch_bounds__(256) reduce_sorted_kernel(long long total, int
 // more than BIN_CROWD of them (counts[3]) a thread owns a sorted row instead: it finds its segment by bisection,
 // the first row of a short one walks it, and the rows of a long one are computed side by side.  The warp that
 // finishes a long one's last row (done[first row], zero before and after) sums the rows, 0.1 us an agent.
-// Binning 16,384 agents x 4, 18, 50 and 256 to a voxel or all in one: 79 -> 56, 133 -> 58, 427 -> 88 us and
-// 19.2 -> 1.7 ms; at 10 to a voxel, where the line lies, 66 and 55, and 5,000 spread agents 34.9 us as before.
+// Binning and update of 16,384 agents x 4 thrown into few voxels, 10, 18, 41 and 256 to each on average or all in
+// one: 93 -> 90, 123 -> 99, 184 -> 95 and 667 -> 244 us, 24.2 -> 6.5 ms; up to 10, about where the line lies, the
+// same to 3 % (x 3 72 -> 74, x 8 88 -> 86), and 5,000 spread agents are binned in 34.9 us as before.
 template <int V>
 __device__ __forceinline__ void crowded_terms(bool row, int p, int q, int SV, int segments, int inside,
 											  const int* seg_start, const int* order, const float* sec, const float* sat,
