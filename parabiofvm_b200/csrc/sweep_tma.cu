@@ -164,14 +164,28 @@ struct tile_line
 };
 
 // Shared-memory tables of the padded partition: the per-element tables transposed to a column per
-// substrate, b' four elements and (tg, tg, G, G) two elements to a 16-byte load, and c.  The columns
-// are 16 bytes longer than their elements, so that the substrates of a warp fall into distinct banks.
+// substrate, b' four elements and (tg, tg, G, G) two elements to four floats, and c.  QUADS: four floats to a
+// load, the columns 16 bytes longer than their elements, so that any eight substrates in a row fall into
+// distinct banks; a warp's lanes, which come back to the first substrate after the last, then meet none twice
+// up to 8 substrates and at 16, and from 17 on a tile has one row.  For 9 to 15 they do (the lanes of 10 go 8, 9, 0, 1), so
+// these read two floats at a time from columns 8 bytes longer, where any sixteen substrates in a row differ.
+// Three sweeps of 140^3 x 9, 132^3 x 10, 120^3 x 14, 192 x 192 x 54 x 12: one element to a load 167, 157, 144, 153 us,
+// four 186, 170, 154, 150, two 165, 154, 148, 144.
 // The per-block tables (gq, tgp, Gp; a few hundred floats read only by the carry folds) stay in
 // global memory and are served by L1.
 __host__ __device__ __forceinline__ int staged_table_floats(int P, int S)
 {
 	const int N = 32 * P;
 	return S * (N + 4) + S * (2 * N + 4) + S;
+}
+
+template <bool QUADS>
+__device__ __forceinline__ float4 table_quad(const float* p)
+{
+	if constexpr (QUADS)
+		return *reinterpret_cast<const float4*>(p);
+	const float2 lo = *reinterpret_cast<const float2*>(p), hi = *reinterpret_cast<const float2*>(p + 2);
+	return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
 // Copy tile wn (if it exists) into a stage whose previous contents every thread has read.
@@ -699,7 +713,7 @@ __global__ void __launch_bounds__(512) grad_deferred_kernel(const __grid_constan
 // registers for either.
 // SC (x sweep): the substrate count when the launch fixes it at compile time (0: read at run time),
 // so that the element strides in shared and global memory become immediate offsets.
-template <bool ROWS, bool NOALLOC, int SLAB, int GRAD, int MODE, bool PAIR, int SC, int THREADS>
+template <bool ROWS, bool NOALLOC, int SLAB, int GRAD, int MODE, bool PAIR, int SC, int THREADS, bool QUADS>
 __global__ void __launch_bounds__(THREADS, 1)
 	sweep_tma_kernel(const __grid_constant__ sweep_args a, const __grid_constant__ CUtensorMap map,
 					 const __grid_constant__ tma_tile tt, const __grid_constant__ grad_fuse gf)
@@ -723,7 +737,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 	const float* const vtab = SLAB == 2 ? tt.chunk_vtab[kc] : a.vtab;
 	const float* const carry_in = SLAB == 2 ? a.slab_carry + (size_t)kc * 2 * a.slab_lines : a.slab_carry;
 	float* tab = stages0 + (size_t)U * NST * tt.stage_floats;
-	const int tg_pitch = 2 * N + 4, b_pitch = N + 4;
+	const int tg_pitch = 2 * N + (QUADS ? 4 : 2), b_pitch = N + (QUADS ? 4 : 2);
 	float* tgtab = tab;					// [S][N / 2] (tg, tg, G, G)
 	float* btab = tab + S * tg_pitch;	// [S][N] b'
 	float* ctab = btab + S * b_pitch;	// [S]
@@ -878,8 +892,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 		const bool ok = mbar_wait(&bars[st], parity, a.wait_limit);
 
 		const float cs = ctab[s];
-		const float4* bcol = reinterpret_cast<const float4*>(btab + s * b_pitch + p); // b' of this block
-		auto bq = [&](int i) { return bcol[i]; };
+		const float* bcol = btab + s * b_pitch + p; // b' of this block
+		auto bq = [&](int i) { return table_quad<QUADS>(bcol + 4 * i); };
 		float d[M];
 		{
 			const float* src = cur + sbase + p * sstride;
@@ -931,8 +945,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 			// X_k = x^{k+1}_p + Gp_{k+1} X_{k+1} from X_{P-1} = the slab's right carry
 			for (int k = P - 1; k > j; k--)
 				Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
-			const float4* tcol = reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p);
-			block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
+			const float* tcol = tgtab + s * tg_pitch + 2 * p;
+			block_fixup(d, C, Xc, [&](int i) { return table_quad<QUADS>(tcol + 4 * i); });
 		}
 		else if (P > 1)
 		{
@@ -959,8 +973,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 				for (int k = P - 2; k > j; k--)
 					Xc = fmaf(__ldg(&Gptab[k * S + s]), Xc, carry_t[k * 32 + lane]);
 			}
-			const float4* tcol = reinterpret_cast<const float4*>(tgtab + s * tg_pitch + 2 * p);
-			block_fixup(d, C, Xc, [&](int i) { return tcol[i]; });
+			const float* tcol = tgtab + s * tg_pitch + 2 * p;
+			block_fixup(d, C, Xc, [&](int i) { return table_quad<QUADS>(tcol + 4 * i); });
 		}
 
 		if (FACES && a.face_apply) // the overwrite after this sweep
@@ -1114,10 +1128,18 @@ static int launch_tma_variant(bfvm_solver* st, const sweep_args& a, const CUtens
 							  size_t smem, const grad_fuse* gfp = nullptr)
 {
 	const int threads = 32 * a.vP * tt.groups;
-	auto kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 640>;
+	auto kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 640, true>;
+	if constexpr (SC == 0)
+		if (a.S > 8 && a.S < 16)
+			kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 640, false>;
 	if constexpr (GRAD == 0 && MODE != 1)
 		if (threads > 640)
-			kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 768>;
+		{
+			kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 768, true>;
+			if constexpr (SC == 0)
+				if (a.S > 8 && a.S < 16)
+					kernel = sweep_tma_kernel<ROWS, NOALLOC, SLAB, GRAD, MODE, PAIR, SC, 768, false>;
+		}
 	int rc = set_smem(kernel, smem);
 	if (rc)
 		return rc;
