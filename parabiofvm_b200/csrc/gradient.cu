@@ -13,6 +13,8 @@
 // column's row and voxel come from multiplications: with two divisions a thread of 2-D, which has one element,
 // executes 40 % more instructions (2000 x 2000 x 4: rows of CTAs 78 us, columns with divisions 82, as it is 66).
 
+#include <algorithm>
+
 #include "bfvm_internal.h"
 #include "small.h"
 #include "sweep_common.cuh"
@@ -155,12 +157,13 @@ __global__ void __launch_bounds__(256) gradient_kernel(const __grid_constant__ g
 // Planes per thread.  A march re-reads the planes at its ends and sets its addresses up once, so up to 8 as
 // long as every SM has four CTAs; longer marches only where they still leave 16 CTAs an SM, as six are
 // resident and a last wave of few costs more (250^3 x 4: 16 planes 168 us, 32 planes 181 us; 97 x 61 x 83 x 5:
-// 8 planes 10.6 us, 2 planes 14.4 us).  The marches are counted rounded up, so that a mesh of few planes is one
-// march where its columns suffice (1000 x 1000 x 3 x 4: 37 us as two, 35 as one; 700 x 700 x 10 x 8 111 and 107).
+// 8 planes 10.6 us, 2 planes 14.4 us).  A mesh of few planes is one march where its columns suffice (1000 x 1000 x
+// 3 x 4: 37 us as two, 35 as one; 700 x 700 x 10 x 8 111 and 107); other marches are counted as if all were whole
+// (301 x 48 x 66 x 40 as 8 of 8 planes and one of 2 100 us, as 4 of 16 and one of 2 105).
 static int planes_per_thread(const bfvm_solver* s, long long ctas)
 {
 	int zc = 1;
-	while (zc < 32 && ctas * ((s->grid[2] + 2 * zc - 1) / (2 * zc)) >= (zc < 8 ? 4LL : 16LL) * sm_count_impl(s->device))
+	while (zc < 32 && ctas * std::max(1, s->grid[2] / (2 * zc)) >= (zc < 8 ? 4LL : 16LL) * sm_count_impl(s->device))
 		zc *= 2;
 	while ((s->grid[2] + zc - 1) / zc > 65535)
 		zc *= 2; // blockIdx.y
