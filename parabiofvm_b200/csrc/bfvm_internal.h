@@ -123,7 +123,7 @@ struct agent_state
 	size_t bin_state_bytes = 0;
 	int* seg_start = nullptr;	 // [A+1]
 	int* seg_count_dev = nullptr; // number of segments, of agents inside the mesh; a voxel holds several; more than BIN_CROWD
-	int* crowd_done = nullptr;	  // rows finished of a crowded voxel's segment, at its first row (one-CTA binning)
+	int* crowd_done = nullptr;	  // behind them: rows finished of a crowded voxel's segment, at its first row (one-CTA binning)
 	float *num = nullptr, *den = nullptr, *fac = nullptr;			 // [A][S] in the sorted order
 	float *red_num = nullptr, *red_den = nullptr, *red_fac = nullptr; // [A][S] by segment
 	bool binned = false;		 // a recompute has run since the last store

@@ -644,11 +644,12 @@ static long long states_per_tile(const bfvm_solver* s)
 int bins_alloc(bfvm_solver* s, int count)
 {
 	agent_state& a = s->ag;
-	const size_t rows = (size_t)std::min(count, BIN_BLOCK_AGENTS);
+	const size_t counts = 4 + (size_t)std::min(count, BIN_BLOCK_AGENTS);
 	int st;
-	if ((st = device_alloc(&a.crowd_done, rows)))
+	if ((st = device_alloc(&a.seg_count_dev, counts)))
 		return st;
-	BFVM_CUDA(cudaMemsetAsync(a.crowd_done, 0, rows * sizeof(int), s->stream));
+	BFVM_CUDA(cudaMemsetAsync(a.seg_count_dev, 0, counts * sizeof(int), s->stream));
+	a.crowd_done = a.seg_count_dev + 4;
 	if (count <= BIN_BLOCK_AGENTS)
 		return BFVM_OK;
 	// the most tiles of any count up to this one

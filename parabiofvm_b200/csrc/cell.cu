@@ -709,7 +709,7 @@ void cell_free(bfvm_solver* s)
 	device_free(a.vals);
 	device_free(a.vals_alt);
 	device_free(a.bin_state);
-	device_free(a.crowd_done);
+	a.crowd_done = nullptr;
 	device_free(a.seg_start);
 	device_free(a.seg_count_dev);
 	device_free(a.move_idx);
@@ -742,8 +742,7 @@ int cell_alloc(bfvm_solver* s, int count)
 			return st;
 	}
 	if ((st = device_alloc(&a.keys, (size_t)count)) || (st = device_alloc(&a.vals, (size_t)count))
-		|| (st = device_alloc(&a.seg_start, (size_t)count + 1)) || (st = device_alloc(&a.seg_count_dev, 4))
-		|| (st = bins_alloc(s, count)))
+		|| (st = device_alloc(&a.seg_start, (size_t)count + 1)) || (st = bins_alloc(s, count)))
 		return st;
 	// indices of some agent, whatever a binning that gave up leaves of them (bins.cu)
 	BFVM_CUDA(cudaMemsetAsync(a.vals, 0, (size_t)count * sizeof(int), s->stream));
