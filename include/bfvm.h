@@ -239,7 +239,9 @@ int bfvm_set_option(bfvm_solver* s, const char* name, int64_t value);
  * on a scratch copy of the field, and keep the fastest.  The choice is also recorded for the rest
  * of the process under the mesh shape, so solvers of the same shape use it without measuring.
  * choices, if not NULL, receives [dims][2] = (groups, stages), (0, 0) for an axis the staged path
- * does not take.  Results do not depend on the launch shape.  Needs one field's worth of scratch.
+ * does not take.  Results do not depend on the launch shape.  Needs one field's worth of scratch.  On a
+ * small mesh (2^21 to 2^24 elements by substrates) the step does not run the staged sweeps: there the
+ * choices serve bfvm_diffusion_sweep and the steps under options that name those sweeps.
  */
 int bfvm_autotune(bfvm_solver* s, int32_t* choices);
 
