@@ -55,5 +55,5 @@ def test_x_sweep_of_one_mesh_keeps_its_time():
         return min(times)
 
     x, z = best(0), best(2)
-    assert x < 1.14 * z, (x, z)  # 1.21 with that form, 1.07 without; runs differ by 1 %
+    assert x < 1.16 * z, (x, z)  # 1.21 with that form, 1.07 to 1.09 without
     s.close()
